@@ -309,11 +309,12 @@ class FixChargeEwald : public Fix {
     DBuf<float> e_r;        // 3 real grids
     DBuf<float> green;      // half spectrum Green function
     DBuf<double> energy_acc;
-    // own FFT path (cubic 32^3 / 64^3 meshes): field interleaved as float4
+    // own FFT path (cubic 32^3, 64^3, 128^3 meshes): field interleaved as float4
     bool own_fft = false;
+    DBuf<float> green_own;  // the Green function as (kx, kz, ky)
     DBuf<double> vir_acc;  // reciprocal-space virial sum (6)
     DBuf<float4> e4;
-    DBuf<float2> tw;        // W_32^k then W_64^k
+    DBuf<float2> tw;        // W_n^k, n the mesh side
     FixChargeEwald(State *s, std::string h, std::string g);
     ~FixChargeEwald() override;
     int setParameters(int nx, int ny, int nz, double rcut, int ord);
@@ -618,7 +619,7 @@ class Batch {
         DBuf<float> rho, e_r;
         DBuf<float2> rho_k, e_k;
         cufftHandle r2c = 0, c2r = 0;
-        // cubic 32^3 / 64^3 meshes: this library's FFT kernels over the
+        // cubic 32^3, 64^3, 128^3 meshes: this library's FFT kernels over the
         // class's replicas (a table of their field pointers), no cuFFT
         bool own = false;
         DBuf<char> tab;

@@ -151,6 +151,9 @@ __global__ void k_spread5(const P3MArgs a0, const P3MArgs *__restrict__ tab) {
 __device__ __forceinline__ int mol_site(int4 ix, int k, int four_site) {
     return four_site ? (k == 0 ? ix.y : (k == 1 ? ix.z : ix.w)) : (k == 0 ? ix.x : (k == 1 ? ix.y : ix.z));
 }
+__device__ __forceinline__ int4 mol_atoms(const P3MArgs &A, int m) {
+    return A.slots ? make_int4(4 * m, 4 * m + 1, 4 * m + 2, 4 * m + 3) : A.mol_idx[m];
+}
 
 // the molecule form: lanes 15 j .. 15 j + 14 of a warp take the three
 // charged sites (five planes each) of one molecule, two molecules per warp,
@@ -163,8 +166,7 @@ __global__ void k_spread_mol(const P3MArgs a0, const P3MArgs *__restrict__ tab) 
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int m = (lane / 15) * W + w;
     if (lane >= 30 || w >= W || m >= A.nmol) return;
-    const int4 ix = A.slots ? make_int4(4 * m, 4 * m + 1, 4 * m + 2, 4 * m + 3) : A.mol_idx[m];
-    spread_plane(A, mol_site(ix, (lane % 15) / 5, A.four_site), lane % 5);
+    spread_plane(A, mol_site(mol_atoms(A, m), (lane % 15) / 5, A.four_site), lane % 5);
 }
 
 // E_d(k) = i k_d G rho on the half spectrum (z halved), batched output
@@ -365,384 +367,538 @@ P3MArgs p3m_args(State &s, FixChargeEwald &f) {
     return A;
 }
 
-// ---- P3M reciprocal solve on our own FFT (cubic 32^3 / 64^3 meshes) --------
-// One warp transforms one line of N = 32 R points held as v[r] = x[32 r + lane]:
-// R-point DFTs inside each lane, twiddles W_N^(lane k1), then a radix-2
-// decimation-in-frequency FFT of 32 points across the lanes (shuffles); lane
-// l then holds X[k1 + R bitrev5(l)] in v[k1].  Unnormalised, as cuFFT.
+// ---- P3M reciprocal solve on our own FFT (cubic 32^3, 64^3, 128^3 meshes) --
+// A line of N points is transformed by TL = 8 lanes of a warp (four lines per
+// warp), each holding P = N/8 points: a P-point DFT in registers over the
+// points TL n1 + l of lane l, twiddles W_N^(l k1), one exchange of the line
+// among its lanes through shared memory, then P/TL DFTs of TL points over the
+// lanes' index.  Lane l ends with X[(l + TL m) + P k2] in v[m TL + k2]; the
+// inverse runs the same steps backwards, from that layout to the points
+// TL n1 + l, so neither direction permutes a line beyond its one exchange.
+// Unnormalised, as cuFFT.  (One line per warp with five radix-2 shuffle
+// stages, the layout before, spent 20 shuffles and as many selects per line
+// and lane, and read and wrote one 8-byte word per 32-byte sector in the x
+// pass; figures at own_solve.)
 // Three kernels replace R2C + E(k) + batched C2R:
-//   k_fft_zy   per x plane: real FFT along z (half spectrum kept) then along y
-//   k_fft_xe   per (ky, kz) line: FFT along x, E_d(k) = i k_d G rho (Nyquist
-//              planes dropped per component, as k_efield), 3 inverse FFTs along x
-//   k_ifft_yz  per (x plane, component): inverse along y, then the real inverse along z of
-//              the Hermitian half spectrum, E written as float4 (Ex, Ey, Ez, 0)
-// so the gather reads one 16-byte field value per stencil point.
+//   k_fft_zy   per x plane: real FFTs along z, two rows packed into one
+//              complex transform (half spectrum kept), then along y
+//   k_fft_xe   per (kz, 32/TL adjacent ky): FFT along x, E_d(k) = i k_d G rho
+//              (Nyquist planes dropped per component, as k_efield), 3 inverse
+//              FFTs along x; whole 32-byte sectors on both sides
+//   k_ifft_yz  per x plane, (Ex, Ey) or Ez: inverse along y, then along z
+//              with (Ex, Ey) of a row, or Ez of two rows, packed into one
+//              complex transform; E interleaved as float4 (Ex, Ey, Ez, unset)
+// so the gather reads one 16-byte value per stencil point.
 struct FFTArgs {
-    int n;                   // points per side (32 or 64)
+    int n;                   // points per side (32, 64 or 128)
     const float *rho;        // [n][n][n]
     float2 *mid1;            // [n][n/2+1][n] (x, kz, ky): after the z and y passes
     float2 *mid2;            // [3][n][n/2+1][n] (d, x, kz, ky): E_d after the inverse x pass
     float4 *e4;              // [n][n][n]
-    const float *green;      // [n][n][n/2+1]
-    const float2 *tw;        // W_32^k (32) then W_64^k (64), forward sign
+    const float *green;      // [n][n/2+1][n] (kx, kz, ky)
+    const float2 *tw;        // W_n^k, forward sign
     float3 tpl;              // 2 pi / L
 };
 
-__device__ __forceinline__ int brev5(int l) { return (int)(__brev((unsigned)l) >> 27); }
-
+__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 operator-(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// times -i (forward) or i (inverse)
+template <bool INV>
+__device__ __forceinline__ float2 rot90(float2 a) {
+    return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
+// times w (forward sign given) or its conjugate
+template <bool INV>
+__device__ __forceinline__ float2 twid(float2 a, float2 w) {
+    return INV ? make_float2(a.x * w.x + a.y * w.y, a.y * w.x - a.x * w.y) : cmul(a, w);
+}
 
-// this lane's twiddles: W_2h^(lane mod h) for the five lane stages and
-// W_N^lane for the R = 2 step (forward sign; conjugated for the inverse)
-struct LaneTw {
-    float2 st[5];
-    float2 wn;
+template <bool INV>
+__device__ __forceinline__ void dft4(float2 &a, float2 &b, float2 &c, float2 &d) {
+    const float2 s0 = a + c, s1 = a - c, s2 = b + d, s3 = rot90<INV>(b - d);
+    a = s0 + s2;
+    b = s1 + s3;
+    c = s0 - s2;
+    d = s1 - s3;
+}
+
+// DFT of the n values v[0], ..., v[n-1] in place (n = 4, 8, 16)
+template <int n, bool INV>
+__device__ __forceinline__ void dft(float2 *v) {
+    constexpr float kR = 0.70710678118654752f;   // cos(pi/4)
+    constexpr float kC = 0.92387953251128674f;   // cos(pi/8)
+    constexpr float kS = 0.38268343236508977f;   // sin(pi/8)
+    if constexpr (n == 4) {
+        dft4<INV>(v[0], v[1], v[2], v[3]);
+    } else if constexpr (n == 8) {
+        float2 e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        dft4<INV>(e[0], e[1], e[2], e[3]);
+        dft4<INV>(o[0], o[1], o[2], o[3]);
+        o[1] = twid<INV>(o[1], make_float2(kR, -kR));
+        o[2] = rot90<INV>(o[2]);
+        o[3] = twid<INV>(o[3], make_float2(-kR, -kR));
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            v[k] = e[k] + o[k];
+            v[k + 4] = e[k] - o[k];
+        }
+    } else {
+        static_assert(n == 16, "4, 8 or 16 points");
+        const float2 w1 = make_float2(kC, -kS), w2 = make_float2(kR, -kR), w3 = make_float2(kS, -kC);
+        float2 y[4][4];  // y[b][k1]: DFT over a of v[4 a + b]
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+#pragma unroll
+            for (int a = 0; a < 4; a++) y[b][a] = v[4 * a + b];
+            dft4<INV>(y[b][0], y[b][1], y[b][2], y[b][3]);
+        }
+        // times W_16^(b k1)
+        y[1][1] = twid<INV>(y[1][1], w1);
+        y[1][2] = twid<INV>(y[1][2], w2);
+        y[1][3] = twid<INV>(y[1][3], w3);
+        y[2][1] = twid<INV>(y[2][1], w2);
+        y[2][2] = rot90<INV>(y[2][2]);
+        y[2][3] = twid<INV>(y[2][3], make_float2(-kR, -kR));
+        y[3][1] = twid<INV>(y[3][1], w3);
+        y[3][2] = twid<INV>(y[3][2], make_float2(-kR, -kR));
+        y[3][3] = twid<INV>(y[3][3], make_float2(-kC, kS));
+#pragma unroll
+        for (int k1 = 0; k1 < 4; k1++) {
+            dft4<INV>(y[0][k1], y[1][k1], y[2][k1], y[3][k1]);
+#pragma unroll
+            for (int k2 = 0; k2 < 4; k2++) v[k1 + 4 * k2] = y[k2][k1];
+        }
+    }
+}
+
+template <int N>
+struct Line {
+    static constexpr int TL = 8;         // lanes per line
+    static constexpr int P = N / TL;     // points per lane
+    static constexpr int LPW = 32 / TL;  // lines per warp
+    static constexpr int NH = N / 2 + 1;
+    // n = 32: fewer points per lane than lanes, so two lanes share each
+    // second-stage transform (its even and odd outputs)
+    static constexpr bool PAIR = P < TL;
+    static constexpr int M2 = PAIR ? 1 : P / TL;  // second-stage DFTs per lane
+    // row pitch of a plane in shared memory: 2 modulo 16 complex words, so
+    // that a column's eight lanes and two adjacent columns hit all banks, and
+    // two rows hold a line of N
+    static constexpr int PITCH = NH + 1;
+    // where value (k1, n2) of a line sits during the exchange: rows of TL
+    // values, rotated so that both the writes (n2 across lanes) and the reads
+    // (k1 across lanes) spread over the banks
+    static __device__ __forceinline__ int slot(int k1, int n2) { return k1 * TL + ((n2 + k1) & (TL - 1)); }
+    // the frequency in v[j] of lane l
+    static __device__ __forceinline__ int freq(int j, int l) {
+        return PAIR ? (l >> 1) + P * (2 * j + (l & 1)) : l + TL * (j / TL) + P * (j % TL);
+    }
 };
 
-template <int R>
-__device__ __forceinline__ LaneTw lane_twiddles(int lane, const float2 *__restrict__ tw) {
-    LaneTw T;
-#pragma unroll
-    for (int s = 0; s < 5; s++) {
-        const int h = 16 >> s;
-        T.st[s] = __ldg(tw + (lane & (h - 1)) * (16 / h));
-    }
-    T.wn = R == 2 ? __ldg(tw + 32 + lane) : make_float2(1.f, 0.f);
-    return T;
+// times W_8^n (forward sign) or its conjugate, n = 0 .. 3 known at compile time
+template <bool INV>
+__device__ __forceinline__ float2 w8(float2 a, int n) {
+    constexpr float kR = 0.70710678118654752f;
+    return n == 0 ? a : (n == 1 ? twid<INV>(a, make_float2(kR, -kR)) : (n == 2 ? rot90<INV>(a)
+                                                                               : twid<INV>(a, make_float2(-kR, -kR))));
 }
 
-// forward (INV = false: W = exp(-2 pi i k / N)) or inverse (W conjugated)
-template <int R, bool INV>
-__device__ __forceinline__ void warp_fft(float2 (&v)[R], int lane, const LaneTw &T) {
-    if (R == 2) {
-        const float2 a = v[0], b = v[1];
-        v[0] = make_float2(a.x + b.x, a.y + b.y);
-        float2 w = T.wn;
-        if (INV) w.y = -w.y;
-        v[1] = cmul(make_float2(a.x - b.x, a.y - b.y), w);
+// buf(pos): the line's exchange buffer, N words that its lanes own; the
+// warp's lanes call together (idle lines carry zeros and touch no buffer)
+template <int N, class Buf>
+__device__ __forceinline__ void fft_line(float2 (&v)[Line<N>::P], int l, bool active, const float2 *__restrict__ tw,
+                                         Buf buf) {
+    using F = Line<N>;
+    dft<F::P, false>(v);
+#pragma unroll
+    for (int k1 = 1; k1 < F::P; k1++) v[k1] = cmul(v[k1], __ldg(tw + l * k1));
+    if (active)
+#pragma unroll
+        for (int k1 = 0; k1 < F::P; k1++) buf(F::slot(k1, l)) = v[k1];
+    __syncwarp();
+    if constexpr (F::PAIR) {
+        // X[k1 + P (2 j + h)] = DFT_P over n of W_8^(n h) (z[n] +- z[n + P])
+        if (active)
+#pragma unroll
+            for (int n = 0; n < F::P; n++) {
+                const float2 a = buf(F::slot(l >> 1, n)), b = buf(F::slot(l >> 1, n + F::P));
+                v[n] = l & 1 ? w8<false>(a - b, n) : a + b;
+            }
+        __syncwarp();
+        dft<F::P, false>(v);
+    } else {
+        if (active)
+#pragma unroll
+            for (int m = 0; m < F::M2; m++)
+#pragma unroll
+                for (int n2 = 0; n2 < F::TL; n2++) v[m * F::TL + n2] = buf(F::slot(l + F::TL * m, n2));
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < F::M2; m++) dft<F::TL, false>(v + m * F::TL);
     }
+}
+
+template <int N, class Buf>
+__device__ __forceinline__ void ifft_line(float2 (&v)[Line<N>::P], int l, bool active, const float2 *__restrict__ tw,
+                                          Buf buf) {
+    using F = Line<N>;
+    if constexpr (F::PAIR) {
+        // the even and the odd frequencies' transforms c_0, c_1 by two lanes;
+        // z[n2] = c_0[n2 mod P] + W_8^-n2 c_1[n2 mod P]
+        dft<F::P, true>(v);
+        if (active)
 #pragma unroll
-    for (int k1 = 0; k1 < R; k1++) {
+            for (int n = 0; n < F::P; n++) buf(F::slot(l >> 1, (l & 1) * F::P + n)) = v[n];
+        __syncwarp();
+        if (active) {
+            const float2 w = __ldg(tw + F::P * l);
 #pragma unroll
-        for (int s = 0; s < 5; s++) {
-            const int h = 16 >> s;
-            const float px = __shfl_xor_sync(0xffffffffu, v[k1].x, h);
-            const float py = __shfl_xor_sync(0xffffffffu, v[k1].y, h);
-            if ((lane & h) == 0) {
-                v[k1] = make_float2(v[k1].x + px, v[k1].y + py);
-            } else {
-                float2 w = T.st[s];
-                if (INV) w.y = -w.y;
-                v[k1] = cmul(make_float2(px - v[k1].x, py - v[k1].y), w);
+            for (int k1 = 0; k1 < F::P; k1++) {
+                const float2 c0 = buf(F::slot(k1, l & (F::P - 1))), c1 = buf(F::slot(k1, F::P + (l & (F::P - 1))));
+                v[k1] = twid<true>(c0 + twid<true>(c1, w), __ldg(tw + l * k1));
             }
         }
-    }
-}
-
-template <int R>
-__device__ __forceinline__ int fft_out_index(int k1, int lane) { return k1 + R * brev5(lane); }
-
-// Inverse transform of a line held the way warp_fft leaves its output (lane
-// l holds Y[k1 + R bitrev5(l)] in v[k1]): radix-2 decimation in time across
-// the lanes (stages h = 1 .. 16, twiddle W_2h^(lane mod h) conjugated, on
-// the bit-reversed positions), then for R = 2 the in-lane step y[l] = z0 +
-// W_N^-l z1, y[l + 32] = z0 - W_N^-l z1.  Lane l then holds y[32 r + l] in
-// v[r]: natural order, no permutation through shared memory.  Unnormalised.
-template <int R>
-__device__ __forceinline__ void warp_ifft_dit(float2 (&v)[R], int lane, const LaneTw &T) {
+        __syncwarp();
+    } else {
 #pragma unroll
-    for (int k1 = 0; k1 < R; k1++) {
+        for (int m = 0; m < F::M2; m++) {
+            dft<F::TL, true>(v + m * F::TL);
 #pragma unroll
-        for (int s = 4; s >= 0; s--) {
-            const int h = 16 >> s;
-            const float px = __shfl_xor_sync(0xffffffffu, v[k1].x, h);
-            const float py = __shfl_xor_sync(0xffffffffu, v[k1].y, h);
-            float2 w = T.st[s];
-            w.y = -w.y;
-            if ((lane & h) == 0) {
-                const float2 t = cmul(make_float2(px, py), w);
-                v[k1] = make_float2(v[k1].x + t.x, v[k1].y + t.y);
-            } else {
-                const float2 t = cmul(v[k1], w);
-                v[k1] = make_float2(px - t.x, py - t.y);
-            }
+            for (int n2 = 1; n2 < F::TL; n2++)
+                v[m * F::TL + n2] = twid<true>(v[m * F::TL + n2], __ldg(tw + (l + F::TL * m) * n2));
         }
+        if (active)
+#pragma unroll
+            for (int m = 0; m < F::M2; m++)
+#pragma unroll
+                for (int n2 = 0; n2 < F::TL; n2++) buf(F::slot(l + F::TL * m, n2)) = v[m * F::TL + n2];
+        __syncwarp();
+        if (active)
+#pragma unroll
+            for (int k1 = 0; k1 < F::P; k1++) v[k1] = buf(F::slot(k1, l));
+        __syncwarp();
     }
-    if (R == 2) {
-        float2 w = T.wn;
-        w.y = -w.y;
-        const float2 z0 = v[0];
-        const float2 t = cmul(v[R - 1], w);
-        v[0] = make_float2(z0.x + t.x, z0.y + t.y);
-        v[R - 1] = make_float2(z0.x - t.x, z0.y - t.y);
-    }
+    dft<F::P, true>(v);
 }
 
-// plane kernels: kFftPlaneWarps warps per block, fixed at compile time so a
-// warp's line loop has a constant trip count and, for the small meshes,
-// unrolls (the lines' loads are in flight together)
-constexpr int kFftPlaneWarps = 16;
+// threads per block of the plane kernels: forward, one line per group for the
+// n/2 row pairs and (a warp more) the n/2+1 columns; inverse, the 2 (n/2+1)
+// columns of part 0 in one round (two at n = 128)
+template <int N>
+constexpr int kZyThreads = N / 2 * Line<N>::TL + 32;
+template <int N>
+constexpr int kYzThreads = N == 32 ? 288 : 544;
 
-template <int R>
-__global__ void __launch_bounds__(kFftPlaneWarps * 32) k_fft_zy(const FFTArgs a0, const FFTArgs *__restrict__ tab) {
-    extern __shared__ float2 plane[];  // [n][n/2+1]
-    constexpr int N = 32 * R, NH = N / 2 + 1;
-    constexpr int nw = kFftPlaneWarps, UNR = R <= 2 ? 4 : 1;
+template <int N>
+__global__ void __launch_bounds__(kZyThreads<N>) k_fft_zy(const FFTArgs a0, const FFTArgs *__restrict__ tab) {
+    extern __shared__ float2 plane[];  // [n][PITCH]
+    using F = Line<N>;
+    constexpr int TL = F::TL, P = F::P, NH = F::NH, PITCH = F::PITCH;
     pdl_wait();
     const FFTArgs A = tab ? tab[blockIdx.y] : a0;  // batched replicas: blockIdx.y
     const int x = blockIdx.x;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const LaneTw T = lane_twiddles<R>(lane, A.tw);
-#pragma unroll UNR
-    for (int y = w; y < N; y += nw) {
-        float2 v[R];
-        const float *line = A.rho + ((size_t)x * N + y) * N;
+    const int l = threadIdx.x % TL, line = threadIdx.x / TL;
+    {
+        // rows 2 line and 2 line + 1 as one complex line
+        const bool active = line < N / 2;
+        float2 v[P];
+        const float *r0 = A.rho + ((size_t)x * N + 2 * (active ? line : 0)) * N + l;
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = make_float2(line[32 * r + lane], 0.f);
-        warp_fft<R, false>(v, lane, T);
+        for (int n1 = 0; n1 < P; n1++) v[n1] = make_float2(__ldg(r0 + TL * n1), __ldg(r0 + N + TL * n1));
+        float2 *const row = plane + 2 * (active ? line : 0) * PITCH;
+        auto buf = [&](int pos) -> float2 & { return row[pos]; };
+        fft_line<N>(v, l, active, A.tw, buf);
+        if (active)
 #pragma unroll
-        for (int k1 = 0; k1 < R; k1++) {
-            const int k = fft_out_index<R>(k1, lane);
-            if (k < NH) plane[y * NH + k] = v[k1];
+            for (int j = 0; j < P; j++) row[F::freq(j, l)] = v[j];
+        __syncwarp();
+        // Z = FFT(a + i b): A = (Z[k] + conj Z[-k]) / 2, B = (Z[k] - conj Z[-k]) / 2i
+        constexpr int H = P / 2;  // k = l, l + TL, ..., below n/2, and n/2 itself by lane 0
+        float2 a[H + 1], b[H + 1];
+#pragma unroll
+        for (int i = 0; i <= H; i++) {
+            const int k = l + TL * i;
+            const float2 p = active && k < NH ? row[k] : make_float2(0.f, 0.f);
+            const float2 q = active && k < NH ? row[(N - k) & (N - 1)] : make_float2(0.f, 0.f);
+            a[i] = make_float2(0.5f * (p.x + q.x), 0.5f * (p.y - q.y));
+            b[i] = make_float2(0.5f * (p.y + q.y), 0.5f * (q.x - p.x));
         }
+        __syncwarp();
+        if (active)
+#pragma unroll
+            for (int i = 0; i <= H; i++) {
+                const int k = l + TL * i;
+                if (k < NH) {
+                    row[k] = a[i];
+                    row[PITCH + k] = b[i];
+                }
+            }
     }
     __syncthreads();
-#pragma unroll UNR
-    for (int kz = w; kz < NH; kz += nw) {
-        float2 v[R];
+    {
+        const bool active = line < NH;
+        const int kz = active ? line : 0;
+        float2 v[P];
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = plane[(32 * r + lane) * NH + kz];
-        warp_fft<R, false>(v, lane, T);
+        for (int n1 = 0; n1 < P; n1++)
+            v[n1] = active ? plane[(TL * n1 + l) * PITCH + kz] : make_float2(0.f, 0.f);
+        __syncwarp();
+        auto buf = [&](int pos) -> float2 & { return plane[pos * PITCH + kz]; };
+        fft_line<N>(v, l, active, A.tw, buf);
+        float2 *out = A.mid1 + ((size_t)x * NH + kz) * N;
+        if (active)
 #pragma unroll
-        for (int k1 = 0; k1 < R; k1++) {
-            const int ky = fft_out_index<R>(k1, lane);
-            A.mid1[((size_t)x * NH + kz) * N + ky] = v[k1];  // a column's 64 ky in one 512-byte row
-        }
+            for (int j = 0; j < P; j++) out[F::freq(j, l)] = v[j];
     }
 }
 
-template <int R>
-__global__ void __launch_bounds__(256) k_fft_xe(const FFTArgs a0, const FFTArgs *__restrict__ tab) {
-    constexpr int N = 32 * R, NH = N / 2 + 1;
+constexpr int kXeWarps = 2;
+
+template <int N>
+__global__ void __launch_bounds__(kXeWarps * 32) k_fft_xe(const FFTArgs a0, const FFTArgs *__restrict__ tab) {
+    using F = Line<N>;
+    constexpr int TL = F::TL, P = F::P, NH = F::NH, LPW = F::LPW;
+    __shared__ float2 sh[kXeWarps][N * LPW];
     pdl_wait();
     const FFTArgs A = tab ? tab[blockIdx.y] : a0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int line_id = blockIdx.x * (blockDim.x >> 5) + w;
-    if (line_id >= N * NH) return;  // warp-uniform; no block barrier below
-    const LaneTw T = lane_twiddles<R>(lane, A.tw);
-    const int ky = line_id / NH, kz = line_id % NH;
-    const size_t stride = (size_t)N * NH;
-    const size_t base = (size_t)ky * NH + kz;
-    float2 v[R];
+    const int task = blockIdx.x * kXeWarps + w;
+    if (task >= NH * (N / LPW)) return;  // warp-uniform; no block barrier below
+    const int sub = lane % LPW, l = lane / LPW;
+    const int kz = task / (N / LPW), ky = task % (N / LPW) * LPW + sub;
+    float2 *const line = sh[w];
+    auto buf = [&](int pos) -> float2 & { return line[pos * LPW + sub]; };
+    const size_t at = (size_t)kz * N + ky;
+    constexpr size_t stride = (size_t)NH * N;
+    float2 q[P];
 #pragma unroll
-    for (int r = 0; r < R; r++) v[r] = A.mid1[(32 * r + lane) * stride + (size_t)kz * N + ky];
-    warp_fft<R, false>(v, lane, T);
-    const float kyv = A.tpl.y * (float)(ky > N / 2 ? ky - N : ky);
-    const float kzv = A.tpl.z * (float)kz;
-    float2 e[3][R];
+    for (int n1 = 0; n1 < P; n1++) q[n1] = A.mid1[(TL * n1 + l) * stride + at];
+    float G[P];
 #pragma unroll
-    for (int k1 = 0; k1 < R; k1++) {
-        const int kx = fft_out_index<R>(k1, lane);
-        const float kxv = A.tpl.x * (float)(kx > N / 2 ? kx - N : kx);
-        const float G = __ldg(A.green + (size_t)kx * stride + base);
-        const float2 q = v[k1];
-        const float gx = (2 * kx == N) ? 0.f : kxv * G;
-        const float gy = (2 * ky == N) ? 0.f : kyv * G;
-        const float gz = (2 * kz == N) ? 0.f : kzv * G;
-        e[0][k1] = make_float2(-gx * q.y, gx * q.x);
-        e[1][k1] = make_float2(-gy * q.y, gy * q.x);
-        e[2][k1] = make_float2(-gz * q.y, gz * q.x);
-    }
-    // the inverse x transforms take the forward's bit-reversed layout as it
-    // stands and leave natural order
+    for (int j = 0; j < P; j++) G[j] = __ldg(A.green + F::freq(j, l) * stride + at);
+    fft_line<N>(q, l, true, A.tw, buf);
+    const float kyv = 2 * ky == N ? 0.f : A.tpl.y * (float)(ky > N / 2 ? ky - N : ky);
+    const float kzv = 2 * kz == N ? 0.f : A.tpl.z * (float)kz;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        float2 u[R];
+        float2 u[P];
 #pragma unroll
-        for (int k1 = 0; k1 < R; k1++) u[k1] = e[d][k1];
-        warp_ifft_dit<R>(u, lane, T);
-        float2 *out = A.mid2 + (size_t)d * N * stride;
+        for (int j = 0; j < P; j++) {
+            const int kx = F::freq(j, l);
+            const float kxv = 2 * kx == N ? 0.f : A.tpl.x * (float)(kx > N / 2 ? kx - N : kx);
+            const float g = (d == 0 ? kxv : (d == 1 ? kyv : kzv)) * G[j];
+            u[j] = make_float2(-g * q[j].y, g * q[j].x);
+        }
+        ifft_line<N>(u, l, true, A.tw, buf);
+        float2 *out = A.mid2 + (size_t)d * N * stride + at;
 #pragma unroll
-        for (int r = 0; r < R; r++) out[(32 * r + lane) * stride + (size_t)kz * N + ky] = u[r];
+        for (int n1 = 0; n1 < P; n1++) out[(TL * n1 + l) * stride] = u[n1];
     }
 }
 
-// one block per (x plane, field component): inverse along y for every kz,
-// then the real inverse along z; component d of the float4 field is written
-template <int R>
-__global__ void __launch_bounds__(kFftPlaneWarps * 32) k_ifft_yz(const FFTArgs a0, const FFTArgs *__restrict__ tab) {
-    extern __shared__ float2 plane[];  // [n][n/2+1]
-    constexpr int N = 32 * R, NH = N / 2 + 1;
-    constexpr int nw = kFftPlaneWarps, UNR = R <= 2 ? 4 : 1;
-    pdl_wait();
-    const FFTArgs A = tab ? tab[blockIdx.z] : a0;  // batched replicas: blockIdx.z
-    const int x = blockIdx.x, d = blockIdx.y;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const LaneTw T = lane_twiddles<R>(lane, A.tw);
-    const size_t stride = (size_t)N * NH;
-    const float2 *src0 = A.mid2 + (size_t)d * N * stride + (size_t)x * stride;
-#pragma unroll UNR
-    for (int kz = w; kz < NH; kz += nw) {
-        float2 v[R];
+// one block per (x plane, part): part 0 the components x and y, part 1 z.
+// Along z, a line of a + i b from the half spectra of two real rows a and b,
+// extended by X[n - k] = conj X[k]: (Ex, Ey) of a row, or Ez of two rows
+template <int N, int D>
+__device__ __forceinline__ void ifft_yz_part(const FFTArgs &A, float2 *plane) {
+    using F = Line<N>;
+    constexpr int TL = F::TL, P = F::P, NH = F::NH, PITCH = F::PITCH;
+    constexpr int kLines = kYzThreads<N> / TL;
+    constexpr int kRoundsY = (D * NH + kLines - 1) / kLines;
+    constexpr int kLinesZ = D == 2 ? N : N / 2, kRoundsZ = (kLinesZ + kLines - 1) / kLines;
+    const int x = blockIdx.x;
+    const int l = threadIdx.x % TL, line = threadIdx.x / TL;
+    constexpr size_t stride = (size_t)NH * N;
+#pragma unroll 1
+    for (int r = 0; r < kRoundsY; r++) {
+        const int t = line + r * kLines;
+        const bool active = t < D * NH;
+        const int d = active ? t / NH : 0, kz = active ? t % NH : 0;
+        float2 v[P];
+        const float2 *src = A.mid2 + ((size_t)(D == 2 ? d : 2) * N + x) * stride + (size_t)kz * N;
 #pragma unroll
-        for (int r = 0; r < R; r++) v[r] = src0[(size_t)kz * N + 32 * r + lane];  // one contiguous ky row
-        warp_fft<R, true>(v, lane, T);
+        for (int j = 0; j < P; j++) v[j] = src[F::freq(j, l)];
+        float2 *const col = plane + (size_t)d * N * PITCH + kz;
+        auto buf = [&](int pos) -> float2 & { return col[pos * PITCH]; };
+        ifft_line<N>(v, l, active, A.tw, buf);
+        if (active)
 #pragma unroll
-        for (int k1 = 0; k1 < R; k1++) plane[fft_out_index<R>(k1, lane) * NH + kz] = v[k1];
+            for (int n1 = 0; n1 < P; n1++) col[(TL * n1 + l) * PITCH] = v[n1];
     }
     __syncthreads();
-    float *e = reinterpret_cast<float *>(A.e4) + d;
-#pragma unroll UNR
-    for (int y = w; y < N; y += nw) {
-        const float2 *row = plane + y * NH;
-        // the Hermitian half spectrum read in the bit-reversed order the
-        // decimation-in-time inverse takes; the line comes out in natural
-        // order (consecutive lanes, consecutive points)
-        float2 v[R];
+#pragma unroll 1
+    for (int r = 0; r < kRoundsZ; r++) {
+        const int t = line + r * kLines;
+        const bool active = t < kLinesZ;
+        // D = 2: row t of both planes; D = 1: rows 2t and 2t + 1
+        float2 *const ra = plane + (size_t)(active ? (D == 2 ? t : 2 * t) : 0) * PITCH;
+        float2 *const rb = ra + (D == 2 ? (size_t)N * PITCH : (size_t)PITCH);
+        float2 v[P];
 #pragma unroll
-        for (int k1 = 0; k1 < R; k1++) {
-            const int n = fft_out_index<R>(k1, lane);
-            float2 X;
-            if (n == 0 || n == N / 2) {
-                X = make_float2(row[n].x, 0.f);
-            } else if (n < N / 2) {
-                X = row[n];
-            } else {
-                const float2 c = row[N - n];
-                X = make_float2(c.x, -c.y);
+        for (int j = 0; j < P; j++) {
+            const int k = F::freq(j, l), kk = k <= N / 2 ? k : N - k;
+            float2 a = active ? ra[kk] : make_float2(0.f, 0.f), b = active ? rb[kk] : make_float2(0.f, 0.f);
+            if (k == 0 || k == N / 2) a.y = b.y = 0.f;
+            if (k > N / 2) {
+                a.y = -a.y;
+                b.y = -b.y;
             }
-            v[k1] = X;
+            v[j] = make_float2(a.x - b.y, a.y + b.x);
         }
-        warp_ifft_dit<R>(v, lane, T);
-        const size_t base = ((size_t)x * N + y) * N;
+        __syncwarp();
+        // the two rows' words are the exchange buffer: one half line in each
+        auto buf = [&](int pos) -> float2 & { return pos < N / 2 ? ra[pos] : rb[pos - N / 2]; };
+        ifft_line<N>(v, l, active, A.tw, buf);
+        if (!active) continue;  // no warp barrier below
+        float *out = reinterpret_cast<float *>(A.e4 + ((size_t)x * N + (D == 2 ? t : 2 * t)) * N + l);
+        if (D == 2) {
 #pragma unroll
-        for (int r = 0; r < R; r++) e[4 * (base + 32 * r + lane)] = v[r].x;
+            for (int n1 = 0; n1 < P; n1++) *reinterpret_cast<float2 *>(out + 4 * TL * n1) = v[n1];
+        } else {
+#pragma unroll
+            for (int n1 = 0; n1 < P; n1++) {
+                out[4 * TL * n1 + 2] = v[n1].x;
+                out[4 * (N + TL * n1) + 2] = v[n1].y;
+            }
+        }
     }
 }
 
-// gather on the interleaved field, five lanes per atom (six atoms per warp):
-// lane t sums the 25 points of stencil plane a = t with one 16-byte load per
-// point; the five partial fields are added with shuffles
-// the field at atom i's stencil plane a = t, weighted (one lane's share)
-__device__ __forceinline__ float3 gather_plane(const P3MArgs &A, const float4 *__restrict__ e4, int i, int t) {
-    const P3MGeom &g = A.g;
-    int3 ng;
-    float3 d;
-    stencil(g, A.xs[i], ng, d);
-    float wx[5], wy[5], wz[5];
-    w5(d.x, wx);
-    w5(d.y, wy);
-    w5(d.z, wz);
-    int pz[5];
-#pragma unroll
-    for (int c = 0; c < 5; c++) pz[c] = wrapi(ng.z + c - 2, g.sz.z);
-    const int px = wrapi(ng.x + t - 2, g.sz.x);
-    const float wa = pick5(wx, t);
-    float ex = 0.f, ey = 0.f, ez = 0.f;
-#pragma unroll
-    for (int b = 0; b < 5; b++) {
-        const int py = wrapi(ng.y + b - 2, g.sz.y);
-        const size_t row = ((size_t)px * g.sz.y + py) * g.sz.z;
-        const float wab = wa * wy[b];
+template <int N>
+__global__ void __launch_bounds__(kYzThreads<N>) k_ifft_yz(const FFTArgs a0, const FFTArgs *__restrict__ tab) {
+    extern __shared__ float2 plane[];  // [2][n][PITCH]
+    pdl_wait();
+    const FFTArgs A = tab ? tab[blockIdx.z] : a0;  // batched replicas: blockIdx.z
+    if (blockIdx.y == 0) ifft_yz_part<N, 2>(A, plane);
+    else ifft_yz_part<N, 1>(A, plane);
+}
+
+// the three kernels for one system (a0) or the nrep systems of tab
+template <int N, class Launch>
+void launch_solve(Launch launch, unsigned nrep) {
+    using F = Line<N>;
+    constexpr size_t row = (size_t)N * F::PITCH * sizeof(float2);
+    launch(k_fft_zy<N>, dim3(N, nrep), dim3(kZyThreads<N>), row);
+    launch(k_fft_xe<N>, dim3((F::NH * (N / F::LPW) + kXeWarps - 1) / kXeWarps, nrep), dim3(kXeWarps * 32), (size_t)0);
+    launch(k_ifft_yz<N>, dim3(N, 2, nrep), dim3(kYzThreads<N>), 2 * row);
+}
+
+// Gather on the interleaved field: a warp takes three charges -- the charged
+// sites of one molecule (MOL; no lane is spent on an uncharged oxygen) or
+// three consecutive atoms.  Lane 3 s + d works out charge s's stencil along
+// dimension d once, into shared memory; then a charge's 125 points go over
+// the lanes in mesh order (four 16-byte loads a lane, the twelve of the three
+// charges in flight), so that a load instruction reads runs of 80 bytes and
+// touches about 8 lines; the nine sums are butterflied.  What bounds it is the
+// L2's bandwidth: 75 rows of 80 bytes per molecule, 34 MB at 4,096 molecules.
+// A lane per stencil plane, the layout before, touched one 32-byte sector
+// per point (49 MB): gather stage of 8,000 atoms on 32^3 12.8 -> 10.8 us, of
+// 32,768 molecules on 128^3 (planar fields then, one thread per site) with the
+// chain, see own_solve.  Neighbouring molecules go to one block for its L1.
+// MOL: stored into a per-step buffer, the uncharged oxygen of a four-site
+// molecule as zero; otherwise stored into (ACC: added to) the forces, whose .w
+// is kept.  Batched replicas (blockIdx.y): each its own field.
+constexpr int kMeshWarps = 4;  // warps per block
+
+struct Stencil {
+    float wx[3][5], wy[3][5], wz[3][5];  // weights
+    int ox[3][5], oy[3][5], pz[3][5];    // offset of plane a, of row b within it, index of point c
+    float q[3];
+};
+
+template <bool MOL>
+__device__ __forceinline__ int unit_atom(const P3MArgs &A, int u, int s) {
+    if (MOL) return mol_site(mol_atoms(A, u), s, A.four_site);
+    return 3 * u + s < A.n ? 3 * u + s : -1;
+}
+template <bool MOL>
+__host__ __device__ __forceinline__ int mesh_units(int n, int nmol) {
+    return MOL ? nmol : (n + 2) / 3;
+}
+template <bool MOL>
+unsigned mesh_blocks(int n, int nmol) {
+    return (unsigned)((mesh_units<MOL>(n, nmol) + kMeshWarps - 1) / kMeshWarps);
+}
+
+template <bool MOL, bool ACC>
+__global__ void __launch_bounds__(kMeshWarps * 32) k_gather4(const P3MArgs a0, const P3MArgs *__restrict__ tab) {
+    __shared__ Stencil sh[kMeshWarps];
+    pdl_wait();
+    MDX_P3M_ARGS;
+    const int u = blockIdx.x * kMeshWarps + (threadIdx.x >> 5);
+    if (u >= mesh_units<MOL>(A.n, A.nmol)) return;  // warp-uniform
+    const int lane = threadIdx.x & 31;
+    Stencil &S = sh[threadIdx.x >> 5];
+    if (lane < 9) {
+        const int s = lane / 3, d = lane % 3;
+        const int i = unit_atom<MOL>(A, u, s);
+        const P3MGeom &g = A.g;
+        const float h = d == 0 ? g.h.x : (d == 1 ? g.h.y : g.h.z);
+        const float lo = d == 0 ? g.lo.x : (d == 1 ? g.lo.y : g.lo.z);
+        const int n = d == 0 ? g.sz.x : (d == 1 ? g.sz.y : g.sz.z);
+        const float p = (i >= 0 ? reinterpret_cast<const float *>(A.xs)[4 * (size_t)i + d] : lo) - lo;
+        const int ng = (int)floorf((p + 0.5f * h) / h);
+        float w[5];
+        w5(p / h - (float)ng, w);
+        float *const ws = d == 0 ? S.wx[s] : (d == 1 ? S.wy[s] : S.wz[s]);
+        int *const os = d == 0 ? S.ox[s] : (d == 1 ? S.oy[s] : S.pz[s]);
+        const int stride = d == 0 ? g.sz.y * g.sz.z : (d == 1 ? g.sz.z : 1);
 #pragma unroll
         for (int c = 0; c < 5; c++) {
-            const float w = wab * wz[c];
-            const float4 e = __ldg(e4 + row + pz[c]);
-            ex += w * e.x;
-            ey += w * e.y;
-            ez += w * e.z;
+            ws[c] = w[c];
+            os[c] = wrapi(ng + c - 2, n) * stride;
+        }
+        if (d == 0) S.q[s] = i >= 0 ? A.qs[i] : 0.f;
+    }
+    __syncwarp();
+    float3 e[3];
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+        e[s] = make_float3(0.f, 0.f, 0.f);
+        if (S.q[s] == 0.f) continue;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int t = 32 * k + lane;
+            if (t < 125) {
+                const int r = t / 5, c = t % 5, a = r / 5, b = r % 5;
+                const float w = S.wx[s][a] * S.wy[s][b] * S.wz[s][c];
+                const float4 v = __ldg(A.e4 + (S.ox[s][a] + S.oy[s][b] + S.pz[s][c]));
+                e[s].x += w * v.x;
+                e[s].y += w * v.y;
+                e[s].z += w * v.z;
+            }
         }
     }
-    return make_float3(ex, ey, ez);
-}
-
-// sum over the five lanes base .. base + 4 (valid in lane base); the whole
-// warp takes part
-__device__ __forceinline__ float3 group5_sum(float3 e, int base) {
-    float3 s = e;
 #pragma unroll
-    for (int k = 1; k < 5; k++) {
-        const int src = (base + k) & 31;
-        s.x += __shfl_sync(0xffffffffu, e.x, src);
-        s.y += __shfl_sync(0xffffffffu, e.y, src);
-        s.z += __shfl_sync(0xffffffffu, e.z, src);
+    for (int s = 0; s < 3; s++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            e[s].x += __shfl_xor_sync(0xffffffffu, e[s].x, o);
+            e[s].y += __shfl_xor_sync(0xffffffffu, e[s].y, o);
+            e[s].z += __shfl_xor_sync(0xffffffffu, e[s].z, o);
+        }
     }
-    return s;
-}
-
-template <bool ACC>
-__device__ __forceinline__ void gather4_body(const P3MArgs &A, const float4 *__restrict__ e4) {
-    const int lane = threadIdx.x & 31;
-    const int t = lane % 5, base = lane - t;
-    const int i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 6 + lane / 5;
-    const bool valid = lane < 30 && i < A.n;
-    const float q = valid ? A.qs[i] : 0.f;
-    const float3 e = q != 0.f ? gather_plane(A, e4, i, t) : make_float3(0.f, 0.f, 0.f);
-    const float3 sm = group5_sum(e, base);
-    if (!valid || t != 0) return;
-    float4 *__restrict__ fs = A.fs;
-    float4 f = fs[i];
-    if (q == 0.f) {
-        if (!ACC) fs[i] = make_float4(0.f, 0.f, 0.f, f.w);
-        return;
-    }
+    if (MOL && lane == 3 && A.four_site) A.fs[mol_atoms(A, u).x] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (lane >= 3) return;
+    const int i = unit_atom<MOL>(A, u, lane);
+    const float q = S.q[lane];
+    if (i < 0 || (ACC && q == 0.f)) return;
+    const float3 m = lane == 0 ? e[0] : (lane == 1 ? e[1] : e[2]);
     const float s = A.g.qunit * q * A.niv;
+    float4 f = MOL ? make_float4(0.f, 0.f, 0.f, 0.f) : A.fs[i];
     if (ACC) {
-        f.x += s * sm.x;
-        f.y += s * sm.y;
-        f.z += s * sm.z;
+        f.x += s * m.x;
+        f.y += s * m.y;
+        f.z += s * m.z;
     } else {
-        f.x = s * sm.x;
-        f.y = s * sm.y;
-        f.z = s * sm.z;
+        f.x = s * m.x;
+        f.y = s * m.y;
+        f.z = s * m.z;
     }
-    fs[i] = f;
-}
-
-template <bool ACC>
-__global__ void k_gather4(const P3MArgs A, const float4 *__restrict__ e4) {
-    pdl_wait();
-    gather4_body<ACC>(A, e4);
-}
-
-// batched replicas (blockIdx.y = replica), each with its own field
-template <bool ACC>
-__global__ void k_gather4_tab(const P3MArgs a0, const P3MArgs *__restrict__ tab) {
-    MDX_P3M_ARGS;
-    if ((blockIdx.x * blockDim.x >> 5) * 6 >= (unsigned)A.n) return;  // past this replica's atoms
-    gather4_body<ACC>(A, A.e4);
-}
-
-// the molecule form of the gather into a per-step buffer (STORE): the
-// mapping of k_spread_mol, each charged site's force stored, the uncharged
-// oxygen of a four-site molecule stored as zero
-__global__ void k_gather_mol(const P3MArgs a0, const P3MArgs *__restrict__ tab, const float4 *__restrict__ e4_one) {
-    pdl_wait();
-    MDX_P3M_ARGS;
-    const float4 *__restrict__ e4 = tab ? A.e4 : e4_one;  // batched: each replica's own field
-    const int lane = threadIdx.x & 31;
-    const int t = lane % 5, base = lane - t;
-    const int W = (A.nmol + 1) / 2;
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int m = (lane / 15) * W + w;
-    const bool valid = lane < 30 && w < W && m < A.nmol;
-    const int k = (lane % 15) / 5;
-    int4 ix = make_int4(0, 0, 0, 0);
-    int i = 0;
-    float q = 0.f;
-    if (valid) {
-        ix = A.slots ? make_int4(4 * m, 4 * m + 1, 4 * m + 2, 4 * m + 3) : A.mol_idx[m];
-        i = mol_site(ix, k, A.four_site);
-        q = A.qs[i];
-    }
-    const float3 e = q != 0.f ? gather_plane(A, e4, i, t) : make_float3(0.f, 0.f, 0.f);
-    const float3 sm = group5_sum(e, base);
-    if (!valid || t != 0) return;
-    const float s = A.g.qunit * q * A.niv;
-    A.fs[i] = make_float4(s * sm.x, s * sm.y, s * sm.z, 0.f);
-    if (A.four_site && k == 0) A.fs[ix.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+    A.fs[i] = f;
 }
 
 }  // namespace
@@ -809,7 +965,7 @@ double FixChargeEwald::findAlpha() {
 }
 
 namespace {
-template <int R>
+template <int N>
 int own_fft_setup();
 }  // namespace
 
@@ -840,22 +996,23 @@ int FixChargeEwald::prepareForRun() {
     }
     cufftSetStream(plan_r2c, s.stream);
     cufftSetStream(plan_c2r, s.stream);
-    // Green function on the half spectrum (Green_function_cu), on the device
-    if (int e = computeGreen(s.stream)) return e;
-    // own FFT for cubic 32^3 / 64^3 meshes (cuFFT for every other size)
     if (int e = f_recip.alloc(std::max(s.gpd.n, 1))) return e;
-    own_fft = sz.x == sz.y && sz.y == sz.z && (sz.x == 32 || sz.x == 64);
+    // own FFT for cubic 32^3, 64^3 and 128^3 meshes (cuFFT for every other
+    // size: two component planes of 256^3 exceed a block's shared memory)
+    own_fft = sz.x == sz.y && sz.y == sz.z && (sz.x == 32 || sz.x == 64 || sz.x == 128);
     if (own_fft) {
         if (int e = e4.alloc(ng)) return e;
-        if (int e = tw.alloc(96)) return e;
-        std::vector<float2> h(96);
-        for (int k = 0; k < 32; k++)
-            h[k] = make_float2((float)std::cos(-2.0 * M_PI * k / 32.0), (float)std::sin(-2.0 * M_PI * k / 32.0));
-        for (int k = 0; k < 64; k++)
-            h[32 + k] = make_float2((float)std::cos(-2.0 * M_PI * k / 64.0), (float)std::sin(-2.0 * M_PI * k / 64.0));
-        MDX_CUDA_TRY(cudaMemcpy(tw.p, h.data(), 96 * sizeof(float2), cudaMemcpyHostToDevice));
-        if (int e = sz.x == 64 ? own_fft_setup<2>() : own_fft_setup<1>()) return e;
+        if (int e = tw.alloc(sz.x)) return e;
+        std::vector<float2> h(sz.x);
+        for (int k = 0; k < sz.x; k++)
+            h[k] = make_float2((float)std::cos(-2.0 * M_PI * k / sz.x), (float)std::sin(-2.0 * M_PI * k / sz.x));
+        MDX_CUDA_TRY(cudaMemcpy(tw.p, h.data(), h.size() * sizeof(float2), cudaMemcpyHostToDevice));
+        if (int e = sz.x == 32 ? own_fft_setup<32>() : (sz.x == 64 ? own_fft_setup<64>() : own_fft_setup<128>()))
+            return e;
+        if (int e = green_own.alloc(nk)) return e;
     }
+    // Green function on the half spectrum (Green_function_cu), on the device
+    if (int e = computeGreen(s.stream)) return e;
     prepared = true;
     return 0;
 }
@@ -868,33 +1025,37 @@ FFTArgs fft_args(State &s, FixChargeEwald &f) {
     A.mid1 = f.rho_k.p;
     A.mid2 = f.e_k.p;
     A.e4 = f.e4.p;
-    A.green = f.green.p;
+    A.green = f.green_own.p;
     A.tw = f.tw.p;
     A.tpl = make_float3((float)(6.28318530717958647693 / s.box.Ld.x), (float)(6.28318530717958647693 / s.box.Ld.y),
                         (float)(6.28318530717958647693 / s.box.Ld.z));
     return A;
 }
 
-template <int R>
+// What bounds the three kernels is latency, a load, two or four line
+// transforms and a store each.  Solve stage (hot, one B200), before -> now:
+// 64^3 19.1 -> 11.3 us, 32^3 7.4 -> 6.2 us; 128^3, cuFFT and the E(k) kernel
+// before, whole chain with spread and gather 179 -> 134 us at 32,768 molecules
+// (there the spread's atomics and the gather's reads are two thirds).
+template <int N>
 int own_solve(State &s, FixChargeEwald &f, cudaStream_t st) {
-    constexpr int N = 32 * R, NH = N / 2 + 1;
     const FFTArgs A = fft_args(s, f);
-    // 512-thread plane blocks (measured +0.8 % per water step against 1024
-    // beside the pair kernel; 256 was slower)
-    const FFTArgs *nt = nullptr;
-    MDX_CUDA_TRY(launch_pdl_prio(true, k_fft_zy<R>, dim3(N), dim3(kFftPlaneWarps * 32), (size_t)N * NH * sizeof(float2), st, A, nt));
-    MDX_CUDA_TRY(launch_pdl_prio(true, k_fft_xe<R>, dim3((N * NH + 7) / 8), dim3(256), 0, st, A, nt));
-    MDX_CUDA_TRY(launch_pdl_prio(true, k_ifft_yz<R>, dim3(N, 3), dim3(kFftPlaneWarps * 32), (size_t)N * NH * sizeof(float2), st, A, nt));
+    cudaError_t err = cudaSuccess;
+    launch_solve<N>(
+        [&](auto kern, dim3 grid, dim3 block, size_t smem) {
+            const cudaError_t e = launch_pdl_prio(true, kern, grid, block, smem, st, A, (const FFTArgs *)nullptr);
+            if (e != cudaSuccess) err = e;
+        },
+        1);
+    MDX_CUDA_TRY(err);
     return 0;
 }
 
-template <int R>
+template <int N>
 int own_fft_setup() {
-    constexpr int N = 32 * R, NH = N / 2 + 1;
-    MDX_CUDA_TRY(cudaFuncSetAttribute(k_ifft_yz<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      N * NH * (int)sizeof(float2)));
-    MDX_CUDA_TRY(cudaFuncSetAttribute(k_fft_zy<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      N * NH * (int)sizeof(float2)));
+    constexpr int row = N * Line<N>::PITCH * (int)sizeof(float2);
+    MDX_CUDA_TRY(cudaFuncSetAttribute(k_fft_zy<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, row));
+    MDX_CUDA_TRY(cudaFuncSetAttribute(k_ifft_yz<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * row));
     return 0;
 }
 }  // namespace
@@ -904,7 +1065,9 @@ namespace {
 // (Green_function_cu, FixChargeEwald.cu:218-294), one thread per k, FP64:
 // sum over the aliasing images m within +-lim of the charge assignment
 // function's transform W^(2 order) and the reference force R(k_m)
-__global__ void k_green(int3 sz, double3 L, double alpha, int lim, float *__restrict__ green) {
+// (green_own, may be null: the same values as (kx, kz, ky), the own FFT's layout)
+__global__ void k_green(int3 sz, double3 L, double alpha, int lim, float *__restrict__ green,
+                        float *__restrict__ green_own) {
     const int nzh = sz.z / 2 + 1;
     const size_t nk = (size_t)sz.x * sz.y * nzh;
     const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -936,6 +1099,7 @@ __global__ void k_green(int3 sz, double3 L, double alpha, int lim, float *__rest
         val = s1 / (s2 * s2) / k2;
     }
     green[id] = (float)val;
+    if (green_own) green_own[((size_t)ix * nzh + iz) * sz.y + iy] = (float)val;
 }
 }  // namespace
 
@@ -945,7 +1109,8 @@ int FixChargeEwald::computeGreen(cudaStream_t st) {
     const double h[3] = {L[0] / sz.x, L[1] / sz.y, L[2] / sz.z};
     const int lim = (int)(alpha * std::pow(h[0] * h[1] * h[2], 1.0 / 3.0) / 3.14159 * std::sqrt(-std::log(10E-7))) + 1;
     const size_t nk = (size_t)sz.x * sz.y * (sz.z / 2 + 1);
-    k_green<<<(unsigned)((nk + 255) / 256), 256, 0, st>>>(sz, make_double3(L[0], L[1], L[2]), alpha, lim, green.p);
+    k_green<<<(unsigned)((nk + 255) / 256), 256, 0, st>>>(sz, make_double3(L[0], L[1], L[2]), alpha, lim, green.p,
+                                                          own_fft ? green_own.p : nullptr);
     MDX_LAUNCHED();
     MDX_CUDA_TRY(cudaGetLastError());
     return 0;
@@ -965,13 +1130,15 @@ int FixChargeEwald::spread(cudaStream_t st) {
     const size_t ng = (size_t)sz.x * sz.y * sz.z;
     MDX_CUDA_TRY(cudaMemsetAsync(rho.p, 0, ng * sizeof(float), st));
     MDX_CUDA_TRY(launch_pdl_prio(true, k_spread5, dim3((s.gpd.n + 47) / 48), dim3(256), 0, st, p3m_args(s, *this),
-                            (const P3MArgs *)nullptr));
+                                 (const P3MArgs *)nullptr));
     return 0;
 }
 
 int FixChargeEwald::solve(cudaStream_t st) {
     State &s = *state;
-    if (own_fft) return sz.x == 64 ? own_solve<2>(s, *this, st) : own_solve<1>(s, *this, st);
+    if (own_fft)
+        return sz.x == 32 ? own_solve<32>(s, *this, st)
+                          : (sz.x == 64 ? own_solve<64>(s, *this, st) : own_solve<128>(s, *this, st));
     const size_t nk = (size_t)sz.x * sz.y * (sz.z / 2 + 1);
     cufftSetStream(plan_r2c, st);
     cufftSetStream(plan_c2r, st);
@@ -992,12 +1159,9 @@ int FixChargeEwald::gather(bool accumulate, cudaStream_t st) {
     State &s = *state;
     const P3MArgs A = p3m_args(s, *this);
     if (own_fft) {
-        if (accumulate)
-            MDX_CUDA_TRY(launch_pdl_prio(true, k_gather4<true>, dim3((s.gpd.n + 47) / 48), dim3(256), 0, st, A,
-                                    (const float4 *)e4.p));
-        else
-            MDX_CUDA_TRY(launch_pdl_prio(true, k_gather4<false>, dim3((s.gpd.n + 47) / 48), dim3(256), 0, st, A,
-                                    (const float4 *)e4.p));
+        MDX_CUDA_TRY(launch_pdl_prio(true, accumulate ? k_gather4<false, true> : k_gather4<false, false>,
+                                     dim3(mesh_blocks<false>(s.gpd.n, 0)), dim3(kMeshWarps * 32), 0, st, A,
+                                     (const P3MArgs *)nullptr));
         return 0;
     }
     if (accumulate)
@@ -1013,8 +1177,8 @@ int FixChargeEwald::gather_to(float4 *out, cudaStream_t st) {
     P3MArgs A = p3m_args(s, *this);
     A.fs = out;
     if (own_fft) {
-        MDX_CUDA_TRY(launch_pdl_prio(true, k_gather4<false>, dim3((s.gpd.n + 47) / 48), dim3(256), 0, st, A,
-                                (const float4 *)e4.p));
+        MDX_CUDA_TRY(launch_pdl_prio(true, k_gather4<false, false>, dim3(mesh_blocks<false>(s.gpd.n, 0)),
+                                     dim3(kMeshWarps * 32), 0, st, A, (const P3MArgs *)nullptr));
     } else {
         k_gather<false><<<(s.gpd.n + 127) / 128, 128, 0, st>>>(A, nullptr);
         MDX_LAUNCHED();
@@ -1063,9 +1227,8 @@ int FixChargeEwald::gather_mol_to(float4 *out, cudaStream_t st, const FixRigid &
     State &s = *state;
     P3MArgs A = mol_args(s, *this, r);
     A.fs = out;
-    const int warps = (A.nmol + 1) / 2;
-    MDX_CUDA_TRY(launch_pdl_prio(true, k_gather_mol, dim3((warps + 1) / 2), dim3(64), 0, st, A,
-                                 (const P3MArgs *)nullptr, (const float4 *)e4.p));
+    MDX_CUDA_TRY(launch_pdl_prio(true, k_gather4<true, false>, dim3(mesh_blocks<true>(0, A.nmol)),
+                                 dim3(kMeshWarps * 32), 0, st, A, (const P3MArgs *)nullptr));
     return 0;
 }
 
@@ -1217,17 +1380,12 @@ int batch_p3m_spread_solve(Batch &b, cudaStream_t st) {
             const unsigned K = (unsigned)c->reps.size();
             const FFTArgs a0 = fft_args(*b.reps[c->reps[0]], *b.reps[c->reps[0]]->ewaldFix());
             const FFTArgs *ft = reinterpret_cast<const FFTArgs *>(c->tab.p);
-            const int N = c->sz.x, NH = N / 2 + 1;
-            const size_t smem = (size_t)N * NH * sizeof(float2);
-            if (N == 64) {
-                k_fft_zy<2><<<dim3(N, K), kFftPlaneWarps * 32, smem, st>>>(a0, ft);
-                k_fft_xe<2><<<dim3((N * NH + 7) / 8, K), 256, 0, st>>>(a0, ft);
-                k_ifft_yz<2><<<dim3(N, 3, K), kFftPlaneWarps * 32, smem, st>>>(a0, ft);
-            } else {
-                k_fft_zy<1><<<dim3(N, K), kFftPlaneWarps * 32, smem, st>>>(a0, ft);
-                k_fft_xe<1><<<dim3((N * NH + 7) / 8, K), 256, 0, st>>>(a0, ft);
-                k_ifft_yz<1><<<dim3(N, 3, K), kFftPlaneWarps * 32, smem, st>>>(a0, ft);
-            }
+            auto launch = [&](auto kern, dim3 grid, dim3 block, size_t smem) {
+                kern<<<grid, block, smem, st>>>(a0, ft);
+            };
+            if (c->sz.x == 32) launch_solve<32>(launch, K);
+            else if (c->sz.x == 64) launch_solve<64>(launch, K);
+            else launch_solve<128>(launch, K);
             g_launches += 3;
         }
         MDX_CUDA_TRY(cudaGetLastError());
@@ -1257,14 +1415,14 @@ int batch_p3m_gather(Batch &b, cudaStream_t st) {
     P3MArgs A = p3m_args(*b.reps[0], *b.reps[0]->ewaldFix());
     A.n = b.max_n;
     if (b.p3m_mol) {  // into each replica's per-step buffer (the second half adds it)
-        const int warps = (b.max_mol + 1) / 2;
-        k_gather_mol<<<dim3((warps + 1) / 2, (unsigned)b.reps.size()), 64, 0, st>>>(
-            A, reinterpret_cast<const P3MArgs *>(b.tab_p3m_mol.p), (const float4 *)nullptr);
+        k_gather4<true, false><<<dim3(mesh_blocks<true>(0, b.max_mol), (unsigned)b.reps.size()), kMeshWarps * 32, 0,
+                                 st>>>(A, reinterpret_cast<const P3MArgs *>(b.tab_p3m_mol.p));
         MDX_LAUNCHED();
         return 0;
     }
     if (b.p3m_own) {
-        k_gather4_tab<true><<<dim3((A.n + 47) / 48, (unsigned)b.reps.size()), 256, 0, st>>>(A, tab);
+        k_gather4<false, true><<<dim3(mesh_blocks<false>(A.n, 0), (unsigned)b.reps.size()), kMeshWarps * 32, 0, st>>>(
+            A, tab);
         MDX_LAUNCHED();
         return 0;
     }
