@@ -67,7 +67,7 @@ void Batch::reset() {
     }
     fft.clear();
     for (DBuf<char> *t : {&tab_pair, &tab_grid, &tab_grid_ps, &tab_build, &tab_p3m, &tab_e3b, &tab_first,
-                          &tab_second, &tab_molgrid, &tab_molscan, &tab_pairmol, &tab_p3m_mol})
+                          &tab_second, &tab_end, &tab_molgrid, &tab_molscan, &tab_pairmol, &tab_p3m_mol})
         t->release();
     max_n = max_mol = max_cell = 0;
     ps.clear();
@@ -219,9 +219,9 @@ int Batch::prepare() {
 
 // the fused step of IntegratorVerlet (P3M chain and E3B on side streams beside
 // the pair kernel) with every launch covering all replicas
-int Batch::step() {
+int Batch::step(bool early) {
     const bool e3b = reps[0]->e3bFix() != nullptr;
-    if (int e = batch_first_half(*this)) return e;
+    if (int e = batch_first_half(*this, early)) return e;
     MDX_CUDA_TRY(cudaEventRecord(ev_fork, stream));
     MDX_CUDA_TRY(cudaStreamWaitEvent(side[0], ev_fork, 0));
     if (int e = batch_p3m_spread_solve(*this, side[0])) return e;
@@ -245,7 +245,7 @@ int Batch::enqueue(int nsteps, bool with_group) {
     if (with_group)
         if (int e = batch_nlist_rebuild(*this)) return e;
     for (int k = 0; k < nsteps; k++)
-        if (int e = step()) return e;
+        if (int e = step(k > 0)) return e;
     return 0;
 }
 

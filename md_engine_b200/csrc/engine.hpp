@@ -535,7 +535,6 @@ class State {
     DeviceStatus *h_status = nullptr;  // pinned
     DBuf<double> red_partials;
     DBuf<double> red_out;
-    DBuf<unsigned int> red_counter;
     // per-site pair energies and their FP64 sum (energy evaluations outside
     // the step; sized at upload so that no evaluation allocates)
     DBuf<float> e_site;
@@ -598,7 +597,7 @@ class Batch {
     int periodicInterval = 10;
     int64_t turn = 0;
     // argument tables (device), one record per replica, built at prepare
-    DBuf<char> tab_pair, tab_grid, tab_build, tab_p3m, tab_e3b, tab_first, tab_second;
+    DBuf<char> tab_pair, tab_grid, tab_build, tab_p3m, tab_e3b, tab_first, tab_second, tab_end;
     // replicas by form: ps (per-site list) and mfi (molecule form); the pair
     // kernel and the rebuild group launch once per form over that form's
     // replicas (tab_grid: every replica, for the skin check; tab_grid_ps,
@@ -637,7 +636,7 @@ class Batch {
     ~Batch();
     int biggest_rep() const;
     int prepare();
-    int step();
+    int step(bool early);
     int enqueue(int nsteps, bool with_group);
     int launchGraph(int nsteps, bool with_group);
     int run(int nturns, double *ms);
@@ -662,7 +661,7 @@ int batch_p3m_spread_solve(Batch &b, cudaStream_t stream);
 int batch_p3m_gather(Batch &b, cudaStream_t stream);
 int batch_e3b_list(Batch &b);
 int batch_e3b_forces(Batch &b, cudaStream_t stream);
-int batch_first_half(Batch &b);
+int batch_first_half(Batch &b, bool early);
 int batch_second_half(Batch &b, bool with_e3b);
 int batch_rigid_maps(Batch &b);
 
@@ -701,7 +700,7 @@ int surrogate_forces_to(State &s, FixE3B &f, float4 *out, cudaStream_t stream);
 int surrogate_compute(State &s, FixE3B &f);
 // rigid + integration (integrate.cu)
 int rigid_update_maps(State &s, FixRigid &r, bool conditional);
-int step_first_half(State &s, bool fused);
+int step_first_half(State &s, bool fused, bool early = false);
 int step_second_half(State &s, bool fused, const float4 *fextra = nullptr, const float4 *frecip = nullptr);
 bool has_free_atoms(State &s);
 int rigid_prepare(State &s, FixRigid &r);

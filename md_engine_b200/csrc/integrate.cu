@@ -19,69 +19,85 @@ namespace mdx {
 // ---------------------------------------------------------------- NH chain
 // exp(x) for the chain's arguments, -dt/8 .. -dt/2 times a thermostat
 // velocity (|x| well below 1/64 for any stable run): the Taylor polynomial of
-// degree 8 (truncation below 1e-22 relative, under FP64 rounding) evaluated
-// by Estrin's scheme -- pairs of terms, then x^2, x^4, x^8 -- a dependent
-// depth of four multiply-adds on the device's serial tail instead of
-// Horner's nine; larger arguments use exp().  Host and device run the same
-// code.
-__host__ __device__ inline double nh_exp(double x) {
-    if (fabs(x) >= 0.015625) return exp(x);
+// degree 6 (truncation below 2^-42 / 5040 = 5e-17 relative, under half an ulp)
+// by Estrin's scheme, a dependent depth of three multiply-adds after x^2.  No
+// test of the argument here: nh_integrate_n looks at all of them at once.
+// Host and device run the same code.
+__host__ __device__ inline double nh_exp_small(double x) {
     const double x2 = x * x;
-    const double x4 = x2 * x2;
-    const double b0 = 1.0 + x;
-    const double b1 = fma(x, 1.0 / 6.0, 0.5);
-    const double b2 = fma(x, 1.0 / 120.0, 1.0 / 24.0);
-    const double b3 = fma(x, 1.0 / 5040.0, 1.0 / 720.0);
-    const double c0 = fma(x2, b1, b0);
-    const double c1 = fma(x2, b3, b2);
-    const double d0 = fma(x4, c1, c0);
-    return fma(x4 * x4, 1.0 / 40320.0, d0);
+    const double c0 = fma(x2, fma(x, 1.0 / 6.0, 0.5), 1.0 + x);
+    const double c1 = fma(x2, 1.0 / 720.0, fma(x, 1.0 / 120.0, 1.0 / 24.0));
+    return fma(x2 * x2, c1, c0);
 }
 
 // thermostatIntegrate (FixNoseHoover.cu:795-866), nTimesteps = n_ys = 1, for
 // a chain of compile-time length N (loops unrolled, so a chain held in
 // registers stays there); C has the fields of NHChain used here.  Divisions
-// by the chain masses are products with their reciprocals.
-template <int N, class C>
-__host__ __device__ __forceinline__ double nh_integrate_n(C &c, bool stepInit) {
-    const double nkt = c.ndf * c.kB * c.T;
-    if (!stepInit) c.force[0] = (c.ke - nkt) * c.inv_mass[0];
-    const double ts = c.dt;
-    const double t2 = 0.5 * ts, t4 = 0.25 * ts, t8 = 0.125 * ts;
+// by the chain masses are products with their reciprocals.  The factor of
+// link k, pf[k] = exp(-dt/8 v[k+1]), is the same in the downward and the
+// upward sweep (v[k+1] changes before the first and after the second), so
+// each is evaluated once.  nh_down: the downward sweep over the links above
+// the first and pf[0], which need no kinetic energy; nh_up: the rest.  SMALL:
+// the polynomial exponential; `most` collects the largest |argument|, and
+// the caller starts over with SMALL = false when it lies outside the range.
+template <int N, bool SMALL>
+__host__ __device__ __forceinline__ double nh_ex(double x, double &most) {
+    if (!SMALL) return exp(x);
+    most = fabs(x) <= most ? most : fabs(x);  // a NaN is kept
+    return nh_exp_small(x);
+}
+constexpr double kNHSmall = 0.015625;
+
+template <int N, bool SMALL, class C>
+__host__ __device__ __forceinline__ void nh_down(C &c, double (&pf)[N - 1], double &most) {
+    const double t4 = 0.25 * c.dt, t8 = 0.125 * c.dt;
     c.vel[N - 1] += t4 * c.force[N - 1];
 #pragma unroll
     for (int k = N - 2; k > 0; --k) {
-        double pf = nh_exp(-t8 * c.vel[k + 1]);
-        c.vel[k] *= pf;
-        c.vel[k] += t4 * c.force[k];
-        c.vel[k] *= pf;
+        pf[k] = nh_ex<N, SMALL>(-t8 * c.vel[k + 1], most);
+        c.vel[k] = fma(c.vel[k], pf[k], t4 * c.force[k]) * pf[k];
     }
-    double pf = nh_exp(-t8 * c.vel[1]);
-    c.vel[0] *= pf;
-    c.vel[0] += t4 * c.force[0];
-    c.vel[0] *= pf;
-    const double sf = nh_exp(-t2 * c.vel[0]);
+    pf[0] = nh_ex<N, SMALL>(-t8 * c.vel[1], most);
+}
+
+template <int N, bool SMALL, class C>
+__host__ __device__ __forceinline__ double nh_up(C &c, const double (&pf)[N - 1], bool stepInit, double &most) {
+    const double nkt = c.ndf * c.kB * c.T, kt = c.kB * c.T;
+    const double t2 = 0.5 * c.dt, t4 = 0.25 * c.dt;
+    if (!stepInit) c.force[0] = (c.ke - nkt) * c.inv_mass[0];
+    c.vel[0] = fma(c.vel[0], pf[0], t4 * c.force[0]) * pf[0];
+    const double sf = nh_ex<N, SMALL>(-t2 * c.vel[0], most);
     c.ke *= sf * sf;
-    c.vel[0] *= pf;
     c.force[0] = (c.ke - nkt) * c.inv_mass[0];
-    c.vel[0] += t4 * c.force[0];
-    c.vel[0] *= pf;
+    c.vel[0] = fma(c.vel[0], pf[0], t4 * c.force[0]) * pf[0];
 #pragma unroll
     for (int k = 1; k < N - 1; ++k) {
-        pf = nh_exp(-t8 * c.vel[k + 1]);
-        c.vel[k] *= pf;
-        c.force[k] = (c.mass[k - 1] * c.vel[k - 1] * c.vel[k - 1] - c.kB * c.T) * c.inv_mass[k];
-        c.vel[k] += t4 * c.force[k];
-        c.vel[k] *= pf;
+        c.force[k] = fma(c.mass[k - 1] * c.vel[k - 1], c.vel[k - 1], -kt) * c.inv_mass[k];
+        c.vel[k] = fma(c.vel[k], pf[k], t4 * c.force[k]) * pf[k];
     }
-    c.force[N - 1] = (c.mass[N - 2] * c.vel[N - 2] * c.vel[N - 2] - c.kB * c.T) * c.inv_mass[N - 1];
+    c.force[N - 1] = fma(c.mass[N - 2] * c.vel[N - 2], c.vel[N - 2], -kt) * c.inv_mass[N - 1];
     c.vel[N - 1] += t4 * c.force[N - 1];
     return sf;
 }
 
-// the chain has kNHChain links (FixNoseHoover's default chain length)
-__host__ __device__ double nh_integrate(NHChain &c, bool stepInit) {
-    return nh_integrate_n<kNHChain>(c, stepInit);
+template <int N, bool SMALL, class C>
+__host__ __device__ __forceinline__ double nh_half(C &c, bool stepInit, double &most) {
+    double pf[N - 1];
+    nh_down<N, SMALL>(c, pf, most);
+    return nh_up<N, SMALL>(c, pf, stepInit, most);
+}
+
+// one half step of the chain on the host (kNHChain links, FixNoseHoover's
+// default chain length)
+double nh_integrate(NHChain &c, bool stepInit) {
+    const NHChain c0 = c;
+    double most = 0.0;
+    double sf = nh_half<kNHChain, true>(c, stepInit, most);
+    if (!(most < kNHSmall)) {
+        c = c0;
+        sf = nh_half<kNHChain, false>(c, stepInit, most);
+    }
+    return sf;
 }
 
 // device copy: [0] = state after stepInit of the coming step ("next"),
@@ -246,10 +262,7 @@ struct MolArgs {
     NHChain *chain;
     DeviceStatus *st;
     double *partials;
-    int part_off, nparts;
-    unsigned int *counter;
-    int nh;
-    double *ke_out;
+    int part_off;
     const float4 *fextra;
     const float4 *frecip;  // P3M reciprocal forces of every site (may be null)
     int nblk;  // blocks of k_second_mol that carry this system's molecules
@@ -278,18 +291,25 @@ __global__ void k_rigid_maps(const MolArgs a0, const MolArgs *__restrict__ tab, 
 }
 
 // ---- first half ---------------------------------------------------------
+// early: the kernel before this one in the stream is k_step_end, behind whose
+// trigger every earlier kernel has completed and which writes no stream, so
+// the loads go ahead of its end; the first step after a rebuild group, or of
+// a captured chunk, waits first.
 // per-atom: NH rescale (rescale_no_tags_cu) + nve_v + nve_x (+ zero force)
 template <bool NH>
 __global__ void k_first_atoms(int n, float4 *__restrict__ xs, float4 *__restrict__ vs, float4 *__restrict__ fs,
                               const uint32_t *__restrict__ ids, const uint8_t *__restrict__ rigid_by_id, float dt,
-                              float dtf, const NHChain *__restrict__ chain) {
+                              float dtf, const NHChain *chain, int early) {
+    if (!early) pdl_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (rigid_by_id && rigid_by_id[ids[i]]) return;
     float4 v = vs[i];
     float4 f = fs[i];
+    float4 x = xs[i];
+    if (early) pdl_wait();
     if (NH) {
-        const float s = (float)chain[0].scale;
+        const float s = (float)__ldcg(&chain[0].scale);
         v.x *= s;
         v.y *= s;
         v.z *= s;
@@ -301,7 +321,6 @@ __global__ void k_first_atoms(int n, float4 *__restrict__ xs, float4 *__restrict
     }
     v = kick(v, f, dtf);
     vs[i] = v;
-    float4 x = xs[i];
     x.x += dt * v.x;
     x.y += dt * v.y;
     x.z += dt * v.z;
@@ -311,8 +330,9 @@ __global__ void k_first_atoms(int n, float4 *__restrict__ xs, float4 *__restrict
 
 // per-molecule fused: NH rescale + save_prev_val + nve_v + nve_x + SETTLE + M-site
 template <bool NH>
-__global__ void k_first_mol(const MolArgs a0, const MolArgs *__restrict__ tab) {
-    MDX_MOL_ARGS;
+__global__ void k_first_mol(const MolArgs a0, const MolArgs *__restrict__ tab, int early) {
+    if (!early) pdl_wait();
+    const MolArgs A = tab ? tab[blockIdx.y] : a0;
     int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= A.nmol) return;
     float4 *__restrict__ xs = A.xs;
@@ -321,11 +341,10 @@ __global__ void k_first_mol(const MolArgs a0, const MolArgs *__restrict__ tab) {
     const RigidConsts &rc = A.rc;
     const Box &box = A.box;
     const float dt = A.dt, dtf = A.dtf;
-    const NHChain *__restrict__ chain = A.chain;
     DeviceStatus *st = A.st;
     const int4 ix = mol_sites(A, m);
     const int id3[3] = {ix.x, ix.y, ix.z};
-    float4 x0[3], x[3], v[3];
+    float4 x0[3], x[3], v[3], f[3];
     // the M site's words read with the rest, not after the SETTLE
     float vmw = 0.f, fmw = 0.f, xmw = 0.f;
     if (rc.foursite) {
@@ -333,20 +352,24 @@ __global__ void k_first_mol(const MolArgs a0, const MolArgs *__restrict__ tab) {
         fmw = fs[ix.w].w;
         xmw = xs[ix.w].w;
     }
-    const float s = NH ? (float)chain[0].scale : 1.0f;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         x0[k] = xs[id3[k]];
         v[k] = vs[id3[k]];
-        const float4 f = fs[id3[k]];
+        f[k] = fs[id3[k]];
+    }
+    if (early) pdl_wait();
+    const float s = NH ? (float)__ldcg(&A.chain[0].scale) : 1.0f;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
         if (NH) {
             v[k].x *= s;
             v[k].y *= s;
             v[k].z *= s;
         }
-        v[k] = kick(v[k], f, dtf);
+        v[k] = kick(v[k], f[k], dtf);
         x[k] = make_float4(x0[k].x + dt * v[k].x, x0[k].y + dt * v[k].y, x0[k].z + dt * v[k].z, x0[k].w);
-        fs[id3[k]] = make_float4(0.f, 0.f, 0.f, f.w);
+        fs[id3[k]] = make_float4(0.f, 0.f, 0.f, f[k].w);
     }
     settle_pos(rc, box, (double)dt, x0, x, v, st);
 #pragma unroll
@@ -378,11 +401,25 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return r;  // valid in thread 0
 }
 
-// the time-dependent part of a chain, held in registers by the last block
+// the time-dependent part of a chain, held in registers
 struct NHRegs {
     double vel[kNHChain], force[kNHChain], mass[kNHChain], inv_mass[kNHChain];
     double ke, ndf, kB, T, dt;
 };
+
+__device__ __forceinline__ void load_chain(NHRegs &c, const NHChain &g) {
+#pragma unroll
+    for (int k = 0; k < kNHChain; k++) {
+        c.vel[k] = __ldcg(&g.vel[k]);
+        c.force[k] = __ldcg(&g.force[k]);
+        c.mass[k] = __ldcg(&g.mass[k]);
+        c.inv_mass[k] = __ldcg(&g.inv_mass[k]);
+    }
+    c.ndf = __ldcg(&g.ndf);
+    c.kB = __ldcg(&g.kB);
+    c.T = __ldcg(&g.T);
+    c.dt = __ldcg(&g.dt);
+}
 
 __device__ __forceinline__ void store_chain(NHChain &d, const NHRegs &c, double last_ke, double scale) {
 #pragma unroll
@@ -395,67 +432,71 @@ __device__ __forceinline__ void store_chain(NHChain &d, const NHRegs &c, double 
     d.scale = scale;
 }
 
-// Last-block epilogue: fixed-order FP64 sum of the block partials, then the
-// Nose-Hoover stepFinal + next stepInit on one thread, and the turn counter.
-// nparts partials are summed; the counter target is this kernel's grid size
-__device__ void finish_step(double *partials, int nparts, unsigned int *counter, NHChain *chain, int nh,
-                            DeviceStatus *st, double *ke_out, unsigned int nblk) {
-    __shared__ bool last;
-    __threadfence();
-    if (threadIdx.x == 0) {
-        unsigned int prev = atomicAdd(counter, 1u);
-        last = (prev == nblk - 1u);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // thread 0 reads the chain into registers (a copy of the struct would
-    // sit in local memory on this serial path) while the partials are read
-    NHRegs c;
-    double mvv = 0.0;
-    if (threadIdx.x == 0 && nh) {
-        const NHChain &g = chain[0];
-#pragma unroll
-        for (int k = 0; k < kNHChain; k++) {
-            c.vel[k] = __ldcg(&g.vel[k]);
-            c.force[k] = __ldcg(&g.force[k]);
-            c.mass[k] = __ldcg(&g.mass[k]);
-            c.inv_mass[k] = __ldcg(&g.inv_mass[k]);
-        }
-        c.ndf = __ldcg(&g.ndf);
-        c.kB = __ldcg(&g.kB);
-        c.T = __ldcg(&g.T);
-        c.dt = __ldcg(&g.dt);
-        mvv = __ldcg(&g.mvv_to_eng);
-    }
-    // every thread of the last block sums a fixed strided share of the
-    // partials (L2 reads), then a fixed-order block reduction: deterministic
+// The end of a step, one block per system, launched behind the second half:
+// the fixed-order FP64 sum of its block partials, the Nose-Hoover stepFinal
+// and the stepInit of the coming step on one thread, and the turn counter.
+// What bounds it is one dependent chain of FP64 operations (8.3 cycles each
+// on B200): resident before the second half ends, the thread has loaded the
+// chain and done the sweep that needs no kinetic energy when the partials
+// arrive.  As the tail of the second half's last block (fence, block counter,
+// then all of it serially with an exponential per link and sweep) it took
+// about 5 us of every step.
+struct EndArgs {
+    const double *partials;
+    int nparts;
+    int nh;
+    NHChain *chain;
+    DeviceStatus *st;
+    double *ke_out;
+};
+constexpr int kEndThreads = 256;
+
+__global__ void __launch_bounds__(kEndThreads) k_step_end(const EndArgs a0, const EndArgs *__restrict__ tab) {
     __shared__ double red[32];
-    double acc = 0.0;
-    for (int b = threadIdx.x; b < nparts; b += blockDim.x) acc += __ldcg(partials + b);
-    const double tot_all = block_sum(acc, red);
-    if (threadIdx.x == 0) {
-        const double tot = tot_all;
-        *counter = 0u;
-        if (ke_out) *ke_out = tot;
-        if (nh) {
-            // constants stay in chain[0/1]
-            c.ke = tot * mvv;
-            const double last_ke = c.ke;
-            const double sf1 = nh_integrate_n<kNHChain>(c, false);  // stepFinal
-            store_chain(chain[1], c, last_ke, sf1);
-            const double sf2 = nh_integrate_n<kNHChain>(c, true);   // stepInit of the next step
-            store_chain(chain[0], c, last_ke, sf1 * sf2);
-        }
-        st->turn += 1;
+    const EndArgs A = tab ? tab[blockIdx.x] : a0;
+    NHRegs c;
+    double pf[kNHChain - 1], mvv = 0.0, most = 0.0;
+    const bool chain = threadIdx.x == 0 && A.nh;
+    if (chain) {
+        // written by this kernel a step ago; everything before the second
+        // half, which is running or done, has completed
+        load_chain(c, A.chain[0]);
+        mvv = __ldcg(&A.chain[0].mvv_to_eng);
+        nh_down<kNHChain, true>(c, pf, most);
     }
+    pdl_wait();
+    // the coming first half may load what this kernel does not write
+    pdl_trigger();
+    double acc = 0.0;
+    for (int b = threadIdx.x; b < A.nparts; b += kEndThreads) acc += __ldcg(A.partials + b);
+    const double tot = block_sum(acc, red);
+    if (threadIdx.x != 0) return;
+    if (A.ke_out) *A.ke_out = tot;
+    A.st->turn += 1;
+    if (!chain) return;
+    // constants stay in chain[0/1]
+    const double ke = tot * mvv;
+    c.ke = ke;
+    double sf1 = nh_up<kNHChain, true>(c, pf, false, most);  // stepFinal
+    NHRegs fin = c;
+    double sf2 = nh_half<kNHChain, true>(c, true, most);  // stepInit of the next step
+    if (!(most < kNHSmall)) {  // outside the polynomial's range: again, with exp()
+        load_chain(c, A.chain[0]);
+        c.ke = ke;
+        sf1 = nh_half<kNHChain, false>(c, false, most);
+        fin = c;
+        sf2 = nh_half<kNHChain, false>(c, true, most);
+    }
+    store_chain(A.chain[0], c, ke, sf1 * sf2);
+    store_chain(A.chain[1], fin, ke, sf1);
 }
 
 // per-atom: postForce_cu (IntegratorVerlet.cu:610-627) + m v^2 partials
 __global__ void k_second_atoms(int n, float4 *__restrict__ vs, const float4 *__restrict__ fs,
                                const uint32_t *__restrict__ ids, const uint8_t *__restrict__ rigid_by_id, float dtf,
-                               double *__restrict__ partials, int part_off, int nparts, unsigned int *counter,
-                               NHChain *chain, int nh, DeviceStatus *st, double *ke_out, int do_finish) {
+                               double *__restrict__ partials, int part_off) {
+    pdl_wait();
+    pdl_trigger();  // k_step_end: one block, resident while this grid runs
     __shared__ double sh[32];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double mv2 = 0.0;
@@ -471,16 +512,16 @@ __global__ void k_second_atoms(int n, float4 *__restrict__ vs, const float4 *__r
     }
     const double b = block_sum(mv2, sh);
     if (threadIdx.x == 0) partials[part_off + blockIdx.x] = b;
-    if (do_finish) finish_step(partials, nparts, counter, chain, nh, st, ke_out, gridDim.x);
 }
 
 // per-molecule fused: postForce + distributeMSite + settleVelocities +
-// validateConstraints + m v^2 partials (+ last-block NH / turn)
+// validateConstraints + m v^2 partials
 // fextra (may be null): per-molecule-atom forces computed beside the pair
 // kernel (E3B), indexed like fs, merged into O/H1/H2 here
 __global__ void k_second_mol(const MolArgs a0, const MolArgs *__restrict__ tab) {
     MDX_MOL_ARGS;
-    if ((int)blockIdx.x >= A.nblk) return;  // the whole block: not counted
+    pdl_trigger();  // k_step_end: one block a system, resident while this grid runs
+    if ((int)blockIdx.x >= A.nblk) return;  // past this replica's molecules: no partial
     __shared__ double sh[32];
     const int nmol = A.nmol;
     const float4 *__restrict__ xs = A.xs;
@@ -555,10 +596,6 @@ __global__ void k_second_mol(const MolArgs a0, const MolArgs *__restrict__ tab) 
     }
     const double b = block_sum(mv2, sh);
     if (threadIdx.x == 0) A.partials[A.part_off + blockIdx.x] = b;
-    // the next step's first half may be scheduled now: it waits for this
-    // grid (the last block's chain update included) before reading anything
-    pdl_trigger();
-    finish_step(A.partials, A.nparts, A.counter, A.chain, A.nh, st, A.ke_out, (unsigned int)A.nblk);
 }
 
 // ---- stand-alone hooks (one kernel per reference hook) ------------------
@@ -796,10 +833,6 @@ MolArgs mol_args(State &s, FixRigid &r) {
     A.st = s.d_status.p;
     A.partials = s.red_partials.p;
     A.part_off = 0;
-    A.nparts = rigid_blocks(A.nmol);
-    A.counter = s.red_counter.p;
-    A.nh = nh ? 1 : 0;
-    A.ke_out = s.red_out.p;
     A.fextra = nullptr;
     A.frecip = nullptr;
     A.nblk = rigid_blocks(A.nmol);
@@ -844,7 +877,7 @@ bool has_free_atoms(State &s) {
     return members < s.atoms.size();
 }
 
-int step_first_half(State &s, bool fused) {
+int step_first_half(State &s, bool fused, bool early) {
     const int n = s.gpd.n;
     const float dt = (float)s.dt;
     const float dtf = (float)(0.5 * s.dt * s.units.ftm_to_v);
@@ -870,33 +903,35 @@ int step_first_half(State &s, bool fused) {
     }
     if (has_free_atoms(s)) {
         const uint8_t *rf = r ? rigid_flags(s) : nullptr;
-        if (nh)
-            k_first_atoms<true><<<(n + 255) / 256, 256, 0, s.stream>>>(n, s.gpd.xs.p, s.gpd.vs.p, s.gpd.fs.p,
-                                                                      s.gpd.ids.p, rf, dt, dtf, chain);
-        else
-            k_first_atoms<false><<<(n + 255) / 256, 256, 0, s.stream>>>(n, s.gpd.xs.p, s.gpd.vs.p, s.gpd.fs.p,
-                                                                       s.gpd.ids.p, rf, dt, dtf, chain);
-        MDX_LAUNCHED();
+        MDX_CUDA_TRY(launch_pdl(nh ? k_first_atoms<true> : k_first_atoms<false>, dim3((n + 255) / 256), dim3(256), 0,
+                                s.stream, n, s.gpd.xs.p, s.gpd.vs.p, s.gpd.fs.p, (const uint32_t *)s.gpd.ids.p, rf, dt,
+                                dtf, chain, early ? 1 : 0));
     }
     if (r) {
         MolArgs A = mol_args(s, *r);
         A.slots = s.mf.on ? 1 : 0;
-        if (nh)
-            MDX_CUDA_TRY(launch_pdl(k_first_mol<true>, dim3(rigid_blocks(A.nmol)), dim3(kMolBlock), 0, s.stream, A,
-                                    (const MolArgs *)nullptr));
-        else
-            MDX_CUDA_TRY(launch_pdl(k_first_mol<false>, dim3(rigid_blocks(A.nmol)), dim3(kMolBlock), 0, s.stream, A,
-                                    (const MolArgs *)nullptr));
+        MDX_CUDA_TRY(launch_pdl(nh ? k_first_mol<true> : k_first_mol<false>, dim3(rigid_blocks(A.nmol)),
+                                dim3(kMolBlock), 0, s.stream, A, (const MolArgs *)nullptr, early ? 1 : 0));
     }
     return 0;
+}
+
+static EndArgs end_args(State &s, int nparts) {
+    FixNoseHoover *nh = s.nhFix();
+    EndArgs E{};
+    E.partials = s.red_partials.p;
+    E.nparts = nparts;
+    E.nh = nh ? 1 : 0;
+    E.chain = nh ? nh->d_chain.p : nullptr;
+    E.st = s.d_status.p;
+    E.ke_out = s.red_out.p;
+    return E;
 }
 
 int step_second_half(State &s, bool fused, const float4 *fextra, const float4 *frecip) {
     const int n = s.gpd.n;
     const float dtf = (float)(0.5 * s.dt * s.units.ftm_to_v);
-    FixNoseHoover *nh = s.nhFix();
     FixRigid *r = s.rigidFix();
-    NHChain *chain = nh ? nh->d_chain.p : nullptr;
     const int ab = (n + 255) / 256;
     const int mb = r ? rigid_blocks((int)r->mol_ids.size()) : 0;
     const bool free_atoms = has_free_atoms(s);
@@ -915,28 +950,24 @@ int step_second_half(State &s, bool fused, const float4 *fextra, const float4 *f
         // stepFinal: reduce m v^2 then the chain on the device (single block)
         k_mv2<<<ab, 256, 0, s.stream>>>(n, s.gpd.vs.p, s.red_partials.p);
         MDX_LAUNCHED();
-        k_second_atoms<<<1, 32, 0, s.stream>>>(0, s.gpd.vs.p, s.gpd.fs.p, nullptr, nullptr, dtf, s.red_partials.p,
-                                               ab, ab + 1, s.red_counter.p, chain, nh ? 1 : 0, s.d_status.p,
-                                               s.red_out.p, 1);
+        k_step_end<<<1, kEndThreads, 0, s.stream>>>(end_args(s, ab), nullptr);
         MDX_LAUNCHED();
         return 0;
     }
-    const uint8_t *rf = r ? rigid_flags(s) : nullptr;
-    if (free_atoms) {
-        k_second_atoms<<<ab, 256, 0, s.stream>>>(n, s.gpd.vs.p, s.gpd.fs.p, s.gpd.ids.p, rf, dtf, s.red_partials.p, 0,
-                                                 nparts, s.red_counter.p, chain, nh ? 1 : 0, s.d_status.p,
-                                                 s.red_out.p, r ? 0 : 1);
-        MDX_LAUNCHED();
-    }
+    if (free_atoms)
+        MDX_CUDA_TRY(launch_pdl(k_second_atoms, dim3(ab), dim3(256), 0, s.stream, n, s.gpd.vs.p,
+                                (const float4 *)s.gpd.fs.p, (const uint32_t *)s.gpd.ids.p,
+                                (const uint8_t *)(r ? rigid_flags(s) : nullptr), dtf, s.red_partials.p, 0));
     if (r) {
         MolArgs A = mol_args(s, *r);
         A.part_off = free_atoms ? ab : 0;
-        A.nparts = nparts;
         A.fextra = fextra;
         A.frecip = frecip;
         A.slots = s.mf.on ? 1 : 0;
         MDX_CUDA_TRY(launch_pdl(k_second_mol, dim3(mb), dim3(kMolBlock), 0, s.stream, A, (const MolArgs *)nullptr));
     }
+    MDX_CUDA_TRY(launch_pdl(k_step_end, dim3(1), dim3(kEndThreads), 0, s.stream, end_args(s, nparts),
+                            (const EndArgs *)nullptr));
     return 0;
 }
 
@@ -1126,6 +1157,10 @@ int batch_mol_tables(Batch &b) {
     if (int e = b.tab_second.alloc(R * sizeof(MolArgs))) return e;
     MDX_CUDA_TRY(cudaMemcpy(b.tab_first.p, h1.data(), R * sizeof(MolArgs), cudaMemcpyHostToDevice));
     MDX_CUDA_TRY(cudaMemcpy(b.tab_second.p, h2.data(), R * sizeof(MolArgs), cudaMemcpyHostToDevice));
+    std::vector<EndArgs> h3(R);
+    for (int r = 0; r < R; r++) h3[r] = end_args(*b.reps[r], h1[r].nblk);
+    if (int e = b.tab_end.alloc(R * sizeof(EndArgs))) return e;
+    MDX_CUDA_TRY(cudaMemcpy(b.tab_end.p, h3.data(), R * sizeof(EndArgs), cudaMemcpyHostToDevice));
     return 0;
 }
 
@@ -1221,21 +1256,22 @@ int batch_rigid_maps(Batch &b) {
     return 0;
 }
 
-int batch_first_half(Batch &b) {
+int batch_first_half(Batch &b, bool early) {
     MolArgs A;
     if (int e = batch_sizing(b, &A)) return e;
-    k_first_mol<true><<<dim3(A.nblk, (unsigned)b.reps.size()), kMolBlock, 0, b.stream>>>(
-        A, reinterpret_cast<const MolArgs *>(b.tab_first.p));
-    MDX_LAUNCHED();
+    MDX_CUDA_TRY(launch_pdl(k_first_mol<true>, dim3(A.nblk, (unsigned)b.reps.size()), dim3(kMolBlock), 0, b.stream, A,
+                            reinterpret_cast<const MolArgs *>(b.tab_first.p), early ? 1 : 0));
     return 0;
 }
 
 int batch_second_half(Batch &b, bool with_e3b) {
     MolArgs A;
     if (int e = batch_sizing(b, &A)) return e;
-    k_second_mol<<<dim3(A.nblk, (unsigned)b.reps.size()), kMolBlock, 0, b.stream>>>(
-        A, reinterpret_cast<const MolArgs *>(with_e3b ? b.tab_second.p : b.tab_first.p));
-    MDX_LAUNCHED();
+    const unsigned R = (unsigned)b.reps.size();
+    MDX_CUDA_TRY(launch_pdl(k_second_mol, dim3(A.nblk, R), dim3(kMolBlock), 0, b.stream, A,
+                            reinterpret_cast<const MolArgs *>(with_e3b ? b.tab_second.p : b.tab_first.p)));
+    MDX_CUDA_TRY(launch_pdl(k_step_end, dim3(R), dim3(kEndThreads), 0, b.stream, EndArgs{},
+                            reinterpret_cast<const EndArgs *>(b.tab_end.p)));
     return 0;
 }
 

@@ -72,12 +72,12 @@ class IntegratorVerlet {
     // fused step: the P3M chain (spread, R2C, E(k), C2R) and E3B run on two
     // side streams beside the pair kernel; they join before the P3M gather
     // and the second half (which merges the E3B forces)
-    int stepFused() {
+    int stepFused(bool early) {
         FixPair *pf = s->pairFix();
         FixChargeEwald *ew = s->ewaldFix();
         FixE3B *e3 = s->e3bFix();
         const bool e3side = e3 && e3->side_ok && s->rigidFix();
-        if (int e = step_first_half(*s, true)) return e;
+        if (int e = step_first_half(*s, true, early)) return e;
         if (ew || e3side) MDX_CUDA_TRY(cudaEventRecord(s->ev_fork, s->stream));
         // all-rigid systems: the gather also runs on the side stream, into a
         // per-step buffer the second half adds (so it overlaps the pair kernel)
@@ -222,8 +222,8 @@ class IntegratorVerlet {
         return s->checkStatus();
     }
 
-    int stepBody() {
-        if (mode == 0) return stepFused();
+    int stepBody(bool early) {
+        if (mode == 0) return stepFused(early);
         if (int e = step_first_half(*s, false)) return e;
         if (int e = forces()) return e;
         if (int e = step_second_half(*s, false)) return e;
@@ -241,7 +241,7 @@ class IntegratorVerlet {
             build_pending = overlap;
         }
         for (int k = 0; k < nsteps; k++)
-            if (int e = stepBody()) return e;
+            if (int e = stepBody(k > 0)) return e;
         if (build_pending) MDX_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->ev_join[2], 0));
         build_pending = false;
         return 0;

@@ -152,11 +152,9 @@ int State::upload() {
     if (int e = d.ids_alt.alloc(n)) return e;
     if (int e = d.idToIdx.alloc(n)) return e;
     if (int e = d.virials.alloc(6 * (size_t)n)) return e;
-    if (int e = red_counter.alloc(1)) return e;
     if (int e = red_out.alloc(4)) return e;
     if (int e = e_site.alloc(n)) return e;
     if (int e = e_sum.alloc(1)) return e;
-    MDX_CUDA_TRY(cudaMemset(red_counter.p, 0, sizeof(unsigned int)));
     MDX_CUDA_TRY(cudaMemset(d.virials.p, 0, 6 * (size_t)n * sizeof(float)));
     std::vector<float4> xs(n), vs(n), fs(n);
     std::vector<float> qs(n);
