@@ -123,7 +123,12 @@ PairArgs make_args(State &s, FixPair &f) {
 // The molecule's own site pairs (the excluded pairs of the reference's list,
 // multiplier by exclusion depth) are added by lane 0.  Forces on the four
 // sites are reduced by shuffles and written by lanes 0..3 (one 64-byte store).
+// blocks per SM the kernel is compiled for: 80 registers, which lets the nine
+// charge pairs of a molecule pair be in flight beside one another.  Alone at
+// 4,096 / 32,768 molecules: 22.6 / 137 us (14 blocks, 72 registers: 24.2 / 144;
+// 10 blocks, 94: 22.5 / 136; 8 blocks, 106: 23.5 / 188)
 constexpr int kMolPairBlock = 64;
+constexpr int kMolPairBlocksPerSM = 12;
 constexpr int kMolQueue = 64;  // queued entries per warp (two chunks)
 
 struct MolPairArgs {
@@ -135,6 +140,7 @@ struct MolPairArgs {
     int cap;
     Box box;
     float far2, qrc2, alpha;
+    float ex2a, twoa;  // -alpha^2 log2(e), 2 alpha / sqrt(pi)
     uint32_t ljm, qm, selfm;  // bit 4a+b: LJ term, charge term, own-molecule pair
     // per site pair ab: rc^2, 48 eps sig^12, 24 eps sig^6, sig^6, eps, the
     // LJ/cut energy shift at rc, qqr q_a q_b, exclusion multiplier (own pairs)
@@ -147,6 +153,27 @@ __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// the warp's sums of f[0..3], site a's in lanes 8 a .. 8 a + 7
+__device__ __forceinline__ float3 site_sum(const float3 (&f)[4], int lane) {
+    const bool h = lane & 16, q = lane & 8;
+    float3 g[2], r;
+    auto halve = [](bool up, float a, float b, int o) {
+        return (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, o);
+    };
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        g[i] = make_float3(halve(h, f[i].x, f[i + 2].x, 16), halve(h, f[i].y, f[i + 2].y, 16),
+                           halve(h, f[i].z, f[i + 2].z, 16));
+    r = make_float3(halve(q, g[0].x, g[1].x, 8), halve(q, g[0].y, g[1].y, 8), halve(q, g[0].z, g[1].z, 8));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        r.x += __shfl_xor_sync(0xffffffffu, r.x, o);
+        r.y += __shfl_xor_sync(0xffffffffu, r.y, o);
+        r.z += __shfl_xor_sync(0xffffffffu, r.z, o);
+    }
+    return r;
 }
 
 template <bool VIR>
@@ -193,20 +220,22 @@ __device__ __forceinline__ float mol_pair_term(const MolPairArgs &A, int ab, flo
         }
     }
     if (EW && topo_q<TOPO>(A, ab)) {
+        // F/r = qq e^{-a^2 r^2} (t P(t) / r + 2 a / sqrt(pi)) / r^2 with
+        // erfc(a r) = t P(t) e^{-a^2 r^2}: the exponential and 1/r^2 (zero
+        // beyond the cutoff) are common factors
         const float r2c = fmaxf(r2, 1e-10f);
         const float rinv = rsqrt_ftz(r2c);
-        const float x = A.alpha * (r2c * rinv);
-        const float expm = exp_neg_sq(x);
-        const float erfcv = pk::erfc_as(x, expm);
+        const float expm = ex2_ftz(r2c * A.ex2a);
+        const float tp = pk::erfc_tp(A.alpha * (r2c * rinv));
         const float qq = A.qq[ab];
-        float fsc = qq * (erfcv * rinv + (2.0f * 0.5641895835477563f * A.alpha) * expm);
-        if (OWN && mult < 1.0f) fsc -= (1.0f - mult) * qq * rinv;
-        const float in = r2 < A.qrc2 ? 1.0f : 0.f;
-        s += fsc * (rinv * rinv) * in;
+        const float r2inv = r2 < A.qrc2 ? rinv * rinv : 0.f;
+        const float g = qq * (expm * r2inv);
+        s += g * fmaf(tp, rinv, A.twoa);
+        if (OWN && mult < 1.0f) s -= (1.0f - mult) * qq * rinv * r2inv;
         if (ENERGY) {
-            float eng = qq * rinv * erfcv;
+            float eng = qq * rinv * (tp * expm);
             if (OWN && mult < 1.0f) eng -= (1.0f - mult) * qq * rinv;
-            e += 0.5f * eng * in;
+            e += r2 < A.qrc2 ? 0.5f * eng : 0.f;
         }
     }
     return s;
@@ -266,7 +295,7 @@ __device__ __forceinline__ void mol_pair_eval(const MolPairArgs &A, const float3
 // BATCH: batched replicas, the arguments of replica blockIdx.y from tab
 // (a0 unused); otherwise a0
 template <int LJ, bool EW, bool VIR, bool ENERGY, int TOPO, bool BATCH = false>
-__global__ void __launch_bounds__(kMolPairBlock, 14) k_pair_mol(const MolPairArgs a0,
+__global__ void __launch_bounds__(kMolPairBlock, kMolPairBlocksPerSM) k_pair_mol(const MolPairArgs a0,
                                                                 const MolPairArgs *__restrict__ tab, int accumulate) {
     pdl_wait();
     const MolPairArgs &A = BATCH ? tab[blockIdx.y] : a0;
@@ -393,17 +422,18 @@ __global__ void __launch_bounds__(kMolPairBlock, 14) k_pair_mol(const MolPairArg
             if (lane < 4) A.energy[4 * k + lane] = lane == 0 ? en[0] : (lane == 1 ? en[1] : (lane == 2 ? en[2] : en[3]));
             continue;
         }
-#pragma unroll
-        for (int a = 0; a < 4; a++) f[a] = make_float3(warp_sum(f[a].x), warp_sum(f[a].y), warp_sum(f[a].z));
         if (VIR) {
 #pragma unroll
             for (int a = 0; a < 4; a++)
 #pragma unroll
                 for (int c = 0; c < 6; c++) v[a][c] = warp_sum(v[a][c]);
         }
-        if (lane < 4) {
-            const float3 fm = lane == 0 ? f[0] : (lane == 1 ? f[1] : (lane == 2 ? f[2] : f[3]));
-            float4 fo = A.fs[4 * k + lane];
+        // sites to lane groups: lanes 8 a .. 8 a + 7 end with site a's sum
+        // (two halving exchanges, then butterflies over the eight lanes)
+        const float3 fm = site_sum(f, lane);
+        const int site = lane >> 3;
+        if ((lane & 7) == 0) {
+            float4 fo = A.fs[4 * k + site];
             if (accumulate) {
                 fo.x += fm.x;
                 fo.y += fm.y;
@@ -413,14 +443,14 @@ __global__ void __launch_bounds__(kMolPairBlock, 14) k_pair_mol(const MolPairArg
                 fo.y = fm.y;
                 fo.z = fm.z;
             }
-            A.fs[4 * k + lane] = fo;
-            if (VIR) {
-                float *vv = A.virials + 6 * (size_t)(4 * k + lane);
+            A.fs[4 * k + site] = fo;
+        }
+        if (VIR && lane < 4) {
+            float *vv = A.virials + 6 * (size_t)(4 * k + lane);
 #pragma unroll
-                for (int c = 0; c < 6; c++) {
-                    const float vm = lane == 0 ? v[0][c] : (lane == 1 ? v[1][c] : (lane == 2 ? v[2][c] : v[3][c]));
-                    vv[c] += 0.5f * vm;
-                }
+            for (int c = 0; c < 6; c++) {
+                const float vm = lane == 0 ? v[0][c] : (lane == 1 ? v[1][c] : (lane == 2 ? v[2][c] : v[3][c]));
+                vv[c] += 0.5f * vm;
             }
         }
     }
@@ -450,6 +480,8 @@ MolPairArgs make_mol_args(State &s, FixPair &f) {
         A.qrc2 = qrc * qrc;
         A.alpha = (float)f.chargeFix->alpha;
     }
+    A.ex2a = (float)(-1.4426950408889634 * (double)A.alpha * A.alpha);
+    A.twoa = (float)(1.1283791670955126 * (double)A.alpha);
     const float qqr = (float)s.units.qqr_to_eng;
     const float coef[3] = {s.specialNeighborCoefs[0], s.specialNeighborCoefs[1], s.specialNeighborCoefs[2]};
     A.ljm = A.qm = A.selfm = 0u;
@@ -519,18 +551,23 @@ int pair_mol_launch(State &s, FixPair &f, int virialMode, bool accumulate, float
     // the four-site water pattern (LJ on sites 0, charges on 1..3) as
     // compile-time masks; any other pattern from the runtime masks
     const bool water4 = ew && A.ljm == 0x1u && A.qm == 0xEEE0u;
-    // blocks per SM of the grid.  Automatic: a pair block holds its SM for
-    // most of the kernel (one molecule per warp, one wave), so with every SM
-    // full the P3M chain beside it (all-rigid water) waits for the pair
-    // kernel at each of its launches; a grid capped below the SMs' capacity
-    // keeps room for it (measured on B200, 4,096 molecules: 10 blocks per SM
-    // without E3B, 7 with the E3B kernel as a third branch).  Else uncapped.
-    int bps = s.pairBlocksPerSM;
-    if (bps == 0) {
-        const bool p3m_beside = ew && s.rigidFix() && !has_free_atoms(s);
-        bps = p3m_beside ? (s.e3bFix() ? 7 : 10) : -1;
+    // the grid's blocks.  With the P3M chain beside it (all-rigid water) the
+    // kernel must leave SM slots for that chain's blocks, and a warp that
+    // takes one molecule more than another is a tail: the grid is cut to the
+    // fewest rounds the SMs' capacity allows and then to the fewest blocks
+    // that need no more rounds.  Measured on B200, water step at 4,096
+    // molecules (two rounds, 7 blocks per SM): 53.0 us; 8, 10, 12 blocks per
+    // SM 53.4, 55.5, 59.4; 6 (three rounds) 65; with E3B 8, 10, 12: 62.9,
+    // 63.3, 64.4; at 32,768 (ten rounds, 11 blocks) 8, 10, 12: 321, 304, 303.
+    // Else, and for pairBlocksPerSM -1, a warp per molecule
+    int mb = 0;
+    if (s.pairBlocksPerSM > 0) {
+        mb = s.pairBlocksPerSM * num_sms();
+    } else if (s.pairBlocksPerSM == 0 && ew && s.rigidFix() && !has_free_atoms(s)) {
+        const int wpb = kMolPairBlock / 32, most = wpb * kMolPairBlocksPerSM * num_sms();
+        const int rounds = (A.nmol + most - 1) / most;
+        mb = ((A.nmol + rounds - 1) / rounds + wpb - 1) / wpb;
     }
-    const int mb = bps > 0 ? bps * num_sms() : 0;
     if (f.lj_kind == 1 && water4) mol_launch_t<1, true, 1>(A, virialMode, en, accumulate, mb, st);
     else if (f.lj_kind == 1 && ew) mol_launch_t<1, true, 0>(A, virialMode, en, accumulate, mb, st);
     else if (f.lj_kind == 1) mol_launch_t<1, false, 0>(A, virialMode, en, accumulate, mb, st);

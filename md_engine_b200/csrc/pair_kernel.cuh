@@ -65,7 +65,8 @@ struct PairArgs {
 // erfc(x) for x >= 0 by Abramowitz & Stegun, Handbook of Mathematical
 // Functions, eq. 7.1.26 (|error| <= 1.5e-7): erfc(x) = t P5(t) exp(-x^2) with
 // t = 1 / (1 + p x).  exp(-x^2) is passed in: the Ewald force needs it anyway.
-__device__ __forceinline__ float erfc_as(float x, float expmx2) {
+// erfc_tp: the factor t P5(t) alone
+__device__ __forceinline__ float erfc_tp(float x) {
     // t only feeds the A&S polynomial (error 1.5e-7): the approximate
     // reciprocal (one SFU op, a few ulp) is plenty
     const float t = rcp_ftz(fmaf(0.3275911f, x, 1.0f));
@@ -73,8 +74,9 @@ __device__ __forceinline__ float erfc_as(float x, float expmx2) {
     poly = fmaf(t, poly, 1.421413741f);
     poly = fmaf(t, poly, -0.284496736f);
     poly = fmaf(t, poly, 0.254829592f);
-    return t * poly * expmx2;
+    return t * poly;
 }
+__device__ __forceinline__ float erfc_as(float x, float expmx2) { return erfc_tp(x) * expmx2; }
 
 // one neighbour: returns the scalar force factor (F = dr * s) and energy
 template <int LJ, int CK, bool ENERGY>
