@@ -34,6 +34,44 @@ using namespace mdx;
         return MDX_ERR_STATE;                                 \
     }
 
+namespace {
+int get_atoms(State &s, double *pos, double *vel, double *force) {
+    if (int e = s.download()) return e;
+    double *const out[3] = {pos, vel, force};
+    if (s.uploaded && (size_t)s.gpd.n == s.atoms.size()) {
+        for (int k = 0; k < 3; k++)
+            if (out[k]) host_copy(out[k], s.stageHost(k), 3 * s.atoms.size() * sizeof(double));
+        return 0;
+    }
+    // with atoms that are not on the device yet
+    for (size_t i = 0; i < s.atoms.size(); i++) {
+        const HostAtom &a = s.atoms[i];
+        for (int d = 0; d < 3; d++) {
+            if (pos) pos[3 * i + d] = a.pos[d];
+            if (vel) vel[3 * i + d] = a.vel[d];
+            if (force) force[3 * i + d] = a.force[d];
+        }
+    }
+    return 0;
+}
+
+int put_atoms(State &s, const double *pos, const double *vel) {
+    if (int e = s.stageAlloc()) return e;
+    MDX_CUDA_TRY(cudaStreamSynchronize(s.stream));  // the staging may be on its way out
+    const double *const in[2] = {pos, vel};
+    for (int k = 0; k < 2; k++)
+        if (in[k])
+            if (int e = s.stagePut(k, in[k])) return e;
+    for (int i = 0; i < s.gpd.n; i++)
+        for (int d = 0; d < 3; d++) {
+            if (pos) s.atoms[i].pos[d] = pos[3 * i + d];
+            if (vel) s.atoms[i].vel[d] = vel[3 * i + d];
+        }
+    MDX_CUDA_TRY(cudaStreamSynchronize(s.stream));
+    return 0;
+}
+}  // namespace
+
 extern "C" {
 
 const char *mdx_last_error(void) { return last_error(); }
@@ -234,51 +272,16 @@ int mdx_state_set_velocities(mdx_state *st, int n, const int *ids, const double 
 
 int mdx_state_get_atoms(mdx_state *st, double *pos, double *vel, double *force) {
     ARG_CHECK(st, "null state");
-    State &s = *st->s;
-    GUARD(if (int e = s.download()) return e;)
-    for (size_t i = 0; i < s.atoms.size(); i++)
-        for (int d = 0; d < 3; d++) {
-            if (pos) pos[3 * i + d] = s.atoms[i].pos[d];
-            if (vel) vel[3 * i + d] = s.atoms[i].vel[d];
-            if (force) force[3 * i + d] = s.atoms[i].force[d];
-        }
-    return 0;
+    GUARD(return get_atoms(*st->s, pos, vel, force);)
 }
-
 int mdx_state_put_atoms(mdx_state *st, const double *pos, const double *vel) {
     ARG_CHECK(st, "null state");
-    State &s = *st->s;
-    if (!s.uploaded) {
+    if (!st->s->uploaded) {
         set_error(MDX_ERR_STATE, "state has no device copy yet (call mdx_prepare or run first)");
         return MDX_ERR_STATE;
     }
-    const int n = s.gpd.n;
-    std::vector<uint32_t> ids(n);
-    std::vector<float4> xs(n), vs(n);
-    MDX_CUDA_TRY(cudaStreamSynchronize(s.stream));
-    MDX_CUDA_TRY(cudaMemcpy(ids.data(), s.gpd.ids.p, n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    MDX_CUDA_TRY(cudaMemcpy(xs.data(), s.gpd.xs.p, n * sizeof(float4), cudaMemcpyDeviceToHost));
-    MDX_CUDA_TRY(cudaMemcpy(vs.data(), s.gpd.vs.p, n * sizeof(float4), cudaMemcpyDeviceToHost));
-    for (int i = 0; i < n; i++) {
-        const uint32_t id = ids[i];
-        if (pos) {
-            xs[i].x = (float)pos[3 * id];
-            xs[i].y = (float)pos[3 * id + 1];
-            xs[i].z = (float)pos[3 * id + 2];
-            for (int d = 0; d < 3; d++) s.atoms[id].pos[d] = pos[3 * id + d];
-        }
-        if (vel) {
-            vs[i].x = (float)vel[3 * id];
-            vs[i].y = (float)vel[3 * id + 1];
-            vs[i].z = (float)vel[3 * id + 2];
-            for (int d = 0; d < 3; d++) s.atoms[id].vel[d] = vel[3 * id + d];
-        }
-    }
-    MDX_CUDA_TRY(cudaMemcpy(s.gpd.xs.p, xs.data(), n * sizeof(float4), cudaMemcpyHostToDevice));
-    MDX_CUDA_TRY(cudaMemcpy(s.gpd.vs.p, vs.data(), n * sizeof(float4), cudaMemcpyHostToDevice));
-    return 0;
+    GUARD(return put_atoms(*st->s, pos, vel);)
 }
-
 int mdx_state_activate_fix(mdx_state *st, mdx_fix *fix) {
     ARG_CHECK(st && fix, "null argument");
     State &s = *st->s;

@@ -379,6 +379,7 @@ struct E3BSurrogate {
     DBuf<float4> fexact;
     // training scratch
     DBuf<__nv_bfloat16> xb, act[3], dz;
+    DBuf<float> xf;  // host rows before their rounding to BF16
     DBuf<float> z[4], yb, da;
     DBuf<double> loss;
     int batch = 0;
@@ -546,6 +547,15 @@ class State {
     // a rebuild step
     cudaStream_t side[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[3] = {nullptr, nullptr, nullptr}, ev_sorted = nullptr;
+    // host arrays by atom id cross here: (n,3) FP64 positions, velocities and
+    // forces, pinned on the host and on the device, which rounds and orders
+    double *stage_h = nullptr;
+    size_t stage_n = 0;
+    DBuf<double> stage_d;
+    int stageAlloc();
+    int stagePut(int k, const double *src);  // array k (0 or 1) onto the device stream, on `stream`
+    int stageGet(int k);                     // array k into stage_h, on `stream`
+    double *stageHost(int k) const { return stage_h + 3 * (size_t)k * gpd.n; }
     bool uploaded = false;   // device copy is authoritative
     bool prepared = false;
     bool requiresCharges = false;
@@ -664,6 +674,9 @@ int batch_e3b_forces(Batch &b, cudaStream_t stream);
 int batch_first_half(Batch &b, bool early);
 int batch_second_half(Batch &b, bool with_e3b);
 int batch_rigid_maps(Batch &b);
+
+// memcpy, in a few threads for long arrays
+void host_copy(void *dst, const void *src, size_t bytes);
 
 // ---------------------------------------------------------------- kernels
 // neighbour list (nlist.cu)

@@ -17,32 +17,6 @@
 
 namespace mdx {
 
-namespace {
-// host-buffer run support: scatter by id into the sorted device streams and
-// gather them back in id order
-// host-buffer runs: (n,3) FP64 arrays by atom id in, rounded to FP32 here
-// (the host cast's round-to-nearest), and widened back out; .w is kept
-__global__ void k_put_by_id(int n, const double *__restrict__ in, const int *__restrict__ idToIdx,
-                            float4 *__restrict__ dst) {
-    int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    const int i = idToIdx[id];
-    const float w = dst[i].w;
-    const double *v = in + 3 * (size_t)id;
-    dst[i] = make_float4((float)v[0], (float)v[1], (float)v[2], w);
-}
-__global__ void k_get_by_id(int n, const float4 *__restrict__ src, const uint32_t *__restrict__ ids,
-                            double *__restrict__ out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 v = src[i];
-    double *o = out + 3 * (size_t)ids[i];
-    o[0] = v.x;
-    o[1] = v.y;
-    o[2] = v.z;
-}
-}  // namespace
-
 class IntegratorVerlet {
    public:
     State *s;
@@ -52,7 +26,8 @@ class IntegratorVerlet {
     explicit IntegratorVerlet(State *st) : s(st) {}
     ~IntegratorVerlet() {
         clearGraphs();
-        if (h_stage) cudaFreeHost(h_stage);
+        for (cudaEvent_t e : ev_out)
+            if (e) cudaEventDestroy(e);
     }
     void clearGraphs() {
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
@@ -374,9 +349,7 @@ class IntegratorVerlet {
     // run with host buffers in/out (the call a host program makes): inputs are
     // copied from pinned staging and scattered by id, outputs gathered by id
     // and copied back, all inside the call
-    double *h_stage = nullptr;  // pinned: 3 arrays of (n,3) FP64
-    size_t h_stage_n = 0;
-    DBuf<double> d_stage;
+    cudaEvent_t ev_out[3] = {nullptr, nullptr, nullptr};
     int runHost(int nturns, const double *pin, const double *vin, double *pout, double *vout, double *fout) {
         if (s->barostatFix() || (s->nhFix() && s->nhFix()->barostatting)) {
             set_error(MDX_ERR_UNSUPPORTED, "a barostat changes the box between steps: use mdx_integrator_run");
@@ -386,29 +359,18 @@ class IntegratorVerlet {
             clearGraphs();
             if (int e = s->prepare()) return e;
         }
-        const int n = s->gpd.n;
-        const size_t a3 = 3 * (size_t)n;  // doubles per array
-        if (h_stage_n < 3 * a3) {
-            if (h_stage) cudaFreeHost(h_stage);
-            MDX_CUDA_TRY(cudaMallocHost(&h_stage, 3 * a3 * sizeof(double)));
-            h_stage_n = 3 * a3;
-        }
-        if (int e = d_stage.alloc(3 * a3)) return e;
+        const size_t bytes = 3 * (size_t)s->gpd.n * sizeof(double);
+        if (int e = s->stageAlloc()) return e;
+        for (cudaEvent_t &e : ev_out)
+            if (!e) MDX_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         // the step graphs of this call exist before any copy is queued
         if (int e = precapture(nturns, 0)) return e;
         // inputs: a plain copy into pinned memory, one async copy each, the
         // FP32 rounding and the scatter by id on the device
         const double *ins[2] = {pin, vin};
-        float4 *dsts[2] = {s->gpd.xs.p, s->gpd.vs.p};
-        for (int k = 0; k < 2; k++) {
-            if (!ins[k]) continue;
-            double *h = h_stage + k * a3;
-            std::memcpy(h, ins[k], a3 * sizeof(double));
-            MDX_CUDA_TRY(cudaMemcpyAsync(d_stage.p + k * a3, h, a3 * sizeof(double), cudaMemcpyHostToDevice,
-                                         s->stream));
-            k_put_by_id<<<(n + 255) / 256, 256, 0, s->stream>>>(n, d_stage.p + k * a3, s->gpd.idToIdx.p, dsts[k]);
-            MDX_LAUNCHED();
-        }
+        for (int k = 0; k < 2; k++)
+            if (ins[k])
+                if (int e = s->stagePut(k, ins[k])) return e;
         const int P = s->periodicInterval > 0 ? s->periodicInterval : 1;
         int done = 0;
         while (done < nturns) {
@@ -422,20 +384,21 @@ class IntegratorVerlet {
         }
         if (nturns > 0)
             if (int e = nh_end_of_run(*s)) return e;
+        // outputs: each array is copied out while the next one crosses
         double *outs[3] = {pout, vout, fout};
-        const float4 *srcs[3] = {s->gpd.xs.p, s->gpd.vs.p, s->gpd.fs.p};
-        for (int k = 0; k < 3; k++) {
-            if (!outs[k]) continue;
-            k_get_by_id<<<(n + 255) / 256, 256, 0, s->stream>>>(n, srcs[k], s->gpd.ids.p, d_stage.p + k * a3);
-            MDX_LAUNCHED();
-            MDX_CUDA_TRY(cudaMemcpyAsync(h_stage + k * a3, d_stage.p + k * a3, a3 * sizeof(double),
-                                         cudaMemcpyDeviceToHost, s->stream));
-        }
         MDX_CUDA_TRY(cudaMemcpyAsync(s->h_status, s->d_status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost,
                                      s->stream));
+        for (int k = 0; k < 3; k++) {
+            if (!outs[k]) continue;
+            if (int e = s->stageGet(k)) return e;
+            MDX_CUDA_TRY(cudaEventRecord(ev_out[k], s->stream));
+        }
+        for (int k = 0; k < 3; k++) {
+            if (!outs[k]) continue;
+            MDX_CUDA_TRY(cudaEventSynchronize(ev_out[k]));
+            host_copy(outs[k], s->stageHost(k), bytes);
+        }
         MDX_CUDA_TRY(cudaStreamSynchronize(s->stream));
-        for (int k = 0; k < 3; k++)
-            if (outs[k]) std::memcpy(outs[k], h_stage + k * a3, a3 * sizeof(double));
         if (s->h_status->bits) return s->checkStatus();
         return 0;
     }

@@ -7,6 +7,9 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <system_error>
+#include <thread>
+#include <vector>
 
 #include "engine.hpp"
 
@@ -53,6 +56,7 @@ State::State() {
 
 State::~State() {
     if (h_status) cudaFreeHost(h_status);
+    if (stage_h) cudaFreeHost(stage_h);
     for (int k = 0; k < 3; k++) {
         if (side[k]) cudaStreamDestroy(side[k]);
         if (ev_join[k]) cudaEventDestroy(ev_join[k]);
@@ -185,25 +189,105 @@ int State::upload() {
     return 0;
 }
 
-// device -> host atoms, back in id order
+void host_copy(void *dst, const void *src, size_t bytes) {
+    // one core copies about 10 GB/s (less into pages it touches first); a
+    // thread costs some 20 us to start: worth it from 2 MB
+    const size_t parts = std::min<size_t>(4, bytes >> 20);
+    if (parts < 2) {
+        std::memcpy(dst, src, bytes);
+        return;
+    }
+    const size_t chunk = (bytes / parts + 4095) / 4096 * 4096;
+    std::vector<std::thread> th;
+    th.reserve(parts);
+    size_t at = chunk;  // the first chunk is this thread's
+    try {
+        for (; at < bytes; at += chunk)
+            th.emplace_back([=] {
+                std::memcpy((char *)dst + at, (const char *)src + at, std::min(chunk, bytes - at));
+            });
+    } catch (const std::system_error &) {  // no more threads: the rest here
+        std::memcpy((char *)dst + at, (const char *)src + at, bytes - at);
+    }
+    std::memcpy(dst, src, std::min(chunk, bytes));
+    for (std::thread &t : th) t.join();
+}
+
+namespace {
+// (n,3) FP64 arrays by atom id, rounded to FP32 here (the host cast's
+// round-to-nearest) into the sorted streams, and widened back out; .w is kept
+__global__ void k_put_by_id(int n, const double *__restrict__ in, const int *__restrict__ idToIdx,
+                            float4 *__restrict__ dst) {
+    int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= n) return;
+    const int i = idToIdx[id];
+    const float w = dst[i].w;
+    const double *v = in + 3 * (size_t)id;
+    dst[i] = make_float4((float)v[0], (float)v[1], (float)v[2], w);
+}
+__global__ void k_get_by_id(int n, const float4 *__restrict__ src, const uint32_t *__restrict__ ids,
+                            double *__restrict__ out) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 v = src[i];
+    double *o = out + 3 * (size_t)ids[i];
+    o[0] = v.x;
+    o[1] = v.y;
+    o[2] = v.z;
+}
+}  // namespace
+
+int State::stageAlloc() {
+    const size_t need = 9 * (size_t)gpd.n;
+    if (stage_n < need) {
+        if (stage_h) cudaFreeHost(stage_h);
+        stage_h = nullptr;
+        stage_n = 0;
+        MDX_CUDA_TRY(cudaMallocHost(&stage_h, need * sizeof(double)));
+        stage_n = need;
+    }
+    return stage_d.alloc(need);
+}
+
+int State::stagePut(int k, const double *src) {
+    const int n = gpd.n;
+    const size_t bytes = 3 * (size_t)n * sizeof(double);
+    double *const d = stage_d.p + 3 * (size_t)k * n;
+    host_copy(stageHost(k), src, bytes);
+    MDX_CUDA_TRY(cudaMemcpyAsync(d, stageHost(k), bytes, cudaMemcpyHostToDevice, stream));
+    k_put_by_id<<<(n + 255) / 256, 256, 0, stream>>>(n, d, gpd.idToIdx.p, k == 0 ? gpd.xs.p : gpd.vs.p);
+    MDX_LAUNCHED();
+    return 0;
+}
+
+int State::stageGet(int k) {
+    const int n = gpd.n;
+    double *const d = stage_d.p + 3 * (size_t)k * n;
+    k_get_by_id<<<(n + 255) / 256, 256, 0, stream>>>(n, k == 0 ? gpd.xs.p : (k == 1 ? gpd.vs.p : gpd.fs.p), gpd.ids.p,
+                                                     d);
+    MDX_LAUNCHED();
+    MDX_CUDA_TRY(cudaMemcpyAsync(stageHost(k), d, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    return 0;
+}
+
+// device -> host atoms, by id
 int State::download() {
     if (!uploaded) return 0;
     const int n = gpd.n;
-    std::vector<float4> xs(n), vs(n), fs(n);
-    std::vector<uint32_t> ids(n);
+    if (int e = stageAlloc()) return e;
+    for (int k = 0; k < 3; k++)
+        if (int e = stageGet(k)) return e;
+    MDX_CUDA_TRY(cudaMemcpyAsync(h_status, d_status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, stream));
     MDX_CUDA_TRY(cudaStreamSynchronize(stream));
-    MDX_CUDA_TRY(cudaMemcpy(xs.data(), gpd.xs.p, n * sizeof(float4), cudaMemcpyDeviceToHost));
-    MDX_CUDA_TRY(cudaMemcpy(vs.data(), gpd.vs.p, n * sizeof(float4), cudaMemcpyDeviceToHost));
-    MDX_CUDA_TRY(cudaMemcpy(fs.data(), gpd.fs.p, n * sizeof(float4), cudaMemcpyDeviceToHost));
-    MDX_CUDA_TRY(cudaMemcpy(ids.data(), gpd.ids.p, n * sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    DeviceStatus st;
-    MDX_CUDA_TRY(cudaMemcpy(&st, d_status.p, sizeof(st), cudaMemcpyDeviceToHost));
-    turn = st.turn;
-    for (int i = 0; i < n; i++) {
-        HostAtom &a = atoms[ids[i]];
-        a.pos[0] = xs[i].x; a.pos[1] = xs[i].y; a.pos[2] = xs[i].z;
-        a.vel[0] = vs[i].x; a.vel[1] = vs[i].y; a.vel[2] = vs[i].z;
-        a.force[0] = fs[i].x; a.force[1] = fs[i].y; a.force[2] = fs[i].z;
+    turn = h_status->turn;
+    const double *x = stageHost(0), *v = stageHost(1), *f = stageHost(2);
+    for (int i = 0; i < n; i++, x += 3, v += 3, f += 3) {
+        HostAtom &a = atoms[i];
+        for (int d = 0; d < 3; d++) {
+            a.pos[d] = x[d];
+            a.vel[d] = v[d];
+            a.force[d] = f[d];
+        }
     }
     return 0;
 }

@@ -369,8 +369,8 @@ __global__ void k_adam(int n, float *__restrict__ w, const float *__restrict__ g
     w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
 }
 
-__global__ void k_to_bf16(int n, const float *__restrict__ w, __nv_bfloat16 *__restrict__ wb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_to_bf16(size_t n, const float *__restrict__ w, __nv_bfloat16 *__restrict__ wb) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) wb[i] = __float2bfloat16(w[i]);
 }
 
@@ -1010,13 +1010,17 @@ int mdx_e3b_surrogate_infer(mdx_state *st, mdx_fix *fix, const float *x, int n, 
     State &s = *st->s;
     S &u = *f->sur;
     const int np = pad16(n) + 64;
-    std::vector<__nv_bfloat16> hb((size_t)np * S::kIn, __float2bfloat16(0.f));
-    for (size_t i = 0; i < (size_t)n * S::kIn; i++) hb[i] = __float2bfloat16(x[i]);
     DBuf<__nv_bfloat16> xd;
     DBuf<float> yd;
-    if (int e = xd.alloc(hb.size())) return e;
+    if (int e = xd.alloc((size_t)np * S::kIn)) return e;
     if (int e = yd.alloc((size_t)np * S::kOut)) return e;
-    MDX_CUDA_TRY(cudaMemcpy(xd.p, hb.data(), hb.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice));
+    // rounded to BF16 on the device; the padding rows are zero
+    const size_t nx = (size_t)n * S::kIn;
+    if (int e = u.xf.alloc(nx)) return e;
+    MDX_CUDA_TRY(cudaMemcpyAsync(u.xf.p, x, nx * sizeof(float), cudaMemcpyHostToDevice, s.stream));
+    MDX_CUDA_TRY(cudaMemsetAsync(xd.p + nx, 0, ((size_t)np * S::kIn - nx) * sizeof(__nv_bfloat16), s.stream));
+    k_to_bf16<<<(unsigned)((nx + 255) / 256), 256, 0, s.stream>>>(nx, u.xf.p, xd.p);
+    MDX_LAUNCHED();
     InferArgs I = infer_args(*f, n, nullptr, 0);
     I.feat = xd.p;
     I.yraw = yd.p;
@@ -1042,10 +1046,12 @@ int mdx_e3b_surrogate_grad(mdx_state *st, mdx_fix *fix, const float *x, const fl
     State &s = *st->s;
     S &u = *f->sur;
     if (int e = sur_batch_alloc(u, n)) return e;
-    std::vector<__nv_bfloat16> hb((size_t)n * S::kIn);
-    for (size_t i = 0; i < hb.size(); i++) hb[i] = __float2bfloat16(x[i]);
-    MDX_CUDA_TRY(cudaMemcpy(u.xb.p, hb.data(), hb.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice));
-    MDX_CUDA_TRY(cudaMemcpy(u.yb.p, t, (size_t)n * S::kOut * sizeof(float), cudaMemcpyHostToDevice));
+    // rounded to BF16 on the device
+    if (int e = u.xf.alloc((size_t)n * S::kIn)) return e;
+    MDX_CUDA_TRY(cudaMemcpyAsync(u.xf.p, x, (size_t)n * S::kIn * sizeof(float), cudaMemcpyHostToDevice, s.stream));
+    k_to_bf16<<<(unsigned)(((size_t)n * S::kIn + 255) / 256), 256, 0, s.stream>>>((size_t)n * S::kIn, u.xf.p, u.xb.p);
+    MDX_LAUNCHED();
+    MDX_CUDA_TRY(cudaMemcpyAsync(u.yb.p, t, (size_t)n * S::kOut * sizeof(float), cudaMemcpyHostToDevice, s.stream));
     if (int e = sur_fwd_bwd(u, n, s.stream)) return e;
     double l = 0.0;
     MDX_CUDA_TRY(cudaMemcpyAsync(&l, u.loss.p, sizeof(double), cudaMemcpyDeviceToHost, s.stream));
