@@ -181,7 +181,7 @@ struct GridGPU {
     float skin = 0.f;    // padding
     DBuf<uint32_t> cell_start, cell_count, cell_fill, block_sums;
     DBuf<int> cell_of;     // per atom (unsorted order)
-    DBuf<int> perm_tmp, perm;  // sort scratch
+    DBuf<int> perm_tmp;    // sort scratch
     DBuf<uint32_t> counts; // per atom neighbour count (all pairs within cut)
     DBuf<uint32_t> counts_int;  // per atom count of pairs that can interact
     DBuf<uint32_t> nlist;  // entries: interacting ones from the front of the

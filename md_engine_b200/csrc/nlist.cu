@@ -63,7 +63,7 @@ struct GridArgs {
     int *idToIdx;
     int *cell_of;
     uint32_t *cell_count, *cell_start, *cell_fill;
-    int *perm_tmp, *perm;
+    int *perm_tmp;
     DeviceStatus *st;
     Box box;
     CellGrid g;
@@ -122,80 +122,93 @@ __global__ void k_wrap_bin(const GridArgs a0, const GridArgs *__restrict__ tab) 
     atomicAdd(A.cell_count + c, 1u);
 }
 
-// exclusive scan of the cell histogram in one block per system (replaces the
-// host cumulativeSum, helpers.h:15-24); also clears the fill counters.  The
-// counts pass through shared memory in tiles of kScanTile cells: coalesced
-// loads and stores, thread t scans its eight consecutive cells in registers,
-// warp and block totals by shuffles, a running carry across tiles.
+// exclusive scan of the cell histogram (replaces the host cumulativeSum,
+// helpers.h:15-24); also clears the fill counters.  A block per tile of
+// kScanTile cells: it sums the counts before its tile itself (coalesced
+// 16-byte loads from L2, no block waits for another), then scans its tile --
+// through shared memory, thread t its eight consecutive cells in registers,
+// warp and block totals by shuffles.  One block walking the tiles one after
+// another took 5.6 us a tile: 74 us for the 104,000 cells of 256,000
+// particles, 6 us so; up to one tile nothing changes.
 constexpr int kScanThreads = 1024;
 constexpr int kScanPer = 8;
 constexpr int kScanTile = kScanThreads * kScanPer;
+inline unsigned scan_tiles(int ncell) { return (unsigned)((ncell + kScanTile - 1) / kScanTile); }
 __global__ void __launch_bounds__(kScanThreads) k_scan_cells(const GridArgs a0, const GridArgs *__restrict__ tab) {
     MDX_GRID_ARGS;
     if (!A.st->rebuild) return;
     const uint32_t *__restrict__ count = A.cell_count;
-    uint32_t *__restrict__ start = A.cell_start;
-    uint32_t *__restrict__ fill = A.cell_fill;
     const int ncell = A.ncell;
+    const int base = (int)blockIdx.x * kScanTile;
+    if (base >= ncell) return;
     __shared__ uint4 tile4[kScanTile / 4];
-    __shared__ uint32_t warp_tot[32];
+    __shared__ uint32_t warp_tot[32], warp_before[32];
     uint32_t *const tile = reinterpret_cast<uint32_t *>(tile4);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    constexpr int nw = kScanThreads / 32;
-    uint32_t carry = 0u;
-    for (int base = 0; base < ncell; base += kScanTile) {
-        const int nt = min(kScanTile, ncell - base);
-#pragma unroll
-        for (int k = 0; k < kScanPer; k++) {
-            const int c = k * kScanThreads + (int)threadIdx.x;
-            tile[c] = c < nt ? count[base + c] : 0u;
+    uint32_t before = 0u;
+    {
+        const uint4 *c4 = reinterpret_cast<const uint4 *>(count);
+#pragma unroll 4
+        for (int k = threadIdx.x; k < base / 4; k += kScanThreads) {
+            const uint4 c = c4[k];
+            before += c.x + c.y + c.z + c.w;
         }
-        __syncthreads();
-        const uint4 a = tile4[2 * threadIdx.x], b = tile4[2 * threadIdx.x + 1];
-        const uint32_t v[kScanPer] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        uint32_t run = 0u;
+    }
 #pragma unroll
-        for (int k = 0; k < kScanPer; k++) run += v[k];
-        uint32_t x = run;
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (lane == 0) warp_before[w] = before;
+    const int nt = min(kScanTile, ncell - base);
+#pragma unroll
+    for (int k = 0; k < kScanPer; k++) {
+        const int c = k * kScanThreads + (int)threadIdx.x;
+        tile[c] = c < nt ? count[base + c] : 0u;
+    }
+    __syncthreads();
+    const uint4 a = tile4[2 * threadIdx.x], b = tile4[2 * threadIdx.x + 1];
+    const uint32_t v[kScanPer] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t run = 0u;
+#pragma unroll
+    for (int k = 0; k < kScanPer; k++) run += v[k];
+    uint32_t x = run;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_tot[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        uint32_t t = warp_tot[lane], bf = warp_before[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) bf += __shfl_xor_sync(0xffffffffu, bf, o);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += y;
         }
-        if (lane == 31) warp_tot[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            uint32_t t = warp_tot[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-                if (lane >= o) t += y;
-            }
-            warp_tot[lane] = t;
-        }
-        __syncthreads();
-        uint32_t excl = carry + (w > 0 ? warp_tot[w - 1] : 0u) + x - run;
-        uint32_t e[kScanPer];
-#pragma unroll
-        for (int k = 0; k < kScanPer; k++) {
-            e[k] = excl;
-            excl += v[k];
-        }
-        tile4[2 * threadIdx.x] = make_uint4(e[0], e[1], e[2], e[3]);
-        tile4[2 * threadIdx.x + 1] = make_uint4(e[4], e[5], e[6], e[7]);
-        carry += warp_tot[nw - 1];
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kScanPer; k++) {
-            const int c = k * kScanThreads + (int)threadIdx.x;
-            if (c < nt) {
-                start[base + c] = tile[c];
-                fill[base + c] = 0u;
-            }
-        }
-        __syncthreads();  // tile and warp_tot are reused by the next tile
+        warp_tot[lane] = bf + t;  // everything up to and with the warp
     }
-    if (threadIdx.x == 0) start[ncell] = carry;
+    __syncthreads();
+    const uint32_t last = warp_tot[w];
+    uint32_t excl = last - __shfl_sync(0xffffffffu, x, 31) + x - run;
+    uint32_t e[kScanPer];
+#pragma unroll
+    for (int k = 0; k < kScanPer; k++) {
+        e[k] = excl;
+        excl += v[k];
+    }
+    tile4[2 * threadIdx.x] = make_uint4(e[0], e[1], e[2], e[3]);
+    tile4[2 * threadIdx.x + 1] = make_uint4(e[4], e[5], e[6], e[7]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kScanPer; k++) {
+        const int c = k * kScanThreads + (int)threadIdx.x;
+        if (c < nt) {
+            A.cell_start[base + c] = tile[c];
+            A.cell_fill[base + c] = 0u;
+        }
+    }
+    if (base + nt == ncell && threadIdx.x == kScanThreads - 1) A.cell_start[ncell] = excl;
 }
 
 __global__ void k_scatter(const GridArgs a0, const GridArgs *__restrict__ tab) {
@@ -208,58 +221,46 @@ __global__ void k_scatter(const GridArgs a0, const GridArgs *__restrict__ tab) {
     A.perm_tmp[A.cell_start[c] + slot] = i;
 }
 
-// deterministic order inside each cell: rank by (type, id); one warp per cell
-__global__ void k_rank(const GridArgs a0, const GridArgs *__restrict__ tab) {
-    MDX_GRID_ARGS;
-    if (!A.st->rebuild) return;
-    int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (c >= A.ncell) return;
-    const int *__restrict__ perm_tmp = A.perm_tmp;
-    const float4 *__restrict__ xs = A.xs;
-    const uint32_t *__restrict__ ids = A.ids;
-    uint32_t s = A.cell_start[c], e = A.cell_start[c + 1];
-    for (uint32_t p = s + lane; p < e; p += 32) {
-        int a = perm_tmp[p];
-        unsigned long long ka = ((unsigned long long)(uint32_t)type_of(xs[a]) << 32) | ids[a];
-        uint32_t r = 0;
-        for (uint32_t q = s; q < e; q++) {
-            int b = perm_tmp[q];
-            unsigned long long kb = ((unsigned long long)(uint32_t)type_of(xs[b]) << 32) | ids[b];
-            r += kb < ka;
-        }
-        A.perm[s + r] = a;
-    }
-}
-
-// sortPerAtomArrays (GridGPU.cu:253-293): gather every stream into the
-// alternate buffers and rebuild idToIdx
+// sortPerAtomArrays (GridGPU.cu:253-293): each atom's place in its cell, the
+// rank of (type, id) among the cell's few atoms (deterministic order), then
+// every stream into the alternate buffers and idToIdx rebuilt.  One thread per
+// atom (a warp per cell had most lanes idle at two atoms a cell: 28 us and a
+// launch of its own at 256,000 atoms).  The histogram is cleared for the next
+// build.
 __global__ void k_gather(const GridArgs a0, const GridArgs *__restrict__ tab) {
     MDX_GRID_ARGS;
     if (!A.st->rebuild) return;
-    int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= A.n) return;
-    int s = A.perm[d];
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int c = p; c < A.ncell; c += gridDim.x * blockDim.x) A.cell_count[c] = 0u;
+    if (p >= A.n) return;
+    const int s = A.perm_tmp[p];
+    const int c = A.cell_of[s];
+    const uint32_t beg = A.cell_start[c], end = A.cell_start[c + 1];
+    float4 x = A.xs[s];
+    const uint32_t id = A.ids[s];
+    const unsigned long long ka = ((unsigned long long)(uint32_t)type_of(x) << 32) | id;
+    uint32_t d = beg;
+    for (uint32_t q = beg; q < end; q++) {
+        const int b = A.perm_tmp[q];
+        const unsigned long long kb = ((unsigned long long)(uint32_t)type_of(A.xs[b]) << 32) | A.ids[b];
+        d += kb < ka;
+    }
     if (A.view) {
         // the view build's copy, wrapped as k_wrap_bin wraps in place
         const Box &box = A.box;
-        float4 p = A.xs[s];
-        const float ix = floorf((p.x - box.lo.x) / box.L.x);
-        const float iy = floorf((p.y - box.lo.y) / box.L.y);
-        const float iz = floorf((p.z - box.lo.z) / box.L.z);
+        const float ix = floorf((x.x - box.lo.x) / box.L.x);
+        const float iy = floorf((x.y - box.lo.y) / box.L.y);
+        const float iz = floorf((x.z - box.lo.z) / box.L.z);
         if (ix != 0.f || iy != 0.f || iz != 0.f) {
-            p.x = p.x - box.L.x * ix;
-            p.y = p.y - box.L.y * iy;
-            p.z = p.z - box.L.z * iz;
+            x.x = x.x - box.L.x * ix;
+            x.y = x.y - box.L.y * iy;
+            x.z = x.z - box.L.z * iz;
         }
-        A.xs2[d] = p;
-    } else {
-        A.xs2[d] = A.xs[s];
     }
+    A.xs2[d] = x;
     A.vs2[d] = A.vs[s];
     A.fs2[d] = A.fs[s];
     A.qs2[d] = A.qs[s];
-    uint32_t id = A.ids[s];
     A.ids2[d] = id;
     if (!A.view) A.idToIdx[id] = d;
 }
@@ -644,17 +645,13 @@ __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(con
     }
 }
 
-// single block: every thread must read the flag before it is cleared
+// the rebuild is over (one thread; the histogram was cleared by the sort)
 __global__ void k_finish(const GridArgs a0, const GridArgs *__restrict__ tab) {
     MDX_GRID_ARGS;
     DeviceStatus *st = A.st;
     if (!st->rebuild) return;
-    for (int c = threadIdx.x; c < A.ncell; c += blockDim.x) A.cell_count[c] = 0u;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (!A.view) st->n_builds += 1;
-        st->rebuild = 0u;
-    }
+    if (!A.view) st->n_builds += 1;
+    st->rebuild = 0u;
 }
 
 // ---- molecule form (all-rigid four-site water) ---------------------------
@@ -740,39 +737,33 @@ __global__ void k_mf_scatter(const MolGridArgs m0, const MolGridArgs *__restrict
     M.perm_tmp[M.cell_start[c] + slot] = m;
 }
 
-// deterministic order inside each cell: by molecule index; one warp per cell
-__global__ void k_mf_rank(const MolGridArgs m0, const MolGridArgs *__restrict__ tab) {
-    MDX_MG_ARGS;
-    if (!M.st->rebuild) return;
-    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (c >= M.ncell) return;
-    const uint32_t s = M.cell_start[c], e = M.cell_start[c + 1];
-    for (uint32_t p = s + lane; p < e; p += 32) {
-        const int a = M.perm_tmp[p];
-        uint32_t r = 0;
-        for (uint32_t q = s; q < e; q++) r += M.perm_tmp[q] < a;
-        M.perm[s + r] = a;
-    }
-}
-
-// slot d <- molecule perm[d]: its four sites into 4d .. 4d+3 of the
-// alternate streams and idToIdx rewritten; one thread per site
+// each molecule's slot d, by its rank among the cell's molecule indices
+// (deterministic), its four sites into 4d .. 4d+3 of the alternate streams and
+// idToIdx rewritten; one thread per site (the four of a molecule each work out
+// the rank).  The histogram is cleared for the next build
 __global__ void k_mf_gather(const MolGridArgs m0, const MolGridArgs *__restrict__ tab) {
     MDX_MG_ARGS;
     if (!M.st->rebuild) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int c = t; c < M.ncell; c += gridDim.x * blockDim.x) M.cell_count[c] = 0u;
     if (t >= 4 * M.nmol) return;
-    const int d = t >> 2, site = t & 3;
-    const int4 ix = M.mol_idx[M.perm[d]];
+    const int site = t & 3;
+    const int a = M.perm_tmp[t >> 2];
+    const int c = M.cell_of[a];
+    const uint32_t beg = M.cell_start[c], end = M.cell_start[c + 1];
+    const int4 ix = M.mol_idx[a];
+    uint32_t d = beg;
+    for (uint32_t q = beg; q < end; q++) d += M.perm_tmp[q] < a;
+    if (site == 0) M.perm[d] = a;
     const int s = site == 0 ? ix.x : (site == 1 ? ix.y : (site == 2 ? ix.z : ix.w));
-    M.xs2[t] = M.xs[s];
-    M.vs2[t] = M.vs[s];
-    M.fs2[t] = M.fs[s];
-    M.qs2[t] = M.qs[s];
+    const int o = 4 * (int)d + site;
+    M.xs2[o] = M.xs[s];
+    M.vs2[o] = M.vs[s];
+    M.fs2[o] = M.fs[s];
+    M.qs2[o] = M.qs[s];
     const uint32_t id = M.ids[s];
-    M.ids2[t] = id;
-    M.idToIdx[id] = t;
+    M.ids2[o] = id;
+    M.idToIdx[id] = o;
 }
 
 // the sorted streams back into the primary buffers, the positions of this
@@ -922,7 +913,6 @@ GridArgs grid_args(State &s) {
     A.cell_start = gr.cell_start.p;
     A.cell_fill = gr.cell_fill.p;
     A.perm_tmp = gr.perm_tmp.p;
-    A.perm = gr.perm.p;
     A.st = s.d_status.p;
     A.box = s.box;
     A.g = make_grid(s);
@@ -1173,8 +1163,11 @@ int nlist_set_interactions(State &s) {
             if (pf->pairActive(a, b)) mask[a] |= 1u << b;
     if (int e = gr.ljmask.alloc(nt)) return e;
     MDX_CUDA_TRY(cudaMemcpy(gr.ljmask.p, mask.data(), nt * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    gr.partition = true;
     gr.part_q = pf->chargeFix != nullptr || pf->dsfFix != nullptr;
+    // without charges and with no zero pair there is nothing to split off
+    bool all = true;
+    for (int a = 0; a < nt; a++) all = all && mask[a] == (nt == 32 ? 0xffffffffu : (1u << nt) - 1u);
+    gr.partition = gr.part_q || !all;
     return 0;
 }
 
@@ -1233,7 +1226,6 @@ int nlist_init(State &s) {
     const int n = s.gpd.n;
     if (int e = gr.cell_of.alloc(n)) return e;
     if (int e = gr.perm_tmp.alloc(n)) return e;
-    if (int e = gr.perm.alloc(n)) return e;
     if (int e = gr.counts.alloc(n)) return e;
     if (int e = gr.counts_int.alloc(n)) return e;
     if (s.nThreadPerAtom > 0) {
@@ -1245,6 +1237,15 @@ int nlist_init(State &s) {
         double vol = s.box.Ld.x * s.box.Ld.y * s.box.Ld.z;
         double nbar = n / vol * 4.18879 * (double)gr.cut * gr.cut * gr.cut;
         gr.team = nbar > 400 ? 32 : (nbar > 256 ? 16 : (nbar > 128 ? 8 : (nbar > 48 ? 4 : 2)));
+        // a small system leaves lanes idle and waits for each row's chain of
+        // gathers: wider teams while they fit the SMs, fewer beside a P3M
+        // chain.  Measured on B200, us per step at team 4, 8, 16, 32 -- LJ
+        // fluid 1,500: 17.2 13.9 12.7 11.8; 4,000: 19.0 16.1 14.9 15.3; 8,000:
+        // 19.9 16.8 16.9 17.7; 16,000: 21.9 19.9 21.5 23.6; 32,000: 26.9 27.7
+        // 30.0; salt with P3M 2,000: 28.8 26.6 26.6 26.5; 8,000: 38.7 35.2
+        // 38.0 40.6; 24,000: 65.6 69.4 70.7
+        const double lanes = (s.ewaldFix() ? 640.0 : 880.0) * num_sms();
+        while (gr.team < 32 && gr.team < nbar && 2.0 * gr.team * n <= lanes) gr.team *= 2;
     }
     if (gr.team != 1 && gr.team != 2 && gr.team != 4 && gr.team != 8 && gr.team != 16 && gr.team != 32) {
         set_error(MDX_ERR_ARG, "nThreadPerAtom must be 1,2,4,8,16 or 32 (got %d)", gr.team);
@@ -1276,9 +1277,8 @@ int nlist_rebuild(State &s, bool force, bool conditional, cudaStream_t bstream) 
     const GridArgs *nt = nullptr;
     MDX_CUDA_TRY(launch_pdl(k_check, dim3(nb), dim3(256), 0, s.stream, A, nt, force ? 1 : 0));
     MDX_CUDA_TRY(launch_pdl(k_wrap_bin, dim3(nb), dim3(256), 0, s.stream, A, nt));
-    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(1), dim3(kScanThreads), 0, s.stream, A, nt));
+    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_tiles(A.ncell)), dim3(kScanThreads), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_scatter, dim3(nb), dim3(256), 0, s.stream, A, nt));
-    MDX_CUDA_TRY(launch_pdl(k_rank, dim3((ncell * 32 + 255) / 256), dim3(256), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_gather, dim3(nb), dim3(256), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_copyback, dim3(nb), dim3(256), 0, s.stream, A, nt));
     // molecule maps of the fixes that keep atom indices
@@ -1309,7 +1309,7 @@ int nlist_rebuild(State &s, bool force, bool conditional, cudaStream_t bstream) 
     if (FixE3B *e3 = s.e3bFix()) {
         if (int e = e3b_build_list(s, *e3, true, bs)) return e;
     }
-    MDX_CUDA_TRY(launch_pdl(k_finish, dim3(1), dim3(1024), 0, bs, A, (const GridArgs *)nullptr));
+    MDX_CUDA_TRY(launch_pdl(k_finish, dim3(1), dim3(1), 0, bs, A, (const GridArgs *)nullptr));
     if (bs != s.stream) MDX_CUDA_TRY(cudaEventRecord(s.ev_join[2], bs));
     gr.built = true;
     return 0;
@@ -1328,9 +1328,8 @@ static int nlist_rebuild_mf(State &s, bool force, cudaStream_t bstream) {
     const int nb_mol = (M.nmol + 255) / 256;
     MDX_CUDA_TRY(launch_pdl(k_check, dim3(nb_atoms), dim3(256), 0, s.stream, A, nt, force ? 1 : 0));
     MDX_CUDA_TRY(launch_pdl(k_mf_wrap_bin, dim3(nb_mol), dim3(256), 0, s.stream, M, mnt));
-    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(1), dim3(kScanThreads), 0, s.stream, Am, nt));
+    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_tiles(Am.ncell)), dim3(kScanThreads), 0, s.stream, Am, nt));
     MDX_CUDA_TRY(launch_pdl(k_mf_scatter, dim3(nb_mol), dim3(256), 0, s.stream, M, mnt));
-    MDX_CUDA_TRY(launch_pdl(k_mf_rank, dim3((M.ncell * 32 + 255) / 256), dim3(256), 0, s.stream, M, mnt));
     MDX_CUDA_TRY(launch_pdl(k_mf_gather, dim3((4 * M.nmol + 255) / 256), dim3(256), 0, s.stream, M, mnt));
     MDX_CUDA_TRY(launch_pdl(k_mf_copyback, dim3((4 * M.nmol + 255) / 256), dim3(256), 0, s.stream, M, mnt));
     cudaStream_t bs = s.stream;
@@ -1343,7 +1342,7 @@ static int nlist_rebuild_mf(State &s, bool force, cudaStream_t bstream) {
     if (FixE3B *e3 = s.e3bFix()) {
         if (int e = e3b_build_list_mf(s, *e3, bs)) return e;
     }
-    MDX_CUDA_TRY(launch_pdl(k_finish, dim3(1), dim3(1024), 0, bs, Am, nt));
+    MDX_CUDA_TRY(launch_pdl(k_finish, dim3(1), dim3(1), 0, bs, Am, nt));
     if (bs != s.stream) MDX_CUDA_TRY(cudaEventRecord(s.ev_join[2], bs));
     s.grid.built = true;
     return 0;
@@ -1365,9 +1364,8 @@ int nlist_build_atoms_view(State &s) {
     const GridArgs *nt = nullptr;
     MDX_CUDA_TRY(launch_pdl(k_check, dim3(nb), dim3(256), 0, s.stream, A, nt, 1));
     MDX_CUDA_TRY(launch_pdl(k_wrap_bin, dim3(nb), dim3(256), 0, s.stream, A, nt));
-    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(1), dim3(kScanThreads), 0, s.stream, A, nt));
+    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_tiles(A.ncell)), dim3(kScanThreads), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_scatter, dim3(nb), dim3(256), 0, s.stream, A, nt));
-    MDX_CUDA_TRY(launch_pdl(k_rank, dim3((ncell * 32 + 255) / 256), dim3(256), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_gather, dim3(nb), dim3(256), 0, s.stream, A, nt));
     if (gr.cap == 0) {
         MDX_CUDA_TRY(cudaMemsetAsync(&s.d_status.p->max_neighbors, 0, sizeof(uint32_t), s.stream));
@@ -1383,7 +1381,7 @@ int nlist_build_atoms_view(State &s) {
         if (int e = gr.nlist.alloc(groups * (size_t)c * (32 / gr.team))) return e;
     }
     launch_build(s, g, cutsq, s.stream);
-    MDX_CUDA_TRY(launch_pdl(k_finish, dim3(1), dim3(1024), 0, s.stream, A, nt));
+    MDX_CUDA_TRY(launch_pdl(k_finish, dim3(1), dim3(1), 0, s.stream, A, nt));
     return 0;
 }
 
@@ -1637,15 +1635,14 @@ static void batch_rebuild_sites(Batch &b, cudaStream_t st) {
     B.ncell = b.max_cell_ps;
     const dim3 nb((b.max_n_ps + 255) / 256, P);
     k_wrap_bin<<<nb, 256, 0, st>>>(A, tg);
-    k_scan_cells<<<dim3(1, P), kScanThreads, 0, st>>>(A, tg);
+    k_scan_cells<<<dim3(scan_tiles(A.ncell), P), kScanThreads, 0, st>>>(A, tg);
     k_scatter<<<nb, 256, 0, st>>>(A, tg);
-    k_rank<<<dim3((b.max_cell_ps * 32 + 255) / 256, P), 256, 0, st>>>(A, tg);
     k_gather<<<nb, 256, 0, st>>>(A, tg);
     k_copyback<<<nb, 256, 0, st>>>(A, tg);
     int hg = 2;
     for (int r : b.ps) hg = std::max(hg, b.reps[r]->grid.home_group);
     launch_build_any<false>(s0.grid.team, hg, build_grid(b.max_cell_ps, P), st, B, tb);
-    g_launches += 6;
+    g_launches += 5;
 }
 
 // the molecule-form replicas' sort by molecule and molecule-pair list
@@ -1662,13 +1659,12 @@ static void batch_rebuild_mols(Batch &b, cudaStream_t st) {
     M.ncell = b.max_mcell;
     const int nb_mol = (b.max_mol_mf + 255) / 256, nb_site = (4 * b.max_mol_mf + 255) / 256;
     k_mf_wrap_bin<<<dim3(nb_mol, Q), 256, 0, st>>>(M, tm);
-    k_scan_cells<<<dim3(1, Q), kScanThreads, 0, st>>>(Am, ts);
+    k_scan_cells<<<dim3(scan_tiles(Am.ncell), Q), kScanThreads, 0, st>>>(Am, ts);
     k_mf_scatter<<<dim3(nb_mol, Q), 256, 0, st>>>(M, tm);
-    k_mf_rank<<<dim3((b.max_mcell * 32 + 255) / 256, Q), 256, 0, st>>>(M, tm);
     k_mf_gather<<<dim3(nb_site, Q), 256, 0, st>>>(M, tm);
     k_mf_copyback<<<dim3(nb_site, Q), 256, 0, st>>>(M, tm);
     k_mf_build<<<dim3(b.max_mol_mf, Q), kMfBuildThreads, 0, st>>>(M, tm);
-    g_launches += 7;
+    g_launches += 6;
 }
 
 int batch_nlist_rebuild(Batch &b) {
@@ -1695,13 +1691,13 @@ int batch_nlist_rebuild(Batch &b) {
     if (!b.ps.empty()) {
         GridArgs Ap = A;
         Ap.n = b.max_n_ps;
-        k_finish<<<dim3(1, (unsigned)b.ps.size()), 1024, 0, st>>>(Ap, reinterpret_cast<const GridArgs *>(b.tab_grid_ps.p));
+        k_finish<<<dim3(1, (unsigned)b.ps.size()), 1, 0, st>>>(Ap, reinterpret_cast<const GridArgs *>(b.tab_grid_ps.p));
         MDX_LAUNCHED();
     }
     if (!b.mfi.empty()) {
         GridArgs Am = mol_scan_args(*b.reps[b.mfi[0]]);
         Am.ncell = b.max_mcell;
-        k_finish<<<dim3(1, (unsigned)b.mfi.size()), 1024, 0, st>>>(Am, reinterpret_cast<const GridArgs *>(b.tab_molscan.p));
+        k_finish<<<dim3(1, (unsigned)b.mfi.size()), 1, 0, st>>>(Am, reinterpret_cast<const GridArgs *>(b.tab_molscan.p));
         MDX_LAUNCHED();
     }
     MDX_CUDA_TRY(cudaGetLastError());
