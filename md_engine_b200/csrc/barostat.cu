@@ -13,7 +13,7 @@ namespace mdx {
 
 int pressure_now(State &s, double *pressure, double virial6[6]) {
     const int n = s.gpd.n;
-    DBuf<float4> keep;
+    DBuf<float4> &keep = s.f_keep;
     if (int e = keep.alloc(n)) return e;
     MDX_CUDA_TRY(cudaMemcpyAsync(keep.p, s.gpd.fs.p, (size_t)n * sizeof(float4), cudaMemcpyDeviceToDevice, s.stream));
     if (int e = s.computeForces(1)) return e;

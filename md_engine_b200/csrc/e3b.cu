@@ -840,12 +840,12 @@ int e3b_energy(State &s, FixE3B &f, double out[2]) {
     const int nmol = (int)f.mol_ids.size();
     out[0] = out[1] = 0.0;
     if (nmol == 0) return 0;
-    DBuf<double> acc;
+    DBuf<double> &acc = f.e_acc;
     if (int e = acc.alloc(2)) return e;
     MDX_CUDA_TRY(cudaMemsetAsync(acc.p, 0, 2 * sizeof(double), s.stream));
     const dim3 blocks = e3b_blocks(nmol);
     // totals are needed by the energy pass: run the force-less totals first
-    DBuf<float4> ftmp;
+    DBuf<float4> &ftmp = s.f_keep;
     if (int e = ftmp.alloc(s.gpd.n)) return e;
     MDX_CUDA_TRY(cudaMemcpyAsync(ftmp.p, s.gpd.fs.p, s.gpd.n * sizeof(float4), cudaMemcpyDeviceToDevice, s.stream));
     E3BArgs A = e3b_args(s, f, ftmp.p);

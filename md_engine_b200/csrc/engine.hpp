@@ -396,6 +396,7 @@ class FixE3B : public Fix {
     DBuf<uint32_t> mcounts, mlist;  // molecule neighbour list (full, team layout)
     DBuf<uint32_t> ccounts, clist;  // per step: the forces pass's partners (mj > m within rmax)
     DBuf<float4> totals;
+    DBuf<double> e_acc;   // the two energies
     DBuf<float4> f_side;  // per-step E3B forces when run beside the pair kernel
     bool side_ok = false; // molecules identical to FixRigid's, in the same order
     int mteam = 8, mcap = 0;
@@ -536,10 +537,13 @@ class State {
     DeviceStatus *h_status = nullptr;  // pinned
     DBuf<double> red_partials;
     DBuf<double> red_out;
-    // per-site pair energies and their FP64 sum (energy evaluations outside
-    // the step; sized at upload so that no evaluation allocates)
+    // per-site pair energies (energy evaluations outside the step), the
+    // partial rows and results of FP64 sums, and the forces put aside by an
+    // observable: kept, so that no evaluation after the first allocates
     DBuf<float> e_site;
-    DBuf<double> e_sum;
+    DBuf<double> sum_partials, sum_out;
+    DBuf<float4> f_keep;
+    int sumsAlloc();
     cudaStream_t stream = nullptr;
     bool own_stream = true;
     int device = -1;  // the CUDA device the state's buffers and streams live on (set at upload)
@@ -722,7 +726,6 @@ int rigid_validate(State &s, FixRigid &r, uint32_t *n_bad);
 int kinetic_sum(State &s, double *out);
 int nh_prepare(State &s, FixNoseHoover &nh);
 int zero_forces(State &s);
-int device_sum(State &s, const double *src, int n, double *out_host);
 int float_sum(State &s, const float *src, int n, double *out_host);
 int virial_sum(State &s, double out[6]);
 int remove_com_velocity(State &s);

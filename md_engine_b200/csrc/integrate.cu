@@ -774,12 +774,34 @@ __global__ void k_reduce_vec(int n, const double *__restrict__ src, int stride, 
     if (threadIdx.x == 0) out[comp] = b;
 }
 
-__global__ void k_reduce_float(int n, const float *__restrict__ src, int stride, int comp, double *out) {
+// FP64 sums of C columns over n rows of floats (row-major), one partial row
+// per block; k_reduce_rows adds the rows in a fixed order.  One block walking
+// all rows, once per column, took 12 us a column at 16,384 rows
+constexpr int kSumThreads = 256;
+template <int C>
+__global__ void __launch_bounds__(kSumThreads) k_sum_floats(int n, const float *__restrict__ src,
+                                                            double *__restrict__ partials) {
     __shared__ double sh[32];
+    const int i = blockIdx.x * kSumThreads + threadIdx.x;
+    double v[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) v[c] = i < n ? (double)src[(size_t)i * C + c] : 0.0;
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+        const double b = block_sum(v[c], sh);
+        if (threadIdx.x == 0) partials[(size_t)blockIdx.x * C + c] = b;
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kSumThreads) k_reduce_rows(int rows, int cols, const double *__restrict__ partials,
+                                                             double *__restrict__ out) {
+    __shared__ double sh[32];
+    const int c = blockIdx.x;
     double acc = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) acc += (double)src[(size_t)i * stride + comp];
+    for (int r = threadIdx.x; r < rows; r += kSumThreads) acc += partials[(size_t)r * cols + c];
     const double b = block_sum(acc, sh);
-    if (threadIdx.x == 0) out[comp] = b;
+    if (threadIdx.x == 0) out[c] = b;
 }
 
 // zero force xyz (group tag in .w kept) and per-atom virials
@@ -1050,35 +1072,46 @@ int remove_com_velocity(State &s) {
 int kinetic_sum(State &s, double *out) {
     const int n = s.gpd.n;
     const int nb = (n + 255) / 256;
-    DBuf<double> part, o;
-    if (int e = part.alloc(nb)) return e;
-    if (int e = o.alloc(1)) return e;
-    k_mv2<<<nb, 256, 0, s.stream>>>(n, s.gpd.vs.p, part.p);
+    if (int e = s.sumsAlloc()) return e;
+    k_mv2<<<nb, 256, 0, s.stream>>>(n, s.gpd.vs.p, s.sum_partials.p);
     MDX_LAUNCHED();
-    k_reduce_vec<<<1, 256, 0, s.stream>>>(nb, part.p, 1, 0, o.p);
+    k_reduce_rows<<<1, kSumThreads, 0, s.stream>>>(nb, 1, s.sum_partials.p, s.sum_out.p);
     MDX_LAUNCHED();
-    MDX_CUDA_TRY(cudaMemcpyAsync(out, o.p, sizeof(double), cudaMemcpyDeviceToHost, s.stream));
+    MDX_CUDA_TRY(cudaMemcpyAsync(out, s.sum_out.p, sizeof(double), cudaMemcpyDeviceToHost, s.stream));
     MDX_CUDA_TRY(cudaStreamSynchronize(s.stream));
     return 0;
 }
 
-// FP64 sum of n floats on the device (one block, fixed order) into *out_host
+int State::sumsAlloc() {
+    if (int e = sum_partials.alloc(6 * (size_t)((gpd.n + kSumThreads - 1) / kSumThreads))) return e;
+    return sum_out.alloc(8);
+}
+
+// FP64 sum of n floats (at most one per atom) on the device, in a fixed order
 int float_sum(State &s, const float *src, int n, double *out_host) {
-    k_reduce_float<<<1, 256, 0, s.stream>>>(n, src, 1, 0, s.e_sum.p);
+    const int nb = (n + kSumThreads - 1) / kSumThreads;
+    if (n > s.gpd.n) {
+        set_error(MDX_ERR_ARG, "sum of %d values: at most one per atom", n);
+        return MDX_ERR_ARG;
+    }
+    if (int e = s.sumsAlloc()) return e;
+    k_sum_floats<1><<<nb, kSumThreads, 0, s.stream>>>(n, src, s.sum_partials.p);
     MDX_LAUNCHED();
-    MDX_CUDA_TRY(cudaMemcpyAsync(out_host, s.e_sum.p, sizeof(double), cudaMemcpyDeviceToHost, s.stream));
+    k_reduce_rows<<<1, kSumThreads, 0, s.stream>>>(nb, 1, s.sum_partials.p, s.sum_out.p);
+    MDX_LAUNCHED();
+    MDX_CUDA_TRY(cudaMemcpyAsync(out_host, s.sum_out.p, sizeof(double), cudaMemcpyDeviceToHost, s.stream));
     MDX_CUDA_TRY(cudaStreamSynchronize(s.stream));
     return 0;
 }
 
 int virial_sum(State &s, double out6[6]) {
-    DBuf<double> o;
-    if (int e = o.alloc(6)) return e;
-    for (int c = 0; c < 6; c++) {
-        k_reduce_float<<<1, 256, 0, s.stream>>>(s.gpd.n, s.gpd.virials.p, 6, c, o.p);
-        MDX_LAUNCHED();
-    }
-    MDX_CUDA_TRY(cudaMemcpyAsync(out6, o.p, 6 * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
+    const int n = s.gpd.n, nb = (n + kSumThreads - 1) / kSumThreads;
+    if (int e = s.sumsAlloc()) return e;
+    k_sum_floats<6><<<nb, kSumThreads, 0, s.stream>>>(n, s.gpd.virials.p, s.sum_partials.p);
+    MDX_LAUNCHED();
+    k_reduce_rows<<<6, kSumThreads, 0, s.stream>>>(nb, 6, s.sum_partials.p, s.sum_out.p);
+    MDX_LAUNCHED();
+    MDX_CUDA_TRY(cudaMemcpyAsync(out6, s.sum_out.p, 6 * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
     MDX_CUDA_TRY(cudaStreamSynchronize(s.stream));
     return 0;
 }

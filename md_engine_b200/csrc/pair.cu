@@ -581,7 +581,7 @@ int pair_mol_launch(State &s, FixPair &f, int virialMode, bool accumulate, float
 // state's energy buffer, summed on the device in FP64 in a fixed order
 int pair_energy(State &s, FixPair &f, double *out) {
     PairArgs A = make_args(s, f);
-    if (s.e_site.n < (size_t)A.n || !s.e_sum.p) {
+    if (s.e_site.n < (size_t)A.n) {
         set_error(MDX_ERR_STATE, "energy buffers not sized (prepare the state)");
         return MDX_ERR_STATE;
     }

@@ -158,7 +158,7 @@ int State::upload() {
     if (int e = d.virials.alloc(6 * (size_t)n)) return e;
     if (int e = red_out.alloc(4)) return e;
     if (int e = e_site.alloc(n)) return e;
-    if (int e = e_sum.alloc(1)) return e;
+    if (int e = sumsAlloc()) return e;
     MDX_CUDA_TRY(cudaMemset(d.virials.p, 0, 6 * (size_t)n * sizeof(float)));
     std::vector<float4> xs(n), vs(n), fs(n);
     std::vector<float> qs(n);
