@@ -67,7 +67,7 @@ void Batch::reset() {
     }
     fft.clear();
     for (DBuf<char> *t : {&tab_pair, &tab_grid, &tab_grid_ps, &tab_build, &tab_p3m, &tab_e3b, &tab_first,
-                          &tab_second, &tab_end, &tab_molgrid, &tab_molscan, &tab_pairmol, &tab_p3m_mol})
+                          &tab_second, &tab_end, &tab_molgrid, &tab_molscan, &tab_molbuild, &tab_pairmol, &tab_p3m_mol})
         t->release();
     max_n = max_mol = max_cell = 0;
     ps.clear();

@@ -618,7 +618,7 @@ class Batch {
     // tab_build, tab_pair: the per-site ones; tab_molgrid, tab_molscan,
     // tab_pairmol: the molecule-form ones, in the order of ps / mfi)
     std::vector<int> ps, mfi;
-    DBuf<char> tab_grid_ps, tab_molgrid, tab_molscan, tab_pairmol;
+    DBuf<char> tab_grid_ps, tab_molgrid, tab_molscan, tab_molbuild, tab_pairmol;
     int max_n_ps = 0, max_cell_ps = 0, max_mol_mf = 0, max_mcell = 0;
     int pair_big = 0;
     int max_n = 0, max_mol = 0, max_cell = 0;

@@ -354,7 +354,9 @@ __device__ __forceinline__ uint32_t excl_depth(const BuildArgs &A, uint32_t myid
 // SPLIT: interacting pairs to the front of a row, provably zero ones to the
 // back (ljmask, part_q); EXCL: exclusion depths from the id window.  Both are
 // compile-time so that the candidate loop carries no tests for them.
-template <int TP, int HG, bool COUNT, bool SPLIT, bool EXCL>
+// STRIDE 4: the molecule-pair list of the molecule form (molecules by the
+// position of their site 0, at 4 k; neither split nor exclusions).
+template <int TP, int HG, bool COUNT, bool SPLIT, bool EXCL, int STRIDE = 1>
 __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(const BuildArgs a0,
                                                                             const BuildArgs *__restrict__ tab) {
     pdl_wait();
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(con
     // bounding box of the home atoms' positions
     float bxl = 3.0e38f, bxh = -3.0e38f, byl = 3.0e38f, byh = -3.0e38f, bzl = 3.0e38f, bzh = -3.0e38f;
     for (int i = cs + lane; i < ce; i += 32) {
-        const float4 p4 = A.xs2[i];
+        const float4 p4 = A.xs2[STRIDE * i];
         bxl = fminf(bxl, p4.x);
         bxh = fmaxf(bxh, p4.x);
         byl = fminf(byl, p4.y);
@@ -543,7 +545,7 @@ __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(con
             const int i = g0 + k;
             const bool v = i < ce;
             const int ii = v ? i : cs;
-            const float4 p4 = A.xs2[ii];
+            const float4 p4 = A.xs2[STRIDE * ii];
             // an absent home slot sits far outside the box: r^2 overflows to
             // infinity and it never hits
             hx[k] = v ? p4.x : 3.0e37f;
@@ -571,7 +573,7 @@ __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(con
                 const uint32_t e = sh_cand[k];
                 pn = e & ((1u << kCandIdxBits) - 1u);
                 shn = sh_shift[e >> kCandIdxBits];
-                pjn = A.xs2[pn];
+                pjn = A.xs2[STRIDE * pn];
                 if (SPLIT) qn = A.qs2[pn];
                 if (EXCL) idn = A.ids2[pn];
             };
@@ -636,9 +638,9 @@ __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(con
                     atomicMax(&A.st->max_neighbors, cnt);
                 } else {
                     A.counts[i] = cnt;
-                    A.counts_int[i] = ci[k];
+                    if (STRIDE == 1) A.counts_int[i] = ci[k];
                     if (cnt > cap) atomicOr(&A.st->bits, kStatusNlistOverflow);
-                    atomicMax(&A.st->max_neighbors, cnt);
+                    atomicMax(STRIDE == 1 ? &A.st->max_neighbors : &A.st->max_mol_neighbors, cnt);
                 }
             }
         }
@@ -672,13 +674,10 @@ struct MolGridArgs {
     int *cell_of;
     uint32_t *cell_count, *cell_start, *cell_fill;
     int *perm_tmp, *perm;
-    uint32_t *counts, *list;
-    int cap, team;
     DeviceStatus *st;
     Box box;
     CellGrid g;
-    int nmol, ncell, m;
-    float cut2;
+    int nmol, ncell;
 };
 
 // one system (m0) or, for batched replicas, tab[blockIdx.y] (m0 then only
@@ -788,101 +787,6 @@ __global__ void k_mf_copyback(const MolGridArgs m0, const MolGridArgs *__restric
     }
 }
 
-// the molecule-pair list: one block per slot, one thread per row of its
-// (2m+1)^2-row stencil (each row one or two contiguous runs of slots: the
-// grid has at least 2m+1 cells per side, so no cell is seen twice).  A
-// candidate is kept when the minimum-image distance of the site-0 positions
-// is below the list radius.  Two passes over the row: count, a block scan of
-// the row counts, then the writes -- rows in stencil order, candidates in slot
-// order (deterministic) -- into the team layout: slot k's e-th entry at
-// (k/G) cap G + (e/T) 32 + (k%G) T + e%T, G = 32/T.  Every row's cell-start
-// loads and candidate loads are in flight at once instead of one row after
-// another.
-constexpr int kMfBuildThreads = 64;  // >= 49 rows (m <= 3)
-
-__device__ __forceinline__ void mf_row_runs(const MolGridArgs &M, int r, int cx, int cy, int cz, int (&b)[2],
-                                            int (&e)[2]) {
-    const CellGrid &g = M.g;
-    const int mm = M.m, side = 2 * mm + 1;
-    int kx = cx - mm + r / side, ky = cy - mm + r % side;
-    kx = kx < 0 ? kx + g.ns.x : (kx >= g.ns.x ? kx - g.ns.x : kx);
-    ky = ky < 0 ? ky + g.ns.y : (ky >= g.ns.y ? ky - g.ns.y : ky);
-    const int rowbase = (kx * g.ns.y + ky) * g.ns.z;
-    const int zlo = cz - mm, zhi = cz + mm;
-    int za[2], zb[2], nr;
-    if (zlo < 0) {
-        za[0] = zlo + g.ns.z; zb[0] = g.ns.z - 1; za[1] = 0; zb[1] = zhi; nr = 2;
-    } else if (zhi >= g.ns.z) {
-        za[0] = zlo; zb[0] = g.ns.z - 1; za[1] = 0; zb[1] = zhi - g.ns.z; nr = 2;
-    } else {
-        za[0] = zlo; zb[0] = zhi; za[1] = 0; zb[1] = -1; nr = 1;
-    }
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-        b[q] = 0;
-        e[q] = 0;
-        if (q < nr) {
-            b[q] = (int)M.cell_start[rowbase + za[q]];
-            e[q] = (int)M.cell_start[rowbase + zb[q] + 1];
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kMfBuildThreads) k_mf_build(const MolGridArgs m0,
-                                                               const MolGridArgs *__restrict__ tab) {
-    MDX_MG_ARGS;
-    if (!M.st->rebuild) return;
-    const int k = blockIdx.x;
-    if (k >= M.nmol) return;  // block-uniform
-    __shared__ uint32_t sh_cnt[kMfBuildThreads];
-    const int r = threadIdx.x;
-    const int side = 2 * M.m + 1;
-    const bool has_row = r < side * side;
-    const float3 p = f3(M.xs2[4 * k]);
-    const int c = cell_of_pos(M.g, p);
-    const int cz = c % M.g.ns.z, cy = (c / M.g.ns.z) % M.g.ns.y, cx = c / (M.g.ns.z * M.g.ns.y);
-    int b[2] = {0, 0}, e[2] = {0, 0};
-    if (has_row) mf_row_runs(M, r, cx, cy, cz, b, e);
-    // pass 1: this row's hits
-    uint32_t n = 0;
-#pragma unroll
-    for (int q = 0; q < 2; q++)
-        for (int j = b[q]; j < e[q]; j++) {
-            if (j == k) continue;
-            const float3 d = min_image(M.box, f3(M.xs2[4 * j]) - p);
-            n += dot3(d, d) < M.cut2 ? 1u : 0u;
-        }
-    // exclusive scan of the row counts over the block (rows in order)
-    sh_cnt[r] = n;
-    __syncthreads();
-    uint32_t off = 0, tot = 0;
-    for (int q = 0; q < kMfBuildThreads; q++) {
-        const uint32_t v = sh_cnt[q];
-        off += q < r ? v : 0u;
-        tot += v;
-    }
-    // pass 2: the writes
-    const int T = M.team, G = 32 / T;
-    uint32_t *const row = M.list + (size_t)(k / G) * M.cap * G + (k % G) * T;
-    const uint32_t cap = (uint32_t)M.cap;
-    uint32_t pos = off;
-#pragma unroll
-    for (int q = 0; q < 2; q++)
-        for (int j = b[q]; j < e[q]; j++) {
-            if (j == k) continue;
-            const float3 d = min_image(M.box, f3(M.xs2[4 * j]) - p);
-            if (dot3(d, d) < M.cut2) {
-                if (pos < cap) row[(pos / T) * 32u + pos % T] = (uint32_t)j;
-                pos++;
-            }
-        }
-    if (r == 0) {
-        M.counts[k] = tot;
-        if (tot > cap) atomicOr(&M.st->bits, kStatusNlistOverflow);
-        atomicMax(&M.st->max_mol_neighbors, tot);
-    }
-}
-
 CellGrid make_grid(const State &s) {
     CellGrid g;
     g.lo = s.box.lo;
@@ -958,17 +862,11 @@ MolGridArgs mol_grid_args(State &s) {
     M.cell_fill = mf.cell_fill.p;
     M.perm_tmp = mf.perm_tmp.p;
     M.perm = mf.perm.p;
-    M.counts = mf.counts.p;
-    M.list = mf.list.p;
-    M.cap = mf.cap;
-    M.team = mf.team;
     M.st = s.d_status.p;
     M.box = s.box;
     M.g = mol_grid(s);
     M.nmol = mf.nmol;
     M.ncell = mf.ns.x * mf.ns.y * mf.ns.z;
-    M.m = mf.m;
-    M.cut2 = mf.cut * mf.cut;
     return M;
 }
 
@@ -1060,6 +958,29 @@ inline dim3 build_grid(int ncell, int nrep) {
 void launch_build(State &s, const CellGrid &g, float cutsq, cudaStream_t st) {
     const BuildArgs A = build_args(s, g, cutsq);
     launch_build_any<false>(s.grid.team, s.grid.home_group, build_grid(A.ncell, 1), st, A, nullptr);
+}
+
+// the molecule-pair list: rows of 32 lanes, its molecules' site 0 within the
+// list radius of site 0.  k_build_cells over the molecule grid: a warp per
+// cell expands the cell's candidates once for its two or three molecules.  (A
+// block per molecule, a thread per stencil row walking it twice: 60 us at
+// 4,096 molecules, 327 us at 32,768.)
+constexpr int kMolHomes = 2;  // home molecules tested at once
+BuildArgs mol_build_args(State &s) {
+    MolForm &mf = s.mf;
+    BuildArgs A{};
+    A.xs2 = s.gpd.xs_alt.p;
+    A.cell_start = mf.cell_start.p;
+    A.counts = mf.counts.p;
+    A.nlist = mf.list.p;
+    A.st = s.d_status.p;
+    A.g = mol_grid(s);
+    A.box = s.box;
+    A.ncell = mf.ns.x * mf.ns.y * mf.ns.z;
+    A.m = mf.m;
+    A.cap = mf.cap;
+    A.cutsq = mf.cut * mf.cut;
+    return A;
 }
 
 void launch_count(State &s, const CellGrid &g, float cutsq) {
@@ -1338,7 +1259,8 @@ static int nlist_rebuild_mf(State &s, bool force, cudaStream_t bstream) {
         MDX_CUDA_TRY(cudaStreamWaitEvent(bstream, s.ev_sorted, 0));
         bs = bstream;
     }
-    MDX_CUDA_TRY(launch_pdl(k_mf_build, dim3(M.nmol), dim3(kMfBuildThreads), 0, bs, M, mnt));
+    MDX_CUDA_TRY(launch_pdl(k_build_cells<32, kMolHomes, false, false, false, 4>, build_grid(M.ncell, 1),
+                            dim3(kBuildCellsPerBlock * 32), 0, bs, mol_build_args(s), (const BuildArgs *)nullptr));
     if (FixE3B *e3 = s.e3bFix()) {
         if (int e = e3b_build_list_mf(s, *e3, bs)) return e;
     }
@@ -1607,15 +1529,19 @@ int batch_nlist_tables(Batch &b) {
     if (Q) {
         std::vector<MolGridArgs> hm(Q);
         std::vector<GridArgs> hs(Q);
+        std::vector<BuildArgs> hb(Q);
         b.max_mcell = 0;
         for (int q = 0; q < Q; q++) {
             State &s = *b.reps[b.mfi[q]];
             hm[q] = mol_grid_args(s);
             hs[q] = mol_scan_args(s);
+            hb[q] = mol_build_args(s);
             b.max_mcell = std::max(b.max_mcell, hs[q].ncell);
         }
         if (int e = b.tab_molgrid.alloc(Q * sizeof(MolGridArgs))) return e;
         if (int e = b.tab_molscan.alloc(Q * sizeof(GridArgs))) return e;
+        if (int e = b.tab_molbuild.alloc(Q * sizeof(BuildArgs))) return e;
+        MDX_CUDA_TRY(cudaMemcpy(b.tab_molbuild.p, hb.data(), Q * sizeof(BuildArgs), cudaMemcpyHostToDevice));
         MDX_CUDA_TRY(cudaMemcpy(b.tab_molgrid.p, hm.data(), Q * sizeof(MolGridArgs), cudaMemcpyHostToDevice));
         MDX_CUDA_TRY(cudaMemcpy(b.tab_molscan.p, hs.data(), Q * sizeof(GridArgs), cudaMemcpyHostToDevice));
     }
@@ -1663,7 +1589,8 @@ static void batch_rebuild_mols(Batch &b, cudaStream_t st) {
     k_mf_scatter<<<dim3(nb_mol, Q), 256, 0, st>>>(M, tm);
     k_mf_gather<<<dim3(nb_site, Q), 256, 0, st>>>(M, tm);
     k_mf_copyback<<<dim3(nb_site, Q), 256, 0, st>>>(M, tm);
-    k_mf_build<<<dim3(b.max_mol_mf, Q), kMfBuildThreads, 0, st>>>(M, tm);
+    k_build_cells<32, kMolHomes, false, false, false, 4><<<build_grid(b.max_mcell, Q), kBuildCellsPerBlock * 32, 0, st>>>(
+        mol_build_args(s0), reinterpret_cast<const BuildArgs *>(b.tab_molbuild.p));
     g_launches += 6;
 }
 
