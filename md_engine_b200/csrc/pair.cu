@@ -70,13 +70,13 @@ PairArgs make_args(State &s, FixPair &f) {
     A.coef2 = s.specialNeighborCoefs[1];
     A.coef3 = s.specialNeighborCoefs[2];
     A.qrc2 = 0.f;
-    A.alpha = 0.f;
+    pk::set_alpha(A, 0.f);
     A.qqr = (float)s.units.qqr_to_eng;
     A.dsf_A = A.dsf_shift = A.dsf_ecut = A.dsf_rc = 0.f;
     if (f.chargeFix) {
         float qrc = (float)f.chargeRCut;
         A.qrc2 = qrc * qrc;
-        A.alpha = (float)f.chargeFix->alpha;
+        pk::set_alpha(A, (float)f.chargeFix->alpha);
     } else if (f.dsfFix) {
         // FixChargePairDSF's evaluator (generateEvaluator, FixChargePairDSF.cu)
         const FixChargePairDSF &d = *f.dsfFix;
@@ -698,7 +698,7 @@ int pair_force_raw(int n, const float4 *xs, float4 *fs, const float *qs, const u
     A.coef3 = coef[2];
     A.dsf_A = A.dsf_shift = A.dsf_ecut = A.dsf_rc = 0.f;
     A.qrc2 = qrc > 0.f ? qrc * qrc : 0.f;
-    A.alpha = alpha;
+    pk::set_alpha(A, alpha);
     A.qqr = qqr;
     A.virials = virials;
     A.energy = nullptr;
@@ -740,7 +740,7 @@ int pair_force_gridgpu(int n, const float4 *xs, float4 *fs, const uint16_t *coun
     A.coef3 = coef[2];
     A.dsf_A = A.dsf_shift = A.dsf_ecut = A.dsf_rc = 0.f;
     A.qrc2 = qcut > 0.f ? qcut * qcut : 0.f;
-    A.alpha = alpha;
+    pk::set_alpha(A, alpha);
     A.qqr = qqr;
     A.virials = virials;
     A.energy = nullptr;

@@ -47,6 +47,7 @@ struct PairArgs {
     Box box;
     float coef1, coef2, coef3;
     float qrc2, alpha, qqr;
+    float ex2a, twoa;  // Ewald: -alpha^2 log2(e), 2 alpha / sqrt(pi) (set_alpha)
     // damped shifted force charges (CK 2): 2 alpha / sqrt(pi), the force
     // shift, erfc(alpha rc) / rc and rc of the charge cutoff
     float dsf_A, dsf_shift, dsf_ecut, dsf_rc;
@@ -78,6 +79,25 @@ __device__ __forceinline__ float erfc_tp(float x) {
 }
 __device__ __forceinline__ float erfc_as(float x, float expmx2) { return erfc_tp(x) * expmx2; }
 
+inline void set_alpha(PairArgs &A, float alpha) {
+    A.alpha = alpha;
+    A.ex2a = (float)(-1.4426950408889634 * (double)alpha * alpha);
+    A.twoa = (float)(1.1283791670955126 * (double)alpha);
+}
+
+// 1/x for a normal x: the hardware's approximation and one Newton step (its
+// error within an ulp), without the range handling of a division
+__device__ __forceinline__ float rcp_newton(float x) {
+    const float r = rcp_ftz(x);
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
+
+// the force kernels of LJ/cut, WCA and force-shifted LJ read one 16-byte word
+// per type pair, {rc^2, 48 eps sig^12, 24 eps sig^6, F(rc)}, formed from the
+// reference's table once per block
+template <int LJ, bool ENERGY>
+constexpr bool kPackedLJ = !ENERGY && (LJ == 1 || LJ == 2 || LJ == 3);
+
 // one neighbour: returns the scalar force factor (F = dr * s) and energy
 template <int LJ, int CK, bool ENERGY>
 __device__ __forceinline__ bool pair_term(const PairArgs &A, const float *sp, int nt2, int ti, float qi, float4 xj,
@@ -88,8 +108,20 @@ __device__ __forceinline__ bool pair_term(const PairArgs &A, const float *sp, in
     if (LJ) {
         const int tj = type_of(xj);
         const int ix = ti * A.ntypes + tj;
-        const float rc2 = sp[ix];
-        if (r2 < rc2) {
+        if constexpr (kPackedLJ<LJ, ENERGY>) {
+            const float4 w = reinterpret_cast<const float4 *>(sp)[ix];
+            if (r2 < w.x) {
+                any = true;
+                // eps = 0 (e.g. TIP4P/2005 H and M sites) contributes exactly zero
+                if (mult != 0.f && w.z != 0.f) {
+                    const float r2inv = rcp_newton(r2);
+                    const float r6inv = r2inv * r2inv * r2inv;
+                    float fs = r6inv * r2inv * (w.y * r6inv - w.z);
+                    if (LJ == 3) fs -= w.w * rsqrtf(r2);  // minus F(rc) / r
+                    s += fs * mult;
+                }
+            }
+        } else if (const float rc2 = sp[ix]; r2 < rc2) {
             any = true;
             if (LJ == 5) {
                 // TICG: F = -C 3/2 (r^2/rc^2 - 1) / (rc r), E = C/2 (x-1)^2 (x+2)/2, x = r/rc
@@ -143,18 +175,18 @@ __device__ __forceinline__ bool pair_term(const PairArgs &A, const float *sp, in
         // q_i q_j = 0 (e.g. the TIP4P/2005 oxygen) contributes exactly zero
         if (r2 < A.qrc2 && qi * qj != 0.f) {
             any = true;
+            // F/r = qq e^{-a^2 r^2} (t P(t) / r + 2 a / sqrt(pi)) / r^2 with
+            // erfc(a r) = t P(t) e^{-a^2 r^2} (the reference: __expf)
             const float r2c = r2 < 1e-10f ? 1e-10f : r2;
             const float rinv = rsqrt_ftz(r2c);
             const float r2inv = rinv * rinv;
-            const float x = A.alpha * (r2c * rinv);  // alpha r
-            const float expm = exp_neg_sq(x);        // exp(-alpha^2 r^2) (the reference: __expf)
+            const float expm = ex2_ftz(r2c * A.ex2a);
+            const float tp = erfc_tp(A.alpha * (r2c * rinv));
             const float qq = A.qqr * qi * qj;
-            const float erfcv = erfc_as(x, expm);
-            float fsc = qq * (erfcv * rinv + (2.0f * 0.5641895835477563f * A.alpha) * expm);
-            if (mult < 1.0f) fsc -= (1.0f - mult) * qq * rinv;
-            s += fsc * r2inv;
+            s += qq * (expm * r2inv) * fmaf(tp, rinv, A.twoa);
+            if (mult < 1.0f) s -= (1.0f - mult) * qq * rinv * r2inv;
             if (ENERGY) {
-                float eng = qq * rinv * erfcv;
+                float eng = qq * rinv * (tp * expm);
                 if (mult < 1.0f) eng -= (1.0f - mult) * qq * rinv;
                 e += 0.5f * eng;
             }
@@ -247,9 +279,17 @@ template <int T, int LJ, int CK, bool VIR, bool ENERGY>
 __global__ void __launch_bounds__(kPairBlock, T >= 32 ? 24 : 1) k_pair(const PairArgs a0, const PairArgs *__restrict__ tab, int accumulate) {
     pdl_wait();
     const PairArgs A = tab ? tab[blockIdx.y] : a0;
-    extern __shared__ float sp[];
+    extern __shared__ float4 sp4[];
+    float *const sp = reinterpret_cast<float *>(sp4);
     const int nt2 = A.ntypes * A.ntypes;
-    if (LJ) {
+    if constexpr (kPackedLJ<LJ, ENERGY>) {
+        for (int k = threadIdx.x; k < nt2; k += blockDim.x) {
+            const float eps24 = A.params[nt2 + k], sig6 = A.params[2 * nt2 + k];
+            sp4[k] = make_float4(A.params[k], eps24 * 2.f * sig6 * sig6, eps24 * sig6,
+                                 LJ == 3 ? A.params[3 * nt2 + k] : 0.f);
+        }
+        __syncthreads();
+    } else if (LJ) {
         for (int k = threadIdx.x; k < A.np * nt2; k += blockDim.x) sp[k] = A.params[k];
         __syncthreads();
     }
@@ -340,15 +380,23 @@ void launch_t(const PairArgs &A, const PairArgs *tab, int nrep, bool vir, bool e
     const int G = 32 / T;
     const int warps = (A.n + G - 1) / G;
     const dim3 blocks((warps * 32 + kPairBlock - 1) / kPairBlock, nrep);
-    const size_t smem = LJ ? (size_t)A.np * A.ntypes * A.ntypes * sizeof(float) : 0;
+    const size_t nt2 = (size_t)A.ntypes * A.ntypes;
+    const size_t smem = LJ ? (size_t)A.np * nt2 * sizeof(float) : 0;
     if (energy) {
         k_pair<T, LJ, CK, false, true><<<blocks, kPairBlock, smem, st>>>(A, tab, 0);
         MDX_LAUNCHED();
-    } else if (vir) {
-        k_pair<T, LJ, CK, true, false><<<blocks, kPairBlock, smem, st>>>(A, tab, accumulate ? 1 : 0);
+        return;
+    }
+    const size_t smem_f = kPackedLJ<LJ, false> ? nt2 * sizeof(float4) : smem;
+    auto kern = vir ? k_pair<T, LJ, CK, true, false> : k_pair<T, LJ, CK, false, false>;
+    // beyond the default limit (55 types; the unpacked table reached it at 64)
+    if (smem_f > 48 * 1024)
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f);
+    if (vir) {
+        kern<<<blocks, kPairBlock, smem_f, st>>>(A, tab, accumulate ? 1 : 0);
         MDX_LAUNCHED();
     } else {
-        launch_pdl(k_pair<T, LJ, CK, false, false>, blocks, dim3(kPairBlock), smem, st, A, tab, accumulate ? 1 : 0);
+        launch_pdl(kern, blocks, dim3(kPairBlock), smem_f, st, A, tab, accumulate ? 1 : 0);
     }
 }
 

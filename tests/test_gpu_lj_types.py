@@ -1,0 +1,56 @@
+"""Pair forces with the packed type-pair table at one species, several, and
+more than the default shared memory holds, with and without zero pairs,
+against a brute-force FP64 sum."""
+import numpy as np
+import pytest
+
+from md_engine_b200 import Bounds, FixLJCut, FixLJCutFS, State, Vector
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("style", [FixLJCut, FixLJCutFS])
+@pytest.mark.parametrize("ntypes,zero", [(1, False), (3, True), (60, False)])
+def test_forces_by_species(style, ntypes, zero):
+    rng = np.random.default_rng(ntypes)
+    n, L, rc = 1000, 11.0, 2.5
+    g = np.stack(np.meshgrid(*[np.arange(10)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = ((g + 0.5) * 1.1 + rng.uniform(-0.1, 0.1, (n, 3))).astype(np.float32).astype(np.float64)
+    types = rng.integers(0, ntypes, n)
+    st = State()
+    st.units.setLJ()
+    st.bounds = Bounds(st, lo=Vector(0, 0, 0), hi=Vector(L, L, L))
+    st.rCut, st.padding, st.dt = rc, 0.3, 0.001
+    names = [f"T{k}" for k in range(ntypes)]
+    for h in names:
+        st.atomParams.addSpecies(h, 1.0, 1)
+    st.addAtoms([names[t] for t in types], pos, np.zeros(n))
+    sig = np.float32(1.0 - 0.1 * rng.random(ntypes)).astype(np.float64)
+    eps = np.float32(0.5 + rng.random(ntypes)).astype(np.float64)
+    if zero:
+        eps[1] = 0.0
+    fix = style(st, "pair")
+    for k, h in enumerate(names):
+        fix.setParameter("sig", h, h, sig[k])
+        fix.setParameter("eps", h, h, eps[k])
+    st.activateFix(fix)
+    st.prepare()
+    st.computeForces()
+    f = st.getAtoms()[2]
+    d = pos[:, None] - pos[None]
+    d -= L * np.round(d / L)
+    r2 = (d ** 2).sum(2)
+    np.fill_diagonal(r2, 1e9)
+    s = np.sqrt(sig[:, None] * sig[None])[types][:, types]  # geometric mixing
+    e = np.sqrt(eps[:, None] * eps[None])[types][:, types]
+
+    def over_r(q2):
+        s6 = s ** 6 / q2 ** 3
+        return 24.0 * e * s6 * (2.0 * s6 - 1.0) / q2
+
+    k = over_r(r2)
+    if style is FixLJCutFS:
+        k = k - over_r(rc * rc) * rc / np.sqrt(r2)
+    ref = np.einsum("ij,ijc->ic", np.where(r2 < rc * rc, k, 0.0), d)
+    rms = np.sqrt(np.mean(np.sum(ref ** 2, 1)))
+    assert np.max(np.linalg.norm(f - ref, axis=1)) < 2e-4 * rms
