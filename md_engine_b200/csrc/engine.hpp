@@ -378,9 +378,9 @@ struct E3BSurrogate {
     DBuf<float4> frame;
     DBuf<float4> fexact;
     // training scratch
-    DBuf<__nv_bfloat16> xb, act[3], dz;
+    DBuf<__nv_bfloat16> xb;
     DBuf<float> xf;  // host rows before their rounding to BF16
-    DBuf<float> z[4], yb, da;
+    DBuf<float> yb;
     DBuf<double> loss;
     int batch = 0;
 };
