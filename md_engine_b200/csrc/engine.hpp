@@ -521,6 +521,8 @@ class State {
     // beside it
     int pairBlocksPerSM = 0;
     MolForm mf;
+    // consecutive steps of a chunk joined by one kernel (step_turn_prepare)
+    bool turn_ok = false;
     // list build tunables, 0 = automatic: cells of >= cut/gridStencil (1..4),
     // home atoms tested at once per warp (2 or 4)
     int gridStencil = 0, gridHomeGroup = 0;
@@ -720,6 +722,8 @@ int rigid_update_maps(State &s, FixRigid &r, bool conditional);
 int step_first_half(State &s, bool fused, bool early = false);
 int step_second_half(State &s, bool fused, const float4 *fextra = nullptr, const float4 *frecip = nullptr);
 bool has_free_atoms(State &s);
+int step_turn_prepare(State &s);
+int step_turn(State &s);
 int rigid_prepare(State &s, FixRigid &r);
 int rigid_hook(State &s, FixRigid &r, int which);
 int rigid_validate(State &s, FixRigid &r, uint32_t *n_bad);

@@ -10,6 +10,8 @@
 // needed per step (the reference syncs for the kinetic energy every step,
 // FixNoseHoover.cu:1044-1056).  Atoms outside rigid molecules use per-atom
 // kernels with the same arithmetic.
+#include <cooperative_groups.h>
+
 #include <cstdio>
 
 #include "engine.hpp"
@@ -40,6 +42,21 @@ __host__ __device__ inline double nh_exp_small(double x) {
 // the first and pf[0], which need no kinetic energy; nh_up: the rest.  SMALL:
 // the polynomial exponential; `most` collects the largest |argument|, and
 // the caller starts over with SMALL = false when it lies outside the range.
+__host__ __device__ __forceinline__ double chain_mass(const NHChain &c, int k) { return c.mass[k]; }
+__host__ __device__ __forceinline__ double chain_inv_mass(const NHChain &c, int k) { return c.inv_mass[k]; }
+
+// the time-dependent part of a chain, held in registers; the links above the
+// first have one mass (nh_prepare)
+struct NHRegs {
+    double vel[kNHChain], force[kNHChain];
+    double mass0, inv_mass0, mass1, inv_mass1;
+    double ke, ndf, kB, T, dt;
+};
+__host__ __device__ __forceinline__ double chain_mass(const NHRegs &c, int k) { return k == 0 ? c.mass0 : c.mass1; }
+__host__ __device__ __forceinline__ double chain_inv_mass(const NHRegs &c, int k) {
+    return k == 0 ? c.inv_mass0 : c.inv_mass1;
+}
+
 template <int N, bool SMALL>
 __host__ __device__ __forceinline__ double nh_ex(double x, double &most) {
     if (!SMALL) return exp(x);
@@ -64,18 +81,18 @@ template <int N, bool SMALL, class C>
 __host__ __device__ __forceinline__ double nh_up(C &c, const double (&pf)[N - 1], bool stepInit, double &most) {
     const double nkt = c.ndf * c.kB * c.T, kt = c.kB * c.T;
     const double t2 = 0.5 * c.dt, t4 = 0.25 * c.dt;
-    if (!stepInit) c.force[0] = (c.ke - nkt) * c.inv_mass[0];
+    if (!stepInit) c.force[0] = (c.ke - nkt) * chain_inv_mass(c, 0);
     c.vel[0] = fma(c.vel[0], pf[0], t4 * c.force[0]) * pf[0];
     const double sf = nh_ex<N, SMALL>(-t2 * c.vel[0], most);
     c.ke *= sf * sf;
-    c.force[0] = (c.ke - nkt) * c.inv_mass[0];
+    c.force[0] = (c.ke - nkt) * chain_inv_mass(c, 0);
     c.vel[0] = fma(c.vel[0], pf[0], t4 * c.force[0]) * pf[0];
 #pragma unroll
     for (int k = 1; k < N - 1; ++k) {
-        c.force[k] = fma(c.mass[k - 1] * c.vel[k - 1], c.vel[k - 1], -kt) * c.inv_mass[k];
+        c.force[k] = fma(chain_mass(c, k - 1) * c.vel[k - 1], c.vel[k - 1], -kt) * chain_inv_mass(c, k);
         c.vel[k] = fma(c.vel[k], pf[k], t4 * c.force[k]) * pf[k];
     }
-    c.force[N - 1] = fma(c.mass[N - 2] * c.vel[N - 2], c.vel[N - 2], -kt) * c.inv_mass[N - 1];
+    c.force[N - 1] = fma(chain_mass(c, N - 2) * c.vel[N - 2], c.vel[N - 2], -kt) * chain_inv_mass(c, N - 1);
     c.vel[N - 1] += t4 * c.force[N - 1];
     return sf;
 }
@@ -401,20 +418,16 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return r;  // valid in thread 0
 }
 
-// the time-dependent part of a chain, held in registers
-struct NHRegs {
-    double vel[kNHChain], force[kNHChain], mass[kNHChain], inv_mass[kNHChain];
-    double ke, ndf, kB, T, dt;
-};
-
 __device__ __forceinline__ void load_chain(NHRegs &c, const NHChain &g) {
 #pragma unroll
     for (int k = 0; k < kNHChain; k++) {
         c.vel[k] = __ldcg(&g.vel[k]);
         c.force[k] = __ldcg(&g.force[k]);
-        c.mass[k] = __ldcg(&g.mass[k]);
-        c.inv_mass[k] = __ldcg(&g.inv_mass[k]);
     }
+    c.mass0 = __ldcg(&g.mass[0]);
+    c.mass1 = __ldcg(&g.mass[1]);
+    c.inv_mass0 = __ldcg(&g.inv_mass[0]);
+    c.inv_mass1 = __ldcg(&g.inv_mass[1]);
     c.ndf = __ldcg(&g.ndf);
     c.kB = __ldcg(&g.kB);
     c.T = __ldcg(&g.T);
@@ -478,17 +491,16 @@ __global__ void __launch_bounds__(kEndThreads) k_step_end(const EndArgs a0, cons
     const double ke = tot * mvv;
     c.ke = ke;
     double sf1 = nh_up<kNHChain, true>(c, pf, false, most);  // stepFinal
-    NHRegs fin = c;
+    store_chain(A.chain[1], c, ke, sf1);
     double sf2 = nh_half<kNHChain, true>(c, true, most);  // stepInit of the next step
     if (!(most < kNHSmall)) {  // outside the polynomial's range: again, with exp()
         load_chain(c, A.chain[0]);
         c.ke = ke;
         sf1 = nh_half<kNHChain, false>(c, false, most);
-        fin = c;
+        store_chain(A.chain[1], c, ke, sf1);
         sf2 = nh_half<kNHChain, false>(c, true, most);
     }
     store_chain(A.chain[0], c, ke, sf1 * sf2);
-    store_chain(A.chain[1], fin, ke, sf1);
 }
 
 // per-atom: postForce_cu (IntegratorVerlet.cu:610-627) + m v^2 partials
@@ -596,6 +608,168 @@ __global__ void k_second_mol(const MolArgs a0, const MolArgs *__restrict__ tab) 
     }
     const double b = block_sum(mv2, sh);
     if (threadIdx.x == 0) A.partials[A.part_off + blockIdx.x] = b;
+}
+
+// ---- from one step to the next --------------------------------------------
+// Small systems of free atoms: the second half of a step, its Nose-Hoover
+// update and the first half of the next step in one kernel, by one
+// thread-block cluster.  Velocities and forces stay in registers between the
+// halves, the kinetic sum crosses the cluster through distributed shared
+// memory, and every block works the chain out itself (a warp of its own:
+// loaded, and swept as far as needs no kinetic energy, before the forces are
+// there), so that no second barrier hands the scale round.  What bounds it is
+// latency: one load, a cluster barrier (about 1 us) and the chain (0.7 us);
+// as three kernels the same work also pays two launches and the reloading.
+// Step of 4,000 LJ atoms: 14.7 -> 13.7 us, of 8,000 ions 32.7 -> 32.1.  One
+// atom per thread of at most 16 blocks, all of them on one GPC: with four
+// atoms per thread 32,000 atoms took 25.4 us a step, as three kernels over
+// the whole chip 24.4, and rigid molecules one per thread (SETTLE in FP64) lost
+// 3 to 4.5 us a step at 512 and 4,096 molecules.  Larger systems and rigid
+// ones keep the three kernels.
+constexpr int kTurnAtoms = 512;  // worker threads per block, one atom each
+constexpr int kTurnBlocks = 16;  // blocks per cluster at most (non-portable size)
+
+struct TurnShared {
+    double warp_sum[32];
+    double block_sum[kTurnBlocks];
+    double vel0[kNHChain], force0[kNHChain];  // the chain before its sweeps
+    float scale;
+};
+
+// The worker warps and the chain warp (the block's last) run their own code
+// between the same barriers (so that neither holds the other's registers):
+// turn_barrier, the cluster barrier, turn_barrier.
+__device__ __forceinline__ void turn_barrier() {
+    asm volatile("bar.sync 1, %0;" ::"n"(kTurnAtoms + 32) : "memory");
+}
+
+// at the kernel's start and before the first use of another block's memory:
+// every block of the cluster runs by then
+__device__ __forceinline__ void turn_started() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void turn_all_started() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
+
+// workers: their m v^2 in, the scale of the coming first half out
+template <bool NH>
+__device__ __forceinline__ float turn_worker(TurnShared &sh, double mv2) {
+    if (!NH) return 1.0f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mv2 += __shfl_xor_sync(0xffffffffu, mv2, o);
+    if ((threadIdx.x & 31) == 0) sh.warp_sum[threadIdx.x >> 5] = mv2;
+    turn_barrier();
+    turn_all_started();
+    cooperative_groups::this_cluster().sync();
+    turn_barrier();
+    return sh.scale;
+}
+
+// the chain warp: the chain loaded and swept as far as needs no kinetic
+// energy (it was written by a kernel that has completed: this one's
+// predecessor waited for it), the cluster's kinetic sum, stepFinal and the
+// coming stepInit; the cluster's first block stores chain and turn
+template <bool NH>
+__device__ __forceinline__ void turn_chain(TurnShared &sh, const EndArgs &E) {
+    namespace cg = cooperative_groups;
+    const auto cluster = cg::this_cluster();
+    const unsigned rank = cluster.block_rank(), nb = cluster.num_blocks();
+    const int lane = threadIdx.x & 31;
+    if (!NH) {
+        pdl_wait();
+        if (lane == 0 && rank == 0) E.st->turn += 1;
+        return;
+    }
+    NHRegs c;
+    double pf[kNHChain - 1], mvv = 0.0, most = 0.0;
+    if (lane == 0) {
+        load_chain(c, E.chain[0]);
+        mvv = __ldcg(&E.chain[0].mvv_to_eng);
+#pragma unroll
+        for (int k = 0; k < kNHChain; k++) {
+            sh.vel0[k] = c.vel[k];
+            sh.force0[k] = c.force[k];
+        }
+        nh_down<kNHChain, true>(c, pf, most);
+    }
+    __syncwarp();
+    pdl_wait();
+    turn_barrier();
+    double t = lane < kTurnAtoms / 32 ? sh.warp_sum[lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    turn_all_started();
+    if ((unsigned)lane < nb) *cluster.map_shared_rank(&sh.block_sum[rank], lane) = t;
+    __syncwarp();
+    cluster.sync();  // no block reads another's memory after this
+    if (lane == 0) {
+        double tot = 0.0;
+        for (unsigned b = 0; b < nb; b++) tot += sh.block_sum[b];
+        const double ke = tot * mvv;
+        c.ke = ke;
+        double sf1 = nh_up<kNHChain, true>(c, pf, false, most);  // stepFinal
+        if (rank == 0) store_chain(E.chain[1], c, ke, sf1);
+        double sf2 = nh_half<kNHChain, true>(c, true, most);  // stepInit of the next step
+        if (!(most < kNHSmall)) {  // outside the polynomial's range: again, with exp()
+#pragma unroll
+            for (int k = 0; k < kNHChain; k++) {
+                c.vel[k] = sh.vel0[k];
+                c.force[k] = sh.force0[k];
+            }
+            c.ke = ke;
+            sf1 = nh_half<kNHChain, false>(c, false, most);
+            if (rank == 0) store_chain(E.chain[1], c, ke, sf1);
+            sf2 = nh_half<kNHChain, false>(c, true, most);
+        }
+        sh.scale = (float)(sf1 * sf2);
+        if (rank == 0) {
+            store_chain(E.chain[0], c, ke, sf1 * sf2);
+            if (E.ke_out) *E.ke_out = tot;
+            E.st->turn += 1;
+        }
+    }
+    __syncwarp();
+    turn_barrier();
+}
+
+template <bool NH>
+__global__ void __launch_bounds__(kTurnAtoms + 32, 1) k_turn_atoms(int n, float4 *__restrict__ xs,
+                                                                   float4 *__restrict__ vs, float4 *__restrict__ fs,
+                                                                   float dt, float dtf, const EndArgs E) {
+    __shared__ TurnShared sh;
+    if (NH) turn_started();
+    if (threadIdx.x >= kTurnAtoms) {
+        turn_chain<NH>(sh, E);
+        return;
+    }
+    pdl_wait();
+    const int i = blockIdx.x * kTurnAtoms + threadIdx.x;
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), f = x, v = make_float4(0.f, 0.f, 0.f, kInvMassless);
+    if (i < n) {
+        x = xs[i];
+        v = vs[i];
+        f = fs[i];
+    }
+    const bool massless = v.w > kInvMassBool;
+    double mv2 = 0.0;
+    if (!massless) {
+        v = kick(v, f, dtf);
+        if (NH) mv2 = ((double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z) / (double)v.w;
+    }
+    const float s = turn_worker<NH>(sh, mv2);
+    if (i < n) {
+        if (massless) {
+            vs[i] = make_float4(0.f, 0.f, 0.f, v.w);
+        } else {
+            if (NH) {
+                v.x *= s;
+                v.y *= s;
+                v.z *= s;
+            }
+            v = kick(v, f, dtf);
+            vs[i] = v;
+            xs[i] = make_float4(x.x + dt * v.x, x.y + dt * v.y, x.z + dt * v.z, x.w);
+        }
+        fs[i] = make_float4(0.f, 0.f, 0.f, f.w);
+    }
+    pdl_trigger();
 }
 
 // ---- stand-alone hooks (one kernel per reference hook) ------------------
@@ -990,6 +1164,75 @@ int step_second_half(State &s, bool fused, const float4 *fextra, const float4 *f
     }
     MDX_CUDA_TRY(launch_pdl(k_step_end, dim3(1), dim3(kEndThreads), 0, s.stream, end_args(s, nparts),
                             (const EndArgs *)nullptr));
+    return 0;
+}
+
+namespace {
+template <typename... KArgs, typename... Args>
+cudaError_t launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, unsigned cluster, cudaStream_t st,
+                           Args... args) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    MDX_LAUNCHED();
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// whether the device takes clusters of this many blocks of the kernel
+template <typename K>
+bool cluster_fits(K kern, int threads, unsigned cluster) {
+    if (cluster > 8 &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(threads);
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return n > 0;
+}
+
+}  // namespace
+
+// at prepare: whether the steps of a chunk are joined by the turn kernel --
+// all atoms free, few enough for one cluster, and the device takes such a
+// cluster
+int step_turn_prepare(State &s) {
+    s.turn_ok = false;
+    const unsigned c = (unsigned)((s.gpd.n + kTurnAtoms - 1) / kTurnAtoms);
+    // (the pair kernel between two turns: the second may read the first's chain
+    // before its own wait)
+    if (!s.pairFix() || s.gpd.n < 1 || s.rigidFix() || c > (unsigned)kTurnBlocks) return 0;
+    s.turn_ok = cluster_fits(s.nhFix() ? k_turn_atoms<true> : k_turn_atoms<false>, kTurnAtoms + 32, c);
+    return 0;
+}
+
+// the second half of a step and the first half of the next (turn_ok)
+int step_turn(State &s) {
+    const unsigned c = (unsigned)((s.gpd.n + kTurnAtoms - 1) / kTurnAtoms);
+    MDX_CUDA_TRY(launch_cluster(s.nhFix() ? k_turn_atoms<true> : k_turn_atoms<false>, dim3(c), dim3(kTurnAtoms + 32), c,
+                                s.stream, s.gpd.n, s.gpd.xs.p, s.gpd.vs.p, s.gpd.fs.p, (float)s.dt,
+                                (float)(0.5 * s.dt * s.units.ftm_to_v), end_args(s, 0)));
     return 0;
 }
 

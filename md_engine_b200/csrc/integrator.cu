@@ -47,12 +47,16 @@ class IntegratorVerlet {
     // fused step: the P3M chain (spread, R2C, E(k), C2R) and E3B run on two
     // side streams beside the pair kernel; they join before the P3M gather
     // and the second half (which merges the E3B forces)
-    int stepFused(bool early) {
+    // first, last: the step's place in its chunk.  Where the state's steps are
+    // joined (turn_ok), a step's second half and the next one's first half are
+    // one kernel
+    int stepFused(bool first, bool last) {
         FixPair *pf = s->pairFix();
         FixChargeEwald *ew = s->ewaldFix();
         FixE3B *e3 = s->e3bFix();
         const bool e3side = e3 && e3->side_ok && s->rigidFix();
-        if (int e = step_first_half(*s, true, early)) return e;
+        if (first || !s->turn_ok)
+            if (int e = step_first_half(*s, true, !first)) return e;
         if (ew || e3side) MDX_CUDA_TRY(cudaEventRecord(s->ev_fork, s->stream));
         // all-rigid systems: the gather also runs on the side stream, into a
         // per-step buffer the second half adds (so it overlaps the pair kernel)
@@ -94,6 +98,7 @@ class IntegratorVerlet {
                 if (int e = ew->gather(true, s->stream)) return e;
         }
         if (e3side) MDX_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->ev_join[1], 0));
+        if (!last && s->turn_ok) return step_turn(*s);
         return step_second_half(*s, true, e3side ? e3->f_side.p : nullptr, recip_side ? ew->f_recip.p : nullptr);
     }
     // the force phase of the fused step alone (fork, the pair kernel beside
@@ -197,8 +202,8 @@ class IntegratorVerlet {
         return s->checkStatus();
     }
 
-    int stepBody(bool early) {
-        if (mode == 0) return stepFused(early);
+    int stepBody(bool first, bool last) {
+        if (mode == 0) return stepFused(first, last);
         if (int e = step_first_half(*s, false)) return e;
         if (int e = forces()) return e;
         if (int e = step_second_half(*s, false)) return e;
@@ -216,7 +221,7 @@ class IntegratorVerlet {
             build_pending = overlap;
         }
         for (int k = 0; k < nsteps; k++)
-            if (int e = stepBody(k > 0)) return e;
+            if (int e = stepBody(k == 0, k + 1 == nsteps)) return e;
         if (build_pending) MDX_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->ev_join[2], 0));
         build_pending = false;
         return 0;

@@ -412,6 +412,7 @@ int State::prepare() {
     if (FixNoseHoover *nh = nhFix()) {
         if (int e = nh_prepare(*this, *nh)) return e;
     }
+    if (int e = step_turn_prepare(*this)) return e;
     MDX_CUDA_TRY(cudaStreamSynchronize(stream));
     MDX_CUDA_TRY(cudaGetLastError());
     if (int e = checkStatus()) return e;
