@@ -328,6 +328,7 @@ struct BuildArgs {
     CellGrid g;
     Box box;
     int ncell, m, use_excl, part_q, cap;
+    int parts;  // warps per cell
     float cutsq;
 };
 
@@ -378,14 +379,16 @@ __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(con
                                   (float)(t / 9 - 1) * A.box.L.z, 0.f);
     }
     __syncthreads();  // the only block-wide barrier: warps own cells from here on
-    const int c = blockIdx.x * kBuildCellsPerBlock + wib;
+    // parts warps share a cell's home groups of HG in turn
+    const int parts = A.parts, gw = blockIdx.x * kBuildCellsPerBlock + wib;
+    const int c = gw / parts, part = gw - c * parts;
     if (c >= A.ncell) return;
     uint32_t *const sh_seg_offc = sh_seg_offc_all[wib];
     int *const sh_seg_beg = sh_seg_beg_all[wib];
     uint32_t *const sh_cand = sh_cand_all[wib];
     const CellGrid &g = A.g;
     const int cs = (int)A.cell_start[c], ce = (int)A.cell_start[c + 1];
-    if (ce <= cs) return;
+    if (ce <= cs + HG * part) return;
     const int cz = c % g.ns.z, cy = (c / g.ns.z) % g.ns.y, cx = c / (g.ns.z * g.ns.y);
     const int m = A.m, side = 2 * m + 1;
     const float cutsq = A.cutsq;
@@ -393,9 +396,10 @@ __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(con
     uint32_t *const nlist = A.nlist;
     const float dsx = 1.0f / g.inv_ds.x, dsy = 1.0f / g.inv_ds.y, dsz = 1.0f / g.inv_ds.z;
     const uint32_t lt = (1u << lane) - 1u;
-    // bounding box of the home atoms' positions
+    // bounding box of this warp's home atoms
     float bxl = 3.0e38f, bxh = -3.0e38f, byl = 3.0e38f, byh = -3.0e38f, bzl = 3.0e38f, bzh = -3.0e38f;
     for (int i = cs + lane; i < ce; i += 32) {
+        if (parts > 1 && (i - cs) / HG % parts != part) continue;
         const float4 p4 = A.xs2[STRIDE * i];
         bxl = fminf(bxl, p4.x);
         bxh = fmaxf(bxh, p4.x);
@@ -534,7 +538,7 @@ __global__ void __launch_bounds__(kBuildCellsPerBlock * 32, 7) k_build_cells(con
         __syncwarp();
     }
     // home atoms HG at a time, in registers (warp-uniform values)
-    for (int g0 = cs; g0 < ce; g0 += HG) {
+    for (int g0 = cs + HG * part; g0 < ce; g0 += HG * parts) {
         float hx[HG], hy[HG], hz[HG], hq[HG];
         uint32_t hmask[HG], hid[HG], ci[HG], cn[HG];
         ulonglong2 hwin[HG];
@@ -880,6 +884,18 @@ GridArgs mol_scan_args(State &s) {
     return A;
 }
 
+// warps per cell of the list build: as many as the SMs hold at once (28 each),
+// to the nearest, four at most.  A small system's build takes as long as its
+// fullest cell's warp: 2,048 water sites (729 cells) 74 us with one warp per
+// cell, 47 with four; 4,096 molecules (1,728 cells) 46 and, with two, 37;
+// 8,000 ions (2,744 cells) 46.5 and 44.3.  Beyond what is resident the cell's
+// candidates are only expanded once more: 32,000 particles (13,824 cells) 63
+// and 71.
+inline int build_parts(int ncell) {
+    const int resident = 28 * num_sms();
+    return std::min(4, std::max(1, (resident + ncell / 2) / std::max(ncell, 1)));
+}
+
 BuildArgs build_args(State &s, const CellGrid &g, float cutsq) {
     GridGPU &gr = s.grid;
     GPUData &d = s.gpd;
@@ -908,6 +924,7 @@ BuildArgs build_args(State &s, const CellGrid &g, float cutsq) {
     A.g = g;
     A.box = s.box;
     A.ncell = g.ns.x * g.ns.y * g.ns.z;
+    A.parts = build_parts(A.ncell);
     A.m = gr.m;
     A.use_excl = gr.have_excl ? 1 : 0;
     A.part_q = gr.part_q ? 1 : 0;
@@ -951,13 +968,13 @@ void launch_build_any(int team, int hg, dim3 grid, cudaStream_t st, const BuildA
     }
 }
 
-inline dim3 build_grid(int ncell, int nrep) {
-    return dim3((ncell + kBuildCellsPerBlock - 1) / kBuildCellsPerBlock, nrep);
+inline dim3 build_grid(int ncell, int parts, int nrep) {
+    return dim3((ncell * parts + kBuildCellsPerBlock - 1) / kBuildCellsPerBlock, nrep);
 }
 
 void launch_build(State &s, const CellGrid &g, float cutsq, cudaStream_t st) {
     const BuildArgs A = build_args(s, g, cutsq);
-    launch_build_any<false>(s.grid.team, s.grid.home_group, build_grid(A.ncell, 1), st, A, nullptr);
+    launch_build_any<false>(s.grid.team, s.grid.home_group, build_grid(A.ncell, A.parts, 1), st, A, nullptr);
 }
 
 // the molecule-pair list: rows of 32 lanes, its molecules' site 0 within the
@@ -977,6 +994,7 @@ BuildArgs mol_build_args(State &s) {
     A.g = mol_grid(s);
     A.box = s.box;
     A.ncell = mf.ns.x * mf.ns.y * mf.ns.z;
+    A.parts = build_parts(A.ncell);
     A.m = mf.m;
     A.cap = mf.cap;
     A.cutsq = mf.cut * mf.cut;
@@ -989,7 +1007,7 @@ void launch_count(State &s, const CellGrid &g, float cutsq) {
     A.ljmask = nullptr;
     A.part_q = 0;
     A.cap = 0;
-    launch_build_any<true>(s.grid.team, s.grid.home_group, build_grid(A.ncell, 1), s.stream, A, nullptr);
+    launch_build_any<true>(s.grid.team, s.grid.home_group, build_grid(A.ncell, A.parts, 1), s.stream, A, nullptr);
 }
 
 }  // namespace
@@ -1259,7 +1277,7 @@ static int nlist_rebuild_mf(State &s, bool force, cudaStream_t bstream) {
         MDX_CUDA_TRY(cudaStreamWaitEvent(bstream, s.ev_sorted, 0));
         bs = bstream;
     }
-    MDX_CUDA_TRY(launch_pdl(k_build_cells<32, kMolHomes, false, false, false, 4>, build_grid(M.ncell, 1),
+    MDX_CUDA_TRY(launch_pdl(k_build_cells<32, kMolHomes, false, false, false, 4>, build_grid(M.ncell, mol_build_args(s).parts, 1),
                             dim3(kBuildCellsPerBlock * 32), 0, bs, mol_build_args(s), (const BuildArgs *)nullptr));
     if (FixE3B *e3 = s.e3bFix()) {
         if (int e = e3b_build_list_mf(s, *e3, bs)) return e;
@@ -1510,6 +1528,7 @@ int batch_nlist_tables(Batch &b) {
             State &s = *b.reps[b.ps[q]];
             hp[q] = hg[b.ps[q]];
             hb[q] = build_args(s, make_grid(s), s.grid.cut * s.grid.cut);
+            hb[q].parts = build_parts(b.max_cell_ps * P);
             // one list-build kernel serves the batch: its exclusion and
             // front/back split forms are compile-time, so they must agree
             if ((hb[q].use_excl != 0) != (hb[0].use_excl != 0) ||
@@ -1538,6 +1557,7 @@ int batch_nlist_tables(Batch &b) {
             hb[q] = mol_build_args(s);
             b.max_mcell = std::max(b.max_mcell, hs[q].ncell);
         }
+        for (BuildArgs &a : hb) a.parts = build_parts(b.max_mcell * Q);
         if (int e = b.tab_molgrid.alloc(Q * sizeof(MolGridArgs))) return e;
         if (int e = b.tab_molscan.alloc(Q * sizeof(GridArgs))) return e;
         if (int e = b.tab_molbuild.alloc(Q * sizeof(BuildArgs))) return e;
@@ -1567,7 +1587,7 @@ static void batch_rebuild_sites(Batch &b, cudaStream_t st) {
     k_copyback<<<nb, 256, 0, st>>>(A, tg);
     int hg = 2;
     for (int r : b.ps) hg = std::max(hg, b.reps[r]->grid.home_group);
-    launch_build_any<false>(s0.grid.team, hg, build_grid(b.max_cell_ps, P), st, B, tb);
+    launch_build_any<false>(s0.grid.team, hg, build_grid(b.max_cell_ps, build_parts(b.max_cell_ps * P), P), st, B, tb);
     g_launches += 5;
 }
 
@@ -1589,7 +1609,7 @@ static void batch_rebuild_mols(Batch &b, cudaStream_t st) {
     k_mf_scatter<<<dim3(nb_mol, Q), 256, 0, st>>>(M, tm);
     k_mf_gather<<<dim3(nb_site, Q), 256, 0, st>>>(M, tm);
     k_mf_copyback<<<dim3(nb_site, Q), 256, 0, st>>>(M, tm);
-    k_build_cells<32, kMolHomes, false, false, false, 4><<<build_grid(b.max_mcell, Q), kBuildCellsPerBlock * 32, 0, st>>>(
+    k_build_cells<32, kMolHomes, false, false, false, 4><<<build_grid(b.max_mcell, build_parts(b.max_mcell * Q), Q), kBuildCellsPerBlock * 32, 0, st>>>(
         mol_build_args(s0), reinterpret_cast<const BuildArgs *>(b.tab_molbuild.p));
     g_launches += 6;
 }

@@ -54,3 +54,20 @@ def test_forces_at_each_team_size(oracle, n):
     ref = oracle.pair_forces(x, np.zeros(n, int), np.zeros(n), prm, np.full(3, L), c, nb)["f"]
     rms = np.sqrt(np.mean(np.sum(ref ** 2, 1)))
     assert np.max(np.linalg.norm(f - ref, axis=1)) < 2e-4 * rms
+
+
+# four, three, two warps and one warp per cell on 148 SMs, about five atoms in a cell
+@pytest.mark.parametrize("side", [9, 11, 13, 15])
+def test_list_with_several_warps_per_cell(oracle, side):
+    n, rcut, skin = 5 * side ** 3, 1.5, 0.2
+    L = side * (1.7 / 2) * 1.0001
+    st = _state(n, L, rcut, skin, side)
+    st.gridStencil = 2
+    st.prepare()
+    assert int(st.cellsPerSide) == side
+    x = st.getAtoms()[0].astype(np.float32)
+    c, nb, _ = st.getNeighborList()
+    co, no = oracle_nlist_for(oracle, x, np.zeros(3), np.full(3, L), neighbor_cut(rcut, skin), ids=np.arange(n))[:2]
+    assert np.array_equal(c, co)
+    for i in range(0, n, 97):
+        assert np.array_equal(np.sort(nb[i, :c[i]]), np.sort(no[i, :co[i]]))
