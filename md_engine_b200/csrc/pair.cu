@@ -121,7 +121,7 @@ PairArgs make_args(State &s, FixPair &f) {
 //    cutoff is within L/2 under it, so it is the pair's minimum image) and
 //    the cutoffs applied as masks, not branches: all lanes run one path.
 // The molecule's own site pairs (the excluded pairs of the reference's list,
-// multiplier by exclusion depth) are added by lane 0.  Forces on the four
+// multiplier by exclusion depth) are added by lanes 0..15, a pair each.  Forces on the four
 // sites are reduced by shuffles and written by lanes 0..3 (one 64-byte store).
 // blocks per SM the kernel is compiled for: 80 registers, which lets the nine
 // charge pairs of a molecule pair be in flight beside one another.  Alone at
@@ -239,6 +239,10 @@ __device__ __forceinline__ float mol_pair_term(const MolPairArgs &A, int ab, flo
         }
     }
     return s;
+}
+
+__device__ __forceinline__ float3 site_of(const float3 (&x)[4], int k) {
+    return k < 2 ? (k == 0 ? x[0] : x[1]) : (k == 2 ? x[2] : x[3]);
 }
 
 // asynchronous 16-byte global -> shared copies (cp.async, cached in L1): a
@@ -397,22 +401,22 @@ __global__ void __launch_bounds__(kMolPairBlock, kMolPairBlocksPerSM) k_pair_mol
             mol_pair_eval<LJ, EW, VIR, ENERGY, TOPO>(A, xi, qj[lane], make_float3(s4.x, s4.y, s4.z), f, en, v);
         }
         __syncwarp();  // the queue and the batch are reused by the warp's next slot
-        // the molecule's own site pairs, once per molecule
-        if (lane == 0 && A.selfm) {
+        // the molecule's own site pairs, one per lane: pair ab in lane ab
+        if (A.selfm) {
+            const int a = lane >> 2 & 3, b = lane & 3, ab = lane & 15;
+            if (lane < 16 && ((A.selfm >> ab) & 1u)) {
+                const float3 dr = site_of(xi, a) - site_of(xi, b);  // the molecule is whole
+                const float r2 = dot3(dr, dr);
+                float e;
+                // (in the water pattern the LJ site has no partner in its molecule)
+                const float sc = mol_pair_term<TOPO == 1 ? 0 : LJ, EW, ENERGY, true, TOPO>(A, ab, r2, A.mult[ab], e);
+                const float3 F = dr * sc;
 #pragma unroll
-            for (int a = 0; a < 4; a++) {
-#pragma unroll
-                for (int b = 0; b < 4; b++) {
-                    const int ab = 4 * a + b;
-                    if (a == b || !((A.selfm >> ab) & 1u)) continue;
-                    const float3 dr = xi[a] - xi[b];  // the molecule is whole
-                    const float r2 = dot3(dr, dr);
-                    float e;
-                    const float sc = mol_pair_term<LJ, EW, ENERGY, true, 0>(A, ab, r2, A.mult[ab], e);
-                    const float3 F = dr * sc;
-                    f[a] += F;
-                    if (ENERGY) en[a] += e;
-                    add_vir<VIR>(v[a], F, dr);
+                for (int k2 = 0; k2 < 4; k2++) {
+                    if (a != k2) continue;
+                    f[k2] += F;
+                    if (ENERGY) en[k2] += e;
+                    add_vir<VIR>(v[k2], F, dr);
                 }
             }
         }
