@@ -125,7 +125,7 @@ PairArgs make_args(State &s, FixPair &f) {
 // sites are reduced by shuffles and written by lanes 0..3 (one 64-byte store).
 // blocks per SM the kernel is compiled for: 80 registers, which lets the nine
 // charge pairs of a molecule pair be in flight beside one another.  Alone at
-// 4,096 / 32,768 molecules: 22.6 / 137 us (14 blocks, 72 registers: 24.2 / 144;
+// 4,096 / 32,768 molecules, own pairs still on one lane: 22.6 / 137 us (14 blocks, 72 registers: 24.2 / 144;
 // 10 blocks, 94: 22.5 / 136; 8 blocks, 106: 23.5 / 188)
 constexpr int kMolPairBlock = 64;
 constexpr int kMolPairBlocksPerSM = 12;
@@ -401,7 +401,9 @@ __global__ void __launch_bounds__(kMolPairBlock, kMolPairBlocksPerSM) k_pair_mol
             mol_pair_eval<LJ, EW, VIR, ENERGY, TOPO>(A, xi, qj[lane], make_float3(s4.x, s4.y, s4.z), f, en, v);
         }
         __syncwarp();  // the queue and the batch are reused by the warp's next slot
-        // the molecule's own site pairs, one per lane: pair ab in lane ab
+        // the molecule's own site pairs, one per lane: pair ab in lane ab (on
+        // lane 0 alone they were a seventh of the kernel's instructions: 28.6
+        // and 146.3 us as a stage at 4,096 and 32,768 molecules, so 27.2, 136.8)
         if (A.selfm) {
             const int a = lane >> 2 & 3, b = lane & 3, ab = lane & 15;
             if (lane < 16 && ((A.selfm >> ab) & 1u)) {
@@ -560,9 +562,9 @@ int pair_mol_launch(State &s, FixPair &f, int virialMode, bool accumulate, float
     // takes one molecule more than another is a tail: the grid is cut to the
     // fewest rounds the SMs' capacity allows and then to the fewest blocks
     // that need no more rounds.  Measured on B200, water step at 4,096
-    // molecules (two rounds, 7 blocks per SM): 53.0 us; 8, 10, 12 blocks per
-    // SM 53.4, 55.5, 59.4; 6 (three rounds) 65; with E3B 8, 10, 12: 62.9,
-    // 63.3, 64.4; at 32,768 (ten rounds, 11 blocks) 8, 10, 12: 321, 304, 303.
+    // molecules (two rounds, 7 blocks per SM): 50.4 us; 8, 10, 12 blocks per
+    // SM 50.3, 52.4, 57.3; with E3B 60.9; 61.0, 62.6, 64.8; at 32,768 (ten
+    // rounds, 11 blocks) 279; 8, 10, 12: 293, 276, 274.
     // Else, and for pairBlocksPerSM -1, a warp per molecule
     int mb = 0;
     if (s.pairBlocksPerSM > 0) {
