@@ -2,13 +2,15 @@
 //
 //  spread   map_charge_to_grid_order_5_cu (:174-217): order-5 charge
 //           assignment W_p_5 (:163-172), float atomics into a REAL grid
-//  FFT      cuFFT R2C (the reference runs C2C on a complex grid with a zero
+//  FFT      own transforms on cubic 32^3, 64^3 and 128^3 meshes (below); on
+//           others cuFFT R2C (the reference runs C2C on a complex grid with a zero
 //           imaginary part, :1307-1309; R2C computes the same half spectrum)
 //  E(k)     E_field_cu (:386-434): E_d(k) = i k_d G(k) rho(k).  The reference
 //           keeps only the real part after its C2C inverse, which drops the
 //           anti-Hermitian Nyquist-plane term of each component; that term is
 //           zeroed here so the C2R inverse gives the identical real field.
-//  inverse  one batched cuFFT C2R for the three components (:1340-1346)
+//  inverse  as the FFT; on other meshes one batched cuFFT C2R for the three
+//           components (:1340-1346)
 //  gather   Ewald_long_range_forces_order_5_cu (:561-630): F = Q q sum W E,
 //           E = -ifft / V
 //  G(k)     Green_function_cu (:314-366), evaluated once per box in FP64.

@@ -5,11 +5,12 @@
 //
 // Fused form (default): one per-molecule kernel does NH rescale + kick + drift
 // + SETTLE positions + M-site, and one does kick + M-site force
-// redistribution + SETTLE velocities + the FP64 sum of m v^2; the last block
-// of that kernel runs the chain update on the device, so no host round trip is
-// needed per step (the reference syncs for the kinetic energy every step,
-// FixNoseHoover.cu:1044-1056).  Atoms outside rigid molecules use per-atom
-// kernels with the same arithmetic.
+// redistribution + SETTLE velocities + the FP64 sum of m v^2 per block; a
+// one-block kernel behind it adds these and runs the chain update on the
+// device, so no host round trip is needed per step (the reference syncs for the
+// kinetic energy every step, FixNoseHoover.cu:1044-1056).  Atoms outside rigid
+// molecules use per-atom kernels with the same arithmetic; a few thousand of
+// them go from one step to the next in one kernel.
 #include <cooperative_groups.h>
 
 #include <cstdio>
