@@ -173,7 +173,10 @@ struct GPUData {
 // lanes read 128 contiguous bytes per row.
 struct GridGPU {
     int team = 8;        // threads per atom in build and force kernels
-    int cap = 0;         // per-atom capacity (multiple of team)
+    int cap = 0;         // per-atom capacity (multiple of team), 0: sized by the next build
+    // what cap and nlist were sized for (nlist_init)
+    int cap_team = 0, cap_n = 0;
+    float cap_cut = 0.f;
     int3 ns{0, 0, 0};    // cells per dimension
     int m = 2;           // stencil half width in cells (cells >= cut/m)
     int home_group = 2;  // home atoms a warp of the list build tests at once

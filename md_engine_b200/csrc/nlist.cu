@@ -1193,6 +1193,16 @@ int nlist_init(State &s) {
         set_error(MDX_ERR_ARG, "nThreadPerAtom must be 1,2,4,8,16 or 32 (got %d)", gr.team);
         return MDX_ERR_ARG;
     }
+    // a state prepared again keeps its list buffer, unless the rows it was
+    // sized for changed: with another team a capacity that is no multiple of
+    // it makes neighbouring rows overlap and the last one pass the buffer's
+    // end, and more atoms or a longer cutoff need more room
+    if (gr.cap_team != gr.team || gr.cap_n != n || gr.cap_cut != gr.cut) {
+        gr.cap = 0;
+        gr.cap_team = gr.team;
+        gr.cap_n = n;
+        gr.cap_cut = gr.cut;
+    }
     return nlist_exclusions(s);
 }
 
