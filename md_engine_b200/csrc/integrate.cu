@@ -316,8 +316,8 @@ __global__ void k_rigid_maps(const MolArgs a0, const MolArgs *__restrict__ tab, 
 // per-atom: NH rescale (rescale_no_tags_cu) + nve_v + nve_x (+ zero force)
 template <bool NH>
 __global__ void k_first_atoms(int n, float4 *__restrict__ xs, float4 *__restrict__ vs, float4 *__restrict__ fs,
-                              const uint32_t *__restrict__ ids, const uint8_t *__restrict__ rigid_by_id, float dt,
-                              float dtf, const NHChain *chain, int early) {
+                              const uint32_t *ids, const uint8_t *__restrict__ rigid_by_id, float dt, float dtf,
+                              const NHChain *chain, int early) {
     if (!early) pdl_wait();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -505,8 +505,11 @@ __global__ void __launch_bounds__(kEndThreads) k_step_end(const EndArgs a0, cons
 }
 
 // per-atom: postForce_cu (IntegratorVerlet.cu:610-627) + m v^2 partials
-__global__ void k_second_atoms(int n, float4 *__restrict__ vs, const float4 *__restrict__ fs,
-                               const uint32_t *__restrict__ ids, const uint8_t *__restrict__ rigid_by_id, float dtf,
+// (fs and ids are written by kernels that may still run when this one starts:
+// not marked __restrict__, which with const would let their loads, whose
+// addresses are known at the start, go ahead of the wait)
+__global__ void k_second_atoms(int n, float4 *__restrict__ vs, const float4 *fs, const uint32_t *ids,
+                               const uint8_t *__restrict__ rigid_by_id, float dtf,
                                double *__restrict__ partials, int part_off) {
     pdl_wait();
     pdl_trigger();  // k_step_end: one block, resident while this grid runs
