@@ -27,13 +27,12 @@ using pk::kPairBlock;
 template <int T>
 int launch_kind(const PairArgs &A, const PairArgs *tab, int nrep, int lj, int ck, bool vir, bool energy, bool acc,
                 cudaStream_t st) {
-    if (lj == 0 && ck == 1) pk::launch_t<T, 0, 1>(A, tab, nrep, vir, energy, acc, st);
-    else if (lj == 1 && ck == 1) pk::launch_t<T, 1, 1>(A, tab, nrep, vir, energy, acc, st);
-    else if (lj == 1 && ck == 0) pk::launch_t<T, 1, 0>(A, tab, nrep, vir, energy, acc, st);
-    else if (lj == 2 && ck == 1) pk::launch_t<T, 2, 1>(A, tab, nrep, vir, energy, acc, st);
-    else if (lj == 2 && ck == 0) pk::launch_t<T, 2, 0>(A, tab, nrep, vir, energy, acc, st);
-    else return pk::pair_launch_styles(A, tab, nrep, T, lj, ck, vir, energy, acc, st);
-    return 0;
+    if (lj == 0 && ck == 1) return pk::launch_t<T, 0, 1>(A, tab, nrep, vir, energy, acc, st);
+    if (lj == 1 && ck == 1) return pk::launch_t<T, 1, 1>(A, tab, nrep, vir, energy, acc, st);
+    if (lj == 1 && ck == 0) return pk::launch_t<T, 1, 0>(A, tab, nrep, vir, energy, acc, st);
+    if (lj == 2 && ck == 1) return pk::launch_t<T, 2, 1>(A, tab, nrep, vir, energy, acc, st);
+    if (lj == 2 && ck == 0) return pk::launch_t<T, 2, 0>(A, tab, nrep, vir, energy, acc, st);
+    return pk::pair_launch_styles(A, tab, nrep, T, lj, ck, vir, energy, acc, st);
 }
 
 int launch_any(const PairArgs &A, int team, int lj, int ck, bool vir, bool energy, bool acc, cudaStream_t st,

@@ -375,31 +375,34 @@ __global__ void __launch_bounds__(kPairBlock, T >= 32 ? 24 : 1) k_pair(const Pai
 
 // nrep > 1: tab holds nrep records, A is the largest replica (grid sizing)
 template <int T, int LJ, int CK>
-void launch_t(const PairArgs &A, const PairArgs *tab, int nrep, bool vir, bool energy, bool accumulate,
-              cudaStream_t st) {
+int launch_t(const PairArgs &A, const PairArgs *tab, int nrep, bool vir, bool energy, bool accumulate,
+             cudaStream_t st) {
     const int G = 32 / T;
     const int warps = (A.n + G - 1) / G;
     const dim3 blocks((warps * 32 + kPairBlock - 1) / kPairBlock, nrep);
-    const size_t nt2 = (size_t)A.ntypes * A.ntypes;
-    const size_t smem = LJ ? (size_t)A.np * nt2 * sizeof(float) : 0;
-    if (energy) {
-        k_pair<T, LJ, CK, false, true><<<blocks, kPairBlock, smem, st>>>(A, tab, 0);
-        MDX_LAUNCHED();
-        return;
+    // the type-pair table: packed words for the force kernels that take them,
+    // else the reference's np floats
+    const size_t words = energy || !kPackedLJ<LJ, false> ? (size_t)A.np : 4;
+    const size_t smem = LJ ? words * A.ntypes * A.ntypes * sizeof(float) : 0;
+    auto kern = energy ? k_pair<T, LJ, CK, false, true>
+                       : (vir ? k_pair<T, LJ, CK, true, false> : k_pair<T, LJ, CK, false, false>);
+    // beyond the default limit: from 56 species at four floats a pair, 65 at three
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        cudaGetLastError();
+        set_error(MDX_ERR_UNSUPPORTED, "the pair parameters of %d species (%zu bytes) exceed a block's shared memory",
+                  A.ntypes, smem);
+        return MDX_ERR_UNSUPPORTED;
     }
-    const size_t smem_f = kPackedLJ<LJ, false> ? nt2 * sizeof(float4) : smem;
-    auto kern = vir ? k_pair<T, LJ, CK, true, false> : k_pair<T, LJ, CK, false, false>;
-    // beyond the default limit (55 types; the unpacked table reached it at 64)
-    if (smem_f > 48 * 1024)
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f);
-    if (vir) {
-        kern<<<blocks, kPairBlock, smem_f, st>>>(A, tab, accumulate ? 1 : 0);
+    if (energy || vir) {
+        kern<<<blocks, kPairBlock, smem, st>>>(A, tab, accumulate && !energy ? 1 : 0);
         MDX_LAUNCHED();
+        MDX_CUDA_TRY(cudaGetLastError());
     } else {
-        launch_pdl(kern, blocks, dim3(kPairBlock), smem_f, st, A, tab, accumulate ? 1 : 0);
+        MDX_CUDA_TRY(launch_pdl(kern, blocks, dim3(kPairBlock), smem, st, A, tab, accumulate ? 1 : 0));
     }
+    return 0;
 }
-
 
 // the pair / charge evaluator pairs outside pair.cu's set (pair_styles.cu)
 int pair_launch_styles(const PairArgs &A, const PairArgs *tab, int nrep, int team, int lj, int ck, bool vir,

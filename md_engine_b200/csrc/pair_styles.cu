@@ -15,16 +15,16 @@ template <int T>
 int styles_kind(const PairArgs &A, const PairArgs *tab, int nrep, int lj, int ck, bool vir, bool energy, bool acc,
                 cudaStream_t st) {
     switch (lj * 3 + ck) {
-        case 0 * 3 + 2: launch_t<T, 0, 2>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 1 * 3 + 2: launch_t<T, 1, 2>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 2 * 3 + 2: launch_t<T, 2, 2>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 3 * 3 + 0: launch_t<T, 3, 0>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 3 * 3 + 1: launch_t<T, 3, 1>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 3 * 3 + 2: launch_t<T, 3, 2>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 4 * 3 + 0: launch_t<T, 4, 0>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 4 * 3 + 1: launch_t<T, 4, 1>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 4 * 3 + 2: launch_t<T, 4, 2>(A, tab, nrep, vir, energy, acc, st); return 0;
-        case 5 * 3 + 0: launch_t<T, 5, 0>(A, tab, nrep, vir, energy, acc, st); return 0;
+        case 0 * 3 + 2: return launch_t<T, 0, 2>(A, tab, nrep, vir, energy, acc, st);
+        case 1 * 3 + 2: return launch_t<T, 1, 2>(A, tab, nrep, vir, energy, acc, st);
+        case 2 * 3 + 2: return launch_t<T, 2, 2>(A, tab, nrep, vir, energy, acc, st);
+        case 3 * 3 + 0: return launch_t<T, 3, 0>(A, tab, nrep, vir, energy, acc, st);
+        case 3 * 3 + 1: return launch_t<T, 3, 1>(A, tab, nrep, vir, energy, acc, st);
+        case 3 * 3 + 2: return launch_t<T, 3, 2>(A, tab, nrep, vir, energy, acc, st);
+        case 4 * 3 + 0: return launch_t<T, 4, 0>(A, tab, nrep, vir, energy, acc, st);
+        case 4 * 3 + 1: return launch_t<T, 4, 1>(A, tab, nrep, vir, energy, acc, st);
+        case 4 * 3 + 2: return launch_t<T, 4, 2>(A, tab, nrep, vir, energy, acc, st);
+        case 5 * 3 + 0: return launch_t<T, 5, 0>(A, tab, nrep, vir, energy, acc, st);
     }
     set_error(MDX_ERR_UNSUPPORTED, "pair evaluator %d with charge evaluator %d is not built", lj, ck);
     return MDX_ERR_UNSUPPORTED;

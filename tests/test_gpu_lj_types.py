@@ -1,6 +1,6 @@
-"""Pair forces with the packed type-pair table at one species, several, and
-more than the default shared memory holds, with and without zero pairs,
-against a brute-force FP64 sum."""
+"""Pair forces, energy and virial with the type-pair table at one species,
+several, and more than the default shared memory holds, with and without zero
+pairs, against a brute-force FP64 sum."""
 import numpy as np
 import pytest
 
@@ -9,8 +9,10 @@ from md_engine_b200 import Bounds, FixLJCut, FixLJCutFS, State, Vector
 pytestmark = pytest.mark.gpu
 
 
+# 55 and 64 species are the last whose table of four and of three floats a pair
+# fits the default
 @pytest.mark.parametrize("style", [FixLJCut, FixLJCutFS])
-@pytest.mark.parametrize("ntypes,zero", [(1, False), (3, True), (60, False)])
+@pytest.mark.parametrize("ntypes,zero", [(1, False), (3, True), (60, False), (70, False)])
 def test_forces_by_species(style, ntypes, zero):
     rng = np.random.default_rng(ntypes)
     n, L, rc = 1000, 11.0, 2.5
@@ -35,8 +37,9 @@ def test_forces_by_species(style, ntypes, zero):
         fix.setParameter("eps", h, h, eps[k])
     st.activateFix(fix)
     st.prepare()
-    st.computeForces()
+    st.computeForces(1)
     f = st.getAtoms()[2]
+    virial, energy = st.virials()[1], st.potentialEnergy()[0]
     d = pos[:, None] - pos[None]
     d -= L * np.round(d / L)
     r2 = (d ** 2).sum(2)
@@ -54,3 +57,34 @@ def test_forces_by_species(style, ntypes, zero):
     ref = np.einsum("ij,ijc->ic", np.where(r2 < rc * rc, k, 0.0), d)
     rms = np.sqrt(np.mean(np.sum(ref ** 2, 1)))
     assert np.max(np.linalg.norm(f - ref, axis=1)) < 2e-4 * rms
+    s6 = np.where(r2 < rc * rc, s ** 6 / r2 ** 3, 0.0)
+    c6 = np.where(r2 < rc * rc, s ** 6 / rc ** 6, 0.0)
+    u = 4.0 * e * (s6 * (s6 - 1.0) - c6 * (c6 - 1.0))
+    if style is FixLJCutFS:
+        u = u + np.where(r2 < rc * rc, over_r(rc * rc) * rc * (np.sqrt(r2) - rc), 0.0)
+    w = np.where(r2 < rc * rc, k, 0.0)
+    refv = 0.5 * np.array([np.sum(w * d[..., a] * d[..., b])
+                           for a, b in ((0, 0), (1, 1), (2, 2), (0, 1), (0, 2), (1, 2))])
+    # FP32 separations are off by up to 2^-23 L = 1.3e-6, 1.6e-6 of the shortest
+    # ones: 12 times that in r^-12, beside the terms' own rounding
+    assert abs(energy - 0.5 * u.sum()) < 3e-5 * 0.5 * np.sum(4.0 * e * (s6 * (s6 + 1.0) + c6))
+    assert np.max(np.abs(virial - refv)) < 3e-5 * 0.5 * np.sum(24.0 * e * s6 * (2.0 * s6 + 1.0))
+
+
+def test_more_species_than_shared_memory_holds():
+    n, ntypes = 150, 130
+    st = State()
+    st.units.setLJ()
+    st.bounds = Bounds(st, lo=Vector(0, 0, 0), hi=Vector(20, 20, 20))
+    st.rCut, st.padding, st.dt = 2.5, 0.3, 0.001
+    names = [f"T{k}" for k in range(ntypes)]
+    for h in names:
+        st.atomParams.addSpecies(h, 1.0, 1)
+    st.addAtoms([names[k % ntypes] for k in range(n)], np.random.default_rng(0).uniform(0, 20, (n, 3)), np.zeros(n))
+    fix = FixLJCut(st, "pair")
+    for h in names:
+        fix.setParameter("sig", h, h, 0.1)
+        fix.setParameter("eps", h, h, 1.0)
+    st.activateFix(fix)
+    with pytest.raises(RuntimeError, match="130 species"):
+        st.prepare()
