@@ -325,7 +325,8 @@ __global__ void __launch_bounds__(kPairBlock, T >= 32 ? 24 : 1) k_pair(const Pai
         }
     }
     if (LJ && CK) {
-        const bool lj_row = valid && ti < 32 && ((A.lj_types >> ti) & 1u);
+        // (with more than 32 species the mask is not kept: every type may have one)
+        const bool lj_row = valid && (ti >= 32 || ((A.lj_types >> ti) & 1u));
         const bool q_row = valid && qi != 0.f;
         if (!__any_sync(0xffffffffu, lj_row)) {
             if (valid) pair_row<T, 0, CK, VIR, ENERGY>(A, sp, nt2, i, ti, qi, xi, row, cnt, t, fx, fy, fz, en, v);

@@ -1,10 +1,12 @@
 """Pair forces, energy and virial with the type-pair table at one species,
 several, and more than the default shared memory holds, with and without zero
 pairs, against a brute-force FP64 sum."""
+import math
+
 import numpy as np
 import pytest
 
-from md_engine_b200 import Bounds, FixLJCut, FixLJCutFS, State, Vector
+from md_engine_b200 import Bounds, FixChargePairDSF, FixLJCut, FixLJCutFS, State, Vector
 
 pytestmark = pytest.mark.gpu
 
@@ -88,3 +90,48 @@ def test_more_species_than_shared_memory_holds():
     st.activateFix(fix)
     with pytest.raises(RuntimeError, match="130 species"):
         st.prepare()
+
+
+def test_charged_species_beyond_the_thirty_second():
+    rng = np.random.default_rng(40)
+    n, L, rc, alpha, ntypes = 1000, 11.0, 2.5, 0.4, 40
+    g = np.stack(np.meshgrid(*[np.arange(10)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = ((g + 0.5) * 1.1 + rng.uniform(-0.1, 0.1, (n, 3))).astype(np.float32).astype(np.float64)
+    types = rng.integers(32, ntypes, n)  # no atom of the first 32 species
+    q = np.where(np.arange(n) % 2 == 0, 0.5, -0.5)
+    st = State()
+    st.units.setLJ()
+    st.bounds = Bounds(st, lo=Vector(0, 0, 0), hi=Vector(L, L, L))
+    st.rCut, st.padding, st.dt = rc, 0.3, 0.001
+    names = [f"T{k}" for k in range(ntypes)]
+    for h in names:
+        st.atomParams.addSpecies(h, 1.0, 1)
+    st.addAtoms([names[t] for t in types], pos, q)
+    fix = FixLJCut(st, "pair")
+    for h in names:
+        fix.setParameter("sig", h, h, 1.0)
+        fix.setParameter("eps", h, h, 1.0)
+    st.activateFix(fix)
+    dsf = FixChargePairDSF(st, "dsf")
+    dsf.setParameters(alpha, rc)
+    st.activateFix(dsf)
+    st.prepare()
+    st.computeForces()
+    f = st.getAtoms()[2]
+    d = pos[:, None] - pos[None]
+    d -= L * np.round(d / L)
+    r2 = (d ** 2).sum(2)
+    np.fill_diagonal(r2, 1e9)
+    r = np.sqrt(r2)
+    erfc = np.vectorize(math.erfc)
+    A = 2.0 * alpha / math.sqrt(math.pi)
+    shift = math.erfc(alpha * rc) / rc ** 2 + A * math.exp(-(alpha * rc) ** 2) / rc
+    near = r < rc
+    lj = 24.0 * (2.0 / r2 ** 6 - 1.0 / r2 ** 3) / r2
+    qq = q[:, None] * q[None]
+    k = np.zeros_like(r)
+    k[near] = lj[near] + qq[near] * (erfc(alpha * r[near]) / r2[near] + A * np.exp(-alpha ** 2 * r2[near]) / r[near]
+                                     - shift) / r[near]
+    ref = np.einsum("ij,ijc->ic", k, d)
+    rms = np.sqrt(np.mean(np.sum(ref ** 2, 1)))
+    assert np.max(np.linalg.norm(f - ref, axis=1)) < 2e-4 * rms
