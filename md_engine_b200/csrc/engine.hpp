@@ -69,6 +69,7 @@ struct DBuf {
     T *p = nullptr;
     size_t n = 0;
     bool own = true;  // false: a view into memory owned elsewhere (a pool)
+    std::shared_ptr<const void> pool;  // of a view: what it keeps alive
     int alloc(size_t count) {
         if (count <= n && p) return 0;
         if (!own) {
@@ -92,12 +93,14 @@ struct DBuf {
         p = nullptr;
         n = 0;
         own = true;
+        pool.reset();
     }
-    void view(T *q, size_t count) {
+    void view(T *q, size_t count, std::shared_ptr<const void> owner) {
         release();
         p = q;
         n = count;
         own = false;
+        pool = std::move(owner);
     }
     ~DBuf() { release(); }
     DBuf() = default;
@@ -576,8 +579,9 @@ class State {
     std::vector<std::vector<int>> molecules;
     std::vector<ConfigWriter *> writers;
     ConfigReader *reader = nullptr;
-    // bumped at every box change (a barostat): captured step graphs hold the
-    // box by value and are rebuilt when it moves
+    // bumped at every box change (a barostat) and when a batch takes the state
+    // in: captured step graphs hold the box by value, and the addresses of the
+    // mesh buffers, and are captured again
     uint64_t box_gen = 0;
     State();
     ~State();
@@ -629,8 +633,9 @@ class Batch {
     int max_n = 0, max_mol = 0, max_cell = 0;
     size_t max_nk = 0;
     // P3M: replicas grouped by mesh size; each class owns contiguous pools
-    // that the replicas' FixChargeEwald buffers view, so one batched cuFFT
-    // plan per class transforms every replica of that class
+    // that the replicas' FixChargeEwald buffers view (and keep alive, for a
+    // state that outlives the batch), so one batched cuFFT plan per class
+    // transforms every replica of that class
     struct FFTClass {
         int3 sz{0, 0, 0};
         std::vector<int> reps;
@@ -648,7 +653,7 @@ class Batch {
     // into each replica's per-step reciprocal buffer
     bool p3m_mol = false;
     DBuf<char> tab_p3m_mol;
-    std::vector<std::unique_ptr<FFTClass>> fft;
+    std::vector<std::shared_ptr<FFTClass>> fft;
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
     std::map<std::pair<int, int>, uint64_t> graph_kernels;
     Batch();

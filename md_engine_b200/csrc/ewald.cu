@@ -1319,10 +1319,11 @@ int batch_p3m_prepare(Batch &b) {
         if (int e = c.e_r.alloc(K * 3 * ng)) return e;
         for (int j = 0; j < K; j++) {
             FixChargeEwald *f = b.reps[c.reps[j]]->ewaldFix();
-            f->rho.view(c.rho.p + j * ng, ng);
-            f->rho_k.view(c.rho_k.p + j * nk, nk);
-            f->e_k.view(c.e_k.p + j * 3 * nk, 3 * nk);
-            f->e_r.view(c.e_r.p + j * 3 * ng, 3 * ng);
+            f->rho.view(c.rho.p + j * ng, ng, cp);
+            f->rho_k.view(c.rho_k.p + j * nk, nk, cp);
+            f->e_k.view(c.e_k.p + j * 3 * nk, 3 * nk, cp);
+            f->e_r.view(c.e_r.p + j * 3 * ng, 3 * ng, cp);
+            b.reps[c.reps[j]]->box_gen++;  // graphs captured so far hold the addresses before
         }
         c.own = true;
         for (int j = 0; j < K; j++) c.own = c.own && b.reps[c.reps[j]]->ewaldFix()->own_fft;

@@ -126,3 +126,26 @@ def test_autotune_picks_a_team_and_keeps_the_trajectory():
         d = np.abs(st.getAtoms()[0] - ref.getAtoms()[0]).max()
         assert d < 1e-3, d
         assert st.status()[0] == 0
+
+
+def test_states_run_alone_before_and_after_a_batch():
+    """the batch moves the replicas' mesh buffers into its pools: graphs that a
+    replica's own integrator captured before, and the state after the batch is
+    gone, must use the buffers as they are then"""
+    m, T, seed = 300, 300.0, 61
+    st, ref = _replica(m, T, seed)[0], _replica(m, T, seed)[0]
+    own, whole = IntegratorVerlet(st), IntegratorVerlet(ref)
+    own.run(10)
+    b = BatchReplicas([st])
+    b.run(10)
+    own.run(10)
+    del b
+    own.run(10)
+    st.computeForces()
+    for _ in range(4):
+        whole.run(10)
+    ref.computeForces()
+    (x, _, f), (xr, _, fr) = st.getAtoms(), ref.getAtoms()
+    assert np.abs(x - xr).max() < 1e-3
+    assert np.abs(f - fr).max() < 2e-2 * np.sqrt(np.mean(np.sum(fr ** 2, 1)))
+    assert st.status()[0] == 0
