@@ -155,6 +155,9 @@ int Batch::prepare() {
     for (State *s : reps)
         if (s->nThreadPerAtom) team = s->nThreadPerAtom;
     if (!team) team = 8;
+    std::vector<State *> other;  // prepared on their own, with the lanes per atom of a single system
+    for (State *s : reps)
+        if (s->prepared && !s->nThreadPerAtom && s->grid.team != team) other.push_back(s);
     for (State *s : reps) {
         if (s->nThreadPerAtom && s->nThreadPerAtom != team) {
             set_error(MDX_ERR_UNSUPPORTED, "replicas ask for different nThreadPerAtom");
@@ -168,6 +171,9 @@ int Batch::prepare() {
     for (State *s : reps)
         if (!s->prepared)
             if (int e = s->prepare()) return e;
+    for (State *s : other)
+        if (!s->mf.on)
+            if (int e = nlist_set_team(*s, team)) return e;
     MDX_CUDA_TRY(cudaDeviceSynchronize());
     max_n = max_mol = max_cell = 0;
     ps.clear();

@@ -580,8 +580,8 @@ class State {
     std::vector<ConfigWriter *> writers;
     ConfigReader *reader = nullptr;
     // bumped at every box change (a barostat) and when a batch takes the state
-    // in: captured step graphs hold the box by value, and the addresses of the
-    // mesh buffers, and are captured again
+    // in: captured step graphs hold the box and the list's shape by value, and
+    // the addresses of the mesh buffers, and are captured again
     uint64_t box_gen = 0;
     State();
     ~State();
@@ -695,6 +695,7 @@ void host_copy(void *dst, const void *src, size_t bytes);
 // ---------------------------------------------------------------- kernels
 // neighbour list (nlist.cu)
 int nlist_rebuild(State &s, bool force, bool conditional, cudaStream_t bstream = nullptr);
+int nlist_set_team(State &s, int team);
 int nlist_init(State &s);
 int nlist_exclusions(State &s);
 int nlist_set_interactions(State &s);

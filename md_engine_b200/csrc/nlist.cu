@@ -1267,6 +1267,14 @@ int nlist_rebuild(State &s, bool force, bool conditional, cudaStream_t bstream) 
     return 0;
 }
 
+// a prepared state's list in rows for another number of lanes per atom
+int nlist_set_team(State &s, int team) {
+    s.grid.team = s.grid.cap_team = team;
+    s.grid.cap = 0;
+    s.box_gen++;
+    return nlist_rebuild(s, true, false);
+}
+
 // The molecule form's rebuild group: the same skin check, then the sort by
 // molecule, then (on bstream when given, beside the step's first half) the
 // molecule-pair list and the E3B molecule list cut from it.

@@ -149,3 +149,28 @@ def test_states_run_alone_before_and_after_a_batch():
     assert np.abs(x - xr).max() < 1e-3
     assert np.abs(f - fr).max() < 2e-2 * np.sqrt(np.mean(np.sum(fr ** 2, 1)))
     assert st.status()[0] == 0
+
+
+@pytest.mark.parametrize("e3b", [False, True])
+def test_replicas_prepared_on_their_own(e3b):
+    """boxes run alone with the automatic lanes per atom of a small system (32
+    and 16, a batch takes 8), then batched: as the same boxes run on alone"""
+    boxes = [systems.water_tip4p2005(nmol=m, T=T, seed=m) for m, T in ((216, 290.0), (900, 310.0))]
+    states, refs = [], []
+    for out in (states, refs):
+        for sysd in boxes:
+            st, _ = systems.build_water_state(sysd, rcut=6.5, skin=1.0, grid=32, e3b=e3b)
+            st.pairForm = 1
+            IntegratorVerlet(st).run(10)
+            out.append(st)
+    assert [int(st.nThreadPerAtom) for st in states] == [32, 16]
+    b = BatchReplicas(states)
+    b.prepare()
+    assert [int(st.nThreadPerAtom) for st in states] == [8, 8]
+    b.run(20)
+    for sysd, st, ref in zip(boxes, states, refs):
+        IntegratorVerlet(ref).run(20)
+        d = st.getAtoms()[0] - ref.getAtoms()[0]
+        d -= sysd.L * np.rint(d / sysd.L)
+        assert np.abs(d).max() < 1e-3
+        assert st.status()[0] == 0
