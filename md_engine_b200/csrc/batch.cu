@@ -72,7 +72,6 @@ void Batch::reset() {
     max_n = max_mol = max_cell = 0;
     ps.clear();
     mfi.clear();
-    max_nk = 0;
     prepared = false;
 }
 

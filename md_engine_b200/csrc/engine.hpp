@@ -631,7 +631,6 @@ class Batch {
     int max_n_ps = 0, max_cell_ps = 0, max_mol_mf = 0, max_mcell = 0;
     int pair_big = 0;
     int max_n = 0, max_mol = 0, max_cell = 0;
-    size_t max_nk = 0;
     // P3M: replicas grouped by mesh size; each class owns contiguous pools
     // that the replicas' FixChargeEwald buffers view (and keep alive, for a
     // state that outlives the batch), so one batched cuFFT plan per class
@@ -646,8 +645,10 @@ class Batch {
         // class's replicas (a table of their field pointers), no cuFFT
         bool own = false;
         DBuf<char> tab;
+        DBuf<char> p3m;  // the P3M records of the class's replicas (batches not all own)
+        int max_n = 0;
     };
-    bool p3m_own = false;  // every class on the own FFT: the gather reads the float4 fields
+    bool p3m_own = false;  // every class on the own FFT: one gather for all replicas
     // and every replica's molecules fit the molecule form of spread and
     // gather: spread and gather by molecule, the gather on the P3M branch
     // into each replica's per-step reciprocal buffer

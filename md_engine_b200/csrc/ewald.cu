@@ -1342,7 +1342,6 @@ int batch_p3m_prepare(Batch &b) {
                 return MDX_ERR_CUDA;
             }
         }
-        b.max_nk = std::max(b.max_nk, nk);
     }
     b.p3m_own = true;
     for (auto &cp : b.fft) b.p3m_own = b.p3m_own && cp->own;
@@ -1350,6 +1349,18 @@ int batch_p3m_prepare(Batch &b) {
     for (int r = 0; r < R; r++) h[r] = p3m_args(*b.reps[r], *b.reps[r]->ewaldFix());
     if (int e = b.tab_p3m.alloc(R * sizeof(P3MArgs))) return e;
     MDX_CUDA_TRY(cudaMemcpy(b.tab_p3m.p, h.data(), R * sizeof(P3MArgs), cudaMemcpyHostToDevice));
+    if (!b.p3m_own)
+        for (auto &cp : b.fft) {
+            const int K = (int)cp->reps.size();
+            std::vector<P3MArgs> hc(K);
+            cp->max_n = 0;
+            for (int j = 0; j < K; j++) {
+                hc[j] = h[cp->reps[j]];
+                cp->max_n = std::max(cp->max_n, hc[j].n);
+            }
+            if (int e = cp->p3m.alloc(K * sizeof(P3MArgs))) return e;
+            MDX_CUDA_TRY(cudaMemcpy(cp->p3m.p, hc.data(), K * sizeof(P3MArgs), cudaMemcpyHostToDevice));
+        }
     // the molecule form of spread and gather, as the single system's fused
     // step: the charged sites of each molecule only, the reciprocal forces
     // stored into each replica's per-step buffer by the P3M branch itself
@@ -1372,7 +1383,6 @@ int batch_p3m_spread_solve(Batch &b, cudaStream_t st) {
     const P3MArgs *tab = reinterpret_cast<const P3MArgs *>(b.tab_p3m.p);
     P3MArgs A = p3m_args(*b.reps[0], *b.reps[0]->ewaldFix());  // sizing only
     A.n = b.max_n;
-    A.nk = b.max_nk;
     for (auto &c : b.fft) MDX_CUDA_TRY(cudaMemsetAsync(c->rho.p, 0, c->rho.n * sizeof(float), st));
     if (b.p3m_mol) {
         const int warps = (b.max_mol + 1) / 2;
@@ -1381,11 +1391,12 @@ int batch_p3m_spread_solve(Batch &b, cudaStream_t st) {
         k_spread5<<<dim3((A.n + 47) / 48, R), 256, 0, st>>>(A, tab);
     }
     MDX_LAUNCHED();
-    if (b.p3m_own) {
-        // each mesh class: R2C + E(k) + 3 C2R as the single system's three
-        // FFT kernels, one launch each over the class's replicas
-        for (auto &c : b.fft) {
-            const unsigned K = (unsigned)c->reps.size();
+    // each mesh class by itself: the three FFT kernels of the single system
+    // over the class's replicas, or batched cuFFT around the E(k) kernel where
+    // the own FFT does not serve the mesh
+    for (auto &c : b.fft) {
+        const unsigned K = (unsigned)c->reps.size();
+        if (c->own) {
             const FFTArgs a0 = fft_args(*b.reps[c->reps[0]], *b.reps[c->reps[0]]->ewaldFix());
             const FFTArgs *ft = reinterpret_cast<const FFTArgs *>(c->tab.p);
             auto launch = [&](auto kern, dim3 grid, dim3 block, size_t smem) {
@@ -1395,26 +1406,24 @@ int batch_p3m_spread_solve(Batch &b, cudaStream_t st) {
             else if (c->sz.x == 64) launch_solve<64>(launch, K);
             else launch_solve<128>(launch, K);
             g_launches += 3;
+            continue;
         }
-        MDX_CUDA_TRY(cudaGetLastError());
-        return 0;
-    }
-    for (auto &c : b.fft) {
         cufftSetStream(c->r2c, st);
         if (cufftExecR2C(c->r2c, c->rho.p, (cufftComplex *)c->rho_k.p) != CUFFT_SUCCESS) {
             set_error(MDX_ERR_CUDA, "batched cufftExecR2C failed");
             return MDX_ERR_CUDA;
         }
-    }
-    k_efield<<<dim3((unsigned)((A.nk + 255) / 256), R), 256, 0, st>>>(A, tab);
-    MDX_LAUNCHED();
-    for (auto &c : b.fft) {
+        const size_t nk = (size_t)c->sz.x * c->sz.y * (c->sz.z / 2 + 1);
+        k_efield<<<dim3((unsigned)((nk + 255) / 256), K), 256, 0, st>>>(A,
+                                                                        reinterpret_cast<const P3MArgs *>(c->p3m.p));
+        MDX_LAUNCHED();
         cufftSetStream(c->c2r, st);
         if (cufftExecC2R(c->c2r, (cufftComplex *)c->e_k.p, c->e_r.p) != CUFFT_SUCCESS) {
             set_error(MDX_ERR_CUDA, "batched cufftExecC2R failed");
             return MDX_ERR_CUDA;
         }
     }
+    MDX_CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
@@ -1434,8 +1443,15 @@ int batch_p3m_gather(Batch &b, cudaStream_t st) {
         MDX_LAUNCHED();
         return 0;
     }
-    k_gather<true><<<dim3((A.n + 127) / 128, (unsigned)b.reps.size()), 128, 0, st>>>(A, tab);
-    MDX_LAUNCHED();
+    for (auto &c : b.fft) {
+        const unsigned K = (unsigned)c->reps.size();
+        const P3MArgs *ct = reinterpret_cast<const P3MArgs *>(c->p3m.p);
+        if (c->own)
+            k_gather4<false, true><<<dim3(mesh_blocks<false>(c->max_n, 0), K), kMeshWarps * 32, 0, st>>>(A, ct);
+        else
+            k_gather<true><<<dim3((c->max_n + 127) / 128, K), 128, 0, st>>>(A, ct);
+        MDX_LAUNCHED();
+    }
     return 0;
 }
 

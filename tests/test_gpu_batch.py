@@ -174,3 +174,28 @@ def test_replicas_prepared_on_their_own(e3b):
         d -= sysd.L * np.rint(d / sysd.L)
         assert np.abs(d).max() < 1e-3
         assert st.status()[0] == 0
+
+
+def test_meshes_of_both_ffts_in_one_batch():
+    """meshes that the own FFT serves (128^3, 32^3) beside one it does not"""
+    spec = [(300, (128, 128, 128)), (256, (64, 32, 32)), (280, (32, 32, 32)), (310, (64, 32, 32))]
+
+    def boxes():
+        out = []
+        for m, mesh in spec:
+            sysd = systems.water_tip4p2005(nmol=m, seed=m)
+            st, fixes = systems.build_water_state(sysd, rcut=RCUT, skin=SKIN, grid=64)
+            fixes["ewald"].setParameters(*mesh, RCUT, 5)
+            st.nThreadPerAtom = 8
+            out.append((sysd, st))
+        return out
+
+    batch, alone = boxes(), boxes()
+    b = BatchReplicas([st for _, st in batch])
+    b.run(20)
+    for (sysd, st), (_, ref) in zip(batch, alone):
+        IntegratorVerlet(ref).run(20)
+        d = st.getAtoms()[0] - ref.getAtoms()[0]
+        d -= sysd.L * np.rint(d / sysd.L)
+        assert np.abs(d).max() < 1e-3
+        assert st.status()[0] == 0
