@@ -36,14 +36,10 @@ using namespace mdx;
 
 namespace {
 int get_atoms(State &s, double *pos, double *vel, double *force) {
-    if (int e = s.download()) return e;
     double *const out[3] = {pos, vel, force};
-    if (s.uploaded && (size_t)s.gpd.n == s.atoms.size()) {
-        for (int k = 0; k < 3; k++)
-            if (out[k]) host_copy(out[k], s.stageHost(k), 3 * s.atoms.size() * sizeof(double));
-        return 0;
-    }
+    if (s.uploaded && (size_t)s.gpd.n == s.atoms.size()) return s.download(out);
     // with atoms that are not on the device yet
+    if (int e = s.download()) return e;
     for (size_t i = 0; i < s.atoms.size(); i++) {
         const HostAtom &a = s.atoms[i];
         for (int d = 0; d < 3; d++) {
@@ -52,22 +48,6 @@ int get_atoms(State &s, double *pos, double *vel, double *force) {
             if (force) force[3 * i + d] = a.force[d];
         }
     }
-    return 0;
-}
-
-int put_atoms(State &s, const double *pos, const double *vel) {
-    if (int e = s.stageAlloc()) return e;
-    MDX_CUDA_TRY(cudaStreamSynchronize(s.stream));  // the staging may be on its way out
-    const double *const in[2] = {pos, vel};
-    for (int k = 0; k < 2; k++)
-        if (in[k])
-            if (int e = s.stagePut(k, in[k])) return e;
-    for (int i = 0; i < s.gpd.n; i++)
-        for (int d = 0; d < 3; d++) {
-            if (pos) s.atoms[i].pos[d] = pos[3 * i + d];
-            if (vel) s.atoms[i].vel[d] = vel[3 * i + d];
-        }
-    MDX_CUDA_TRY(cudaStreamSynchronize(s.stream));
     return 0;
 }
 }  // namespace
@@ -280,7 +260,7 @@ int mdx_state_put_atoms(mdx_state *st, const double *pos, const double *vel) {
         set_error(MDX_ERR_STATE, "state has no device copy yet (call mdx_prepare or run first)");
         return MDX_ERR_STATE;
     }
-    GUARD(return put_atoms(*st->s, pos, vel);)
+    GUARD(return st->s->put(pos, vel);)
 }
 int mdx_state_activate_fix(mdx_state *st, mdx_fix *fix) {
     ARG_CHECK(st && fix, "null argument");

@@ -559,15 +559,7 @@ class State {
     // a rebuild step
     cudaStream_t side[3] = {nullptr, nullptr, nullptr};
     cudaEvent_t ev_fork = nullptr, ev_join[3] = {nullptr, nullptr, nullptr}, ev_sorted = nullptr;
-    // host arrays by atom id cross here: (n,3) FP64 positions, velocities and
-    // forces, pinned on the host and on the device, which rounds and orders
-    double *stage_h = nullptr;
-    size_t stage_n = 0;
-    DBuf<double> stage_d;
-    int stageAlloc();
-    int stagePut(int k, const double *src);  // array k (0 or 1) onto the device stream, on `stream`
-    int stageGet(int k);                     // array k into stage_h, on `stream`
-    double *stageHost(int k) const { return stage_h + 3 * (size_t)k * gpd.n; }
+    std::shared_ptr<void> stage_own;  // staging of its own (StagingUse::take)
     bool uploaded = false;   // device copy is authoritative
     bool prepared = false;
     bool requiresCharges = false;
@@ -588,7 +580,11 @@ class State {
     int typeFromHandle(const std::string &h) const;
     void setBox();
     int upload();
-    int download();
+    // the device's positions, velocities and forces into the host atoms and,
+    // where given, into out's (n,3) arrays by atom id
+    int download(double *const *out = nullptr);
+    // (n,3) arrays by atom id (either may be null) into the device's streams
+    int put(const double *pos, const double *vel);
     int prepare();
     int buildNeighborList(bool force);
     int computeForces(int virialMode);
@@ -692,6 +688,27 @@ int batch_rigid_maps(Batch &b);
 
 // memcpy, in a few threads for long arrays
 void host_copy(void *dst, const void *src, size_t bytes);
+
+// (n,3) FP64 arrays by atom id crossing between the host and the device's
+// sorted FP32 streams, which the device rounds, widens and orders.  They go
+// in pieces through a staging slot, taken for the time of one call: the
+// state's device is current meanwhile, and nothing is under way in the slot
+// when it is handed on (state.cu)
+struct StagingSlot;
+struct StagingUse {
+    State &s;
+    StagingSlot *slot = nullptr;
+    int back = -1;      // the device to go back to
+    bool busy = false;  // copies may be under way
+    int pieces = 0;
+    explicit StagingUse(State &st) : s(st) {}
+    ~StagingUse();
+    StagingUse(const StagingUse &) = delete;
+    StagingUse &operator=(const StagingUse &) = delete;
+    int take(size_t want);               // a slot of this many doubles, or the most there is
+    int put(int k, const double *src);   // positions (0) or velocities (1), queued on the state's stream
+    int get(double *const out[3]);       // positions, velocities, forces (any may be null), complete on return
+};
 
 // ---------------------------------------------------------------- kernels
 // neighbour list (nlist.cu)

@@ -26,8 +26,6 @@ class IntegratorVerlet {
     explicit IntegratorVerlet(State *st) : s(st) {}
     ~IntegratorVerlet() {
         clearGraphs();
-        for (cudaEvent_t e : ev_out)
-            if (e) cudaEventDestroy(e);
     }
     void clearGraphs() {
         for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
@@ -354,7 +352,6 @@ class IntegratorVerlet {
     // run with host buffers in/out (the call a host program makes): inputs are
     // copied from pinned staging and scattered by id, outputs gathered by id
     // and copied back, all inside the call
-    cudaEvent_t ev_out[3] = {nullptr, nullptr, nullptr};
     int runHost(int nturns, const double *pin, const double *vin, double *pout, double *vout, double *fout) {
         if (s->barostatFix() || (s->nhFix() && s->nhFix()->barostatting)) {
             set_error(MDX_ERR_UNSUPPORTED, "a barostat changes the box between steps: use mdx_integrator_run");
@@ -364,10 +361,8 @@ class IntegratorVerlet {
             clearGraphs();
             if (int e = s->prepare()) return e;
         }
-        const size_t bytes = 3 * (size_t)s->gpd.n * sizeof(double);
-        if (int e = s->stageAlloc()) return e;
-        for (cudaEvent_t &e : ev_out)
-            if (!e) MDX_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        StagingUse use(*s);
+        if (int e = use.take(6 * (size_t)s->gpd.n)) return e;
         // the step graphs of this call exist before any copy is queued
         if (int e = precapture(nturns, 0)) return e;
         // inputs: a plain copy into pinned memory, one async copy each, the
@@ -375,7 +370,7 @@ class IntegratorVerlet {
         const double *ins[2] = {pin, vin};
         for (int k = 0; k < 2; k++)
             if (ins[k])
-                if (int e = s->stagePut(k, ins[k])) return e;
+                if (int e = use.put(k, ins[k])) return e;
         const int P = s->periodicInterval > 0 ? s->periodicInterval : 1;
         int done = 0;
         while (done < nturns) {
@@ -393,17 +388,9 @@ class IntegratorVerlet {
         double *outs[3] = {pout, vout, fout};
         MDX_CUDA_TRY(cudaMemcpyAsync(s->h_status, s->d_status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost,
                                      s->stream));
-        for (int k = 0; k < 3; k++) {
-            if (!outs[k]) continue;
-            if (int e = s->stageGet(k)) return e;
-            MDX_CUDA_TRY(cudaEventRecord(ev_out[k], s->stream));
-        }
-        for (int k = 0; k < 3; k++) {
-            if (!outs[k]) continue;
-            MDX_CUDA_TRY(cudaEventSynchronize(ev_out[k]));
-            host_copy(outs[k], s->stageHost(k), bytes);
-        }
+        if (int e = use.get(outs)) return e;
         MDX_CUDA_TRY(cudaStreamSynchronize(s->stream));
+        use.busy = false;
         if (s->h_status->bits) return s->checkStatus();
         return 0;
     }

@@ -7,6 +7,8 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <map>
+#include <mutex>
 #include <system_error>
 #include <thread>
 #include <vector>
@@ -50,13 +52,101 @@ int num_sms() {
     return cache[dev];
 }
 
+// Host arrays cross in pieces through pinned and device memory that all states
+// of a device share: kStageMost doubles at most, for two pieces under way (or
+// one that is all there is), in kSlots slots of which a call takes a free one
+// (a state takes one of its own when there is none), given back with the
+// process's last state.
+// Pinned memory for each state, 72 bytes an atom taken by its first getAtoms,
+// made the first pass of 64 new replicas 50 ms; it takes 34 so.
+constexpr size_t kStageMost = size_t(1) << 21;
+struct StagingSlot {
+    std::mutex mu;
+    double *h = nullptr, *d = nullptr;
+    cudaEvent_t done[2] = {nullptr, nullptr};  // of the two pieces under way
+    size_t size = 0;  // doubles
+    int reserve(size_t want) {
+        for (cudaEvent_t &e : done)
+            if (!e) MDX_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        want = std::min((want + 0x3fff) & ~size_t(0x3fff), kStageMost);
+        if (want <= size) return 0;
+        drop();
+        MDX_CUDA_TRY(cudaMallocHost(&h, want * sizeof(double)));
+        MDX_CUDA_TRY(cudaMalloc(&d, want * sizeof(double)));
+        size = want;
+        return 0;
+    }
+    void drop() {
+        if (h) cudaFreeHost(h);
+        if (d) cudaFree(d);
+        h = d = nullptr;
+        size = 0;
+    }
+    ~StagingSlot() {
+        drop();
+        for (cudaEvent_t e : done)
+            if (e) cudaEventDestroy(e);
+    }
+};
+
+namespace {
+struct Staging {
+    static constexpr int kSlots = 4;
+    std::mutex mu;
+    int states = 0;
+    std::map<int, StagingSlot[kSlots]> devices;  // (entries stay where they are)
+    static Staging &all() {
+        static Staging *const s = new Staging;  // outlives every state
+        return *s;
+    }
+    void arrive() {
+        std::lock_guard<std::mutex> l(mu);
+        states++;
+    }
+    void leave() {
+        std::lock_guard<std::mutex> l(mu);
+        if (--states == 0) devices.clear();
+    }
+    StagingSlot *slots(int device) {
+        std::lock_guard<std::mutex> l(mu);
+        return devices[device];
+    }
+};
+}  // namespace
+
+int StagingUse::take(size_t want) {
+    int cur = 0;
+    MDX_CUDA_TRY(cudaGetDevice(&cur));
+    if (s.device >= 0 && cur != s.device) {
+        MDX_CUDA_TRY(cudaSetDevice(s.device));
+        back = cur;
+    }
+    StagingSlot *const all = Staging::all().slots(s.device);
+    for (int k = 0; k < Staging::kSlots && !slot; k++)
+        if (all[k].mu.try_lock()) slot = all + k;
+    if (!slot) {
+        if (!s.stage_own) s.stage_own = std::make_shared<StagingSlot>();
+        StagingSlot *const own = static_cast<StagingSlot *>(s.stage_own.get());
+        own->mu.lock();
+        slot = own;
+    }
+    return slot->reserve(want);
+}
+
+StagingUse::~StagingUse() {
+    if (busy) cudaStreamSynchronize(s.stream);  // left early
+    if (slot) slot->mu.unlock();
+    if (back >= 0) cudaSetDevice(back);
+}
+
 State::State() {
     units.setLJ();
+    Staging::all().arrive();
 }
 
 State::~State() {
+    Staging::all().leave();
     if (h_status) cudaFreeHost(h_status);
-    if (stage_h) cudaFreeHost(stage_h);
     for (int k = 0; k < 3; k++) {
         if (side[k]) cudaStreamDestroy(side[k]);
         if (ev_join[k]) cudaEventDestroy(ev_join[k]);
@@ -214,81 +304,159 @@ void host_copy(void *dst, const void *src, size_t bytes) {
 }
 
 namespace {
-// (n,3) FP64 arrays by atom id, rounded to FP32 here (the host cast's
-// round-to-nearest) into the sorted streams, and widened back out; .w is kept
-__global__ void k_put_by_id(int n, const double *__restrict__ in, const int *__restrict__ idToIdx,
+// atoms first, first + 1, ... by id (idToIdx from the first on): rounded to
+// FP32 here (the host cast's round-to-nearest) into the sorted streams, .w
+// kept, and widened back out
+__global__ void k_put_by_id(int m, const double *__restrict__ in, const int *__restrict__ idToIdx,
                             float4 *__restrict__ dst) {
-    int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    const int i = idToIdx[id];
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= m) return;
+    const int i = idToIdx[j];
     const float w = dst[i].w;
-    const double *v = in + 3 * (size_t)id;
+    const double *v = in + 3 * (size_t)j;
     dst[i] = make_float4((float)v[0], (float)v[1], (float)v[2], w);
 }
-__global__ void k_get_by_id(int n, const float4 *__restrict__ src, const uint32_t *__restrict__ ids,
-                            double *__restrict__ out) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 v = src[i];
-    double *o = out + 3 * (size_t)ids[i];
+// streams a, b, c after one another (blockIdx.y)
+__global__ void k_get_by_id(int m, const int *__restrict__ idToIdx, const float4 *__restrict__ a,
+                            const float4 *__restrict__ b, const float4 *__restrict__ c, double *__restrict__ out) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= m) return;
+    const int i = idToIdx[j];
+    const float4 v = blockIdx.y == 0 ? a[i] : (blockIdx.y == 1 ? b[i] : c[i]);
+    double *o = out + 3 * ((size_t)blockIdx.y * m + j);
     o[0] = v.x;
     o[1] = v.y;
     o[2] = v.z;
 }
+
+// runs pieces 0 .. n-1 of a slot: send queues one, read takes it in once it
+// has arrived, with the next one on its way meanwhile
+// (piece p in the slot's half p modulo 2)
+template <class Send, class Read>
+int in_pieces(State &s, StagingSlot &g, int n, Send send, Read read) {
+    for (int p = 0; p <= n; p++) {
+        if (p < n) {
+            const size_t at = (p & 1) * (g.size / 2);
+            const size_t doubles = send(p, g.d + at);
+            MDX_LAUNCHED();
+            MDX_CUDA_TRY(
+                cudaMemcpyAsync(g.h + at, g.d + at, doubles * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
+            MDX_CUDA_TRY(cudaEventRecord(g.done[p & 1], s.stream));
+        }
+        if (p == 0) continue;
+        MDX_CUDA_TRY(cudaEventSynchronize(g.done[(p - 1) & 1]));
+        read(p - 1, g.h + ((p - 1) & 1) * (g.size / 2));
+    }
+    MDX_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
 }  // namespace
 
-int State::stageAlloc() {
-    const size_t need = 9 * (size_t)gpd.n;
-    if (stage_n < need) {
-        if (stage_h) cudaFreeHost(stage_h);
-        stage_h = nullptr;
-        stage_n = 0;
-        MDX_CUDA_TRY(cudaMallocHost(&stage_h, need * sizeof(double)));
-        stage_n = need;
+int StagingUse::put(int k, const double *src) {
+    StagingSlot &g = *slot;
+    const size_t half = g.size / 2;
+    const int n = s.gpd.n, most = (int)(half / 3);
+    busy = true;
+    for (int first = 0; first < n; first += most, pieces++) {
+        const int m = std::min(most, n - first);
+        const size_t bytes = 3 * (size_t)m * sizeof(double);
+        double *const d = g.d + (pieces & 1) * half, *const h = g.h + (pieces & 1) * half;
+        if (pieces >= 2) MDX_CUDA_TRY(cudaEventSynchronize(g.done[pieces & 1]));
+        host_copy(h, src + 3 * (size_t)first, bytes);
+        MDX_CUDA_TRY(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s.stream));
+        k_put_by_id<<<(m + 255) / 256, 256, 0, s.stream>>>(m, d, s.gpd.idToIdx.p + first,
+                                                           k == 0 ? s.gpd.xs.p : s.gpd.vs.p);
+        MDX_LAUNCHED();
+        MDX_CUDA_TRY(cudaEventRecord(g.done[pieces & 1], s.stream));
     }
-    return stage_d.alloc(need);
-}
-
-int State::stagePut(int k, const double *src) {
-    const int n = gpd.n;
-    const size_t bytes = 3 * (size_t)n * sizeof(double);
-    double *const d = stage_d.p + 3 * (size_t)k * n;
-    host_copy(stageHost(k), src, bytes);
-    MDX_CUDA_TRY(cudaMemcpyAsync(d, stageHost(k), bytes, cudaMemcpyHostToDevice, stream));
-    k_put_by_id<<<(n + 255) / 256, 256, 0, stream>>>(n, d, gpd.idToIdx.p, k == 0 ? gpd.xs.p : gpd.vs.p);
-    MDX_LAUNCHED();
     return 0;
 }
 
-int State::stageGet(int k) {
-    const int n = gpd.n;
-    double *const d = stage_d.p + 3 * (size_t)k * n;
-    k_get_by_id<<<(n + 255) / 256, 256, 0, stream>>>(n, k == 0 ? gpd.xs.p : (k == 1 ? gpd.vs.p : gpd.fs.p), gpd.ids.p,
-                                                     d);
-    MDX_LAUNCHED();
-    MDX_CUDA_TRY(cudaMemcpyAsync(stageHost(k), d, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, stream));
+int StagingUse::get(double *const out[3]) {
+    StagingSlot &g = *slot;
+    const GPUData &d = s.gpd;
+    const int n = d.n, most = (int)(g.size / 6), per = (n + most - 1) / most;
+    const float4 *src[3];
+    double *dst[3];
+    int na = 0;
+    for (int k = 0; k < 3; k++) {
+        if (!out[k]) continue;
+        src[na] = k == 0 ? d.xs.p : (k == 1 ? d.vs.p : d.fs.p);
+        dst[na++] = out[k];
+    }
+    busy = true;
+    // array by array, so that each is copied out in long stretches
+    const int e = in_pieces(
+        s, g, na * per,
+        [&](int p, double *buf) {
+            const int first = p % per * most, m = std::min(most, n - first);
+            const float4 *const a = src[p / per];
+            k_get_by_id<<<(m + 255) / 256, 256, 0, s.stream>>>(m, d.idToIdx.p + first, a, a, a, buf);
+            return 3 * (size_t)m;
+        },
+        [&](int p, const double *buf) {
+            const int first = p % per * most, m = std::min(most, n - first);
+            host_copy(dst[p / per] + 3 * (size_t)first, buf, 3 * (size_t)m * sizeof(double));
+        });
+    if (e) return e;
+    if (na) busy = false;  // all that was queued before has completed too
     return 0;
 }
 
-// device -> host atoms, by id
-int State::download() {
+int State::download(double *const *out) {
     if (!uploaded) return 0;
     const int n = gpd.n;
-    if (int e = stageAlloc()) return e;
-    for (int k = 0; k < 3; k++)
-        if (int e = stageGet(k)) return e;
+    StagingUse use(*this);
+    if (int e = use.take(9 * (size_t)n)) return e;
+    use.busy = true;
     MDX_CUDA_TRY(cudaMemcpyAsync(h_status, d_status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, stream));
-    MDX_CUDA_TRY(cudaStreamSynchronize(stream));
+    // all three arrays of some atoms to a piece: a host atom is touched once
+    const size_t size = use.slot->size;
+    const int most = 9 * (size_t)n <= size ? n : (int)(size / 2 / 9);
+    const int e = in_pieces(
+        *this, *use.slot, (n + most - 1) / most,
+        [&](int p, double *buf) {
+            const int first = p * most, m = std::min(most, n - first);
+            k_get_by_id<<<dim3((m + 255) / 256, 3), 256, 0, stream>>>(m, gpd.idToIdx.p + first, gpd.xs.p, gpd.vs.p,
+                                                                      gpd.fs.p, buf);
+            return 9 * (size_t)m;
+        },
+        [&](int p, const double *x) {
+            const int first = p * most, m = std::min(most, n - first);
+            const double *v = x + 3 * (size_t)m, *f = v + 3 * (size_t)m;
+            for (int k = 0; k < 3; k++)
+                if (out && out[k])
+                    host_copy(out[k] + 3 * (size_t)first, x + 3 * (size_t)k * m, 3 * (size_t)m * sizeof(double));
+            for (int i = first; i < first + m; i++, x += 3, v += 3, f += 3) {
+                HostAtom &a = atoms[i];
+                for (int c = 0; c < 3; c++) {
+                    a.pos[c] = x[c];
+                    a.vel[c] = v[c];
+                    a.force[c] = f[c];
+                }
+            }
+        });
+    if (e) return e;
+    use.busy = false;
     turn = h_status->turn;
-    const double *x = stageHost(0), *v = stageHost(1), *f = stageHost(2);
-    for (int i = 0; i < n; i++, x += 3, v += 3, f += 3) {
-        HostAtom &a = atoms[i];
+    return 0;
+}
+
+int State::put(const double *pos, const double *vel) {
+    const int n = gpd.n;
+    StagingUse use(*this);
+    if (int e = use.take(6 * (size_t)n)) return e;
+    if (pos)
+        if (int e = use.put(0, pos)) return e;
+    if (vel)
+        if (int e = use.put(1, vel)) return e;
+    for (int i = 0; i < n; i++)
         for (int d = 0; d < 3; d++) {
-            a.pos[d] = x[d];
-            a.vel[d] = v[d];
-            a.force[d] = f[d];
+            if (pos) atoms[i].pos[d] = pos[3 * (size_t)i + d];
+            if (vel) atoms[i].vel[d] = vel[3 * (size_t)i + d];
         }
-    }
+    MDX_CUDA_TRY(cudaStreamSynchronize(stream));
+    use.busy = false;
     return 0;
 }
 
