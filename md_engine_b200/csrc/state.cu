@@ -9,7 +9,6 @@
 #include <limits>
 #include <map>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -289,14 +288,16 @@ void host_copy(void *dst, const void *src, size_t bytes) {
     }
     const size_t chunk = (bytes / parts + 4095) / 4096 * 4096;
     std::vector<std::thread> th;
-    th.reserve(parts);
     size_t at = chunk;  // the first chunk is this thread's
     try {
+        th.reserve(parts);
         for (; at < bytes; at += chunk)
             th.emplace_back([=] {
                 std::memcpy((char *)dst + at, (const char *)src + at, std::min(chunk, bytes - at));
             });
-    } catch (const std::system_error &) {  // no more threads: the rest here
+    } catch (...) {
+        // no more threads, or no memory for one: the rest here (an exception
+        // that left with threads running would end the process)
         std::memcpy((char *)dst + at, (const char *)src + at, bytes - at);
     }
     std::memcpy(dst, src, std::min(chunk, bytes));
