@@ -123,92 +123,106 @@ __global__ void k_wrap_bin(const GridArgs a0, const GridArgs *__restrict__ tab) 
 }
 
 // exclusive scan of the cell histogram (replaces the host cumulativeSum,
-// helpers.h:15-24); also clears the fill counters.  A block per tile of
-// kScanTile cells: it sums the counts before its tile itself (coalesced
-// 16-byte loads from L2, no block waits for another), then scans its tile --
-// through shared memory, thread t its eight consecutive cells in registers,
-// warp and block totals by shuffles.  One block walking the tiles one after
-// another took 5.6 us a tile: 74 us for the 104,000 cells of 256,000
-// particles, 6 us so; up to one tile nothing changes.
+// helpers.h:15-24); also clears the fill counters.  Tiles of kScanTile cells,
+// a block for each up to kScanBlocks, beyond that a block for as many in a
+// row as share them out: it sums the counts before its tiles itself (coalesced
+// 16-byte loads from L2, no block waits for another), then scans them one
+// after another -- through shared memory, thread t its eight consecutive cells
+// in registers, warp and block totals by shuffles.  One block walking all
+// tiles took 5.6 us a tile: 74 us for the 104,000 cells of 256,000 particles,
+// 6 us so.  With a block to every tile, whatever their number, the counts read
+// again grow with the square of the cells: rebuild of 4,000 atoms in a dilute
+// box of 20 million cells 8.6 ms, 5.5 so (20.7 with one block); of 4 million
+// 1.01, 0.93.
 constexpr int kScanThreads = 1024;
 constexpr int kScanPer = 8;
 constexpr int kScanTile = kScanThreads * kScanPer;
-inline unsigned scan_tiles(int ncell) { return (unsigned)((ncell + kScanTile - 1) / kScanTile); }
+constexpr int kScanBlocks = 128;
+__host__ __device__ inline int scan_tiles(int ncell) { return (ncell + kScanTile - 1) / kScanTile; }
+inline unsigned scan_blocks(int ncell) { return (unsigned)std::min(scan_tiles(ncell), kScanBlocks); }
 __global__ void __launch_bounds__(kScanThreads) k_scan_cells(const GridArgs a0, const GridArgs *__restrict__ tab) {
     MDX_GRID_ARGS;
     if (!A.st->rebuild) return;
     const uint32_t *__restrict__ count = A.cell_count;
     const int ncell = A.ncell;
-    const int base = (int)blockIdx.x * kScanTile;
-    if (base >= ncell) return;
+    const int mine = (scan_tiles(ncell) + kScanBlocks - 1) / kScanBlocks * kScanTile;  // a block's cells
+    if ((long long)blockIdx.x * mine >= ncell) return;
+    const int first = (int)blockIdx.x * mine, end = first + min(mine, ncell - first);
     __shared__ uint4 tile4[kScanTile / 4];
     __shared__ uint32_t warp_tot[32], warp_before[32];
     uint32_t *const tile = reinterpret_cast<uint32_t *>(tile4);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t before = 0u;
+    uint32_t before = 0u;  // this thread's share of the counts before the tile
     {
         const uint4 *c4 = reinterpret_cast<const uint4 *>(count);
 #pragma unroll 4
-        for (int k = threadIdx.x; k < base / 4; k += kScanThreads) {
+        for (int k = threadIdx.x; k < first / 4; k += kScanThreads) {
             const uint4 c = c4[k];
             before += c.x + c.y + c.z + c.w;
         }
     }
+#pragma unroll 1
+    for (int base = first;;) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
-    if (lane == 0) warp_before[w] = before;
-    const int nt = min(kScanTile, ncell - base);
+        for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+        if (lane == 0) warp_before[w] = before;
+        const int nt = min(kScanTile, end - base);
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-        const int c = k * kScanThreads + (int)threadIdx.x;
-        tile[c] = c < nt ? count[base + c] : 0u;
-    }
-    __syncthreads();
-    const uint4 a = tile4[2 * threadIdx.x], b = tile4[2 * threadIdx.x + 1];
-    const uint32_t v[kScanPer] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint32_t run = 0u;
+        for (int k = 0; k < kScanPer; k++) {
+            const int c = k * kScanThreads + (int)threadIdx.x;
+            tile[c] = c < nt ? count[base + c] : 0u;
+        }
+        __syncthreads();
+        const uint4 a = tile4[2 * threadIdx.x], b = tile4[2 * threadIdx.x + 1];
+        const uint32_t v[kScanPer] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        uint32_t run = 0u;
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) run += v[k];
-    uint32_t x = run;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        uint32_t t = warp_tot[lane], bf = warp_before[lane];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) bf += __shfl_xor_sync(0xffffffffu, bf, o);
+        for (int k = 0; k < kScanPer; k++) run += v[k];
+        uint32_t x = run;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += y;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-        warp_tot[lane] = bf + t;  // everything up to and with the warp
-    }
-    __syncthreads();
-    const uint32_t last = warp_tot[w];
-    uint32_t excl = last - __shfl_sync(0xffffffffu, x, 31) + x - run;
-    uint32_t e[kScanPer];
+        if (lane == 31) warp_tot[w] = x;
+        __syncthreads();
+        if (w == 0) {
+            uint32_t t = warp_tot[lane], bf = warp_before[lane];
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-        e[k] = excl;
-        excl += v[k];
-    }
-    tile4[2 * threadIdx.x] = make_uint4(e[0], e[1], e[2], e[3]);
-    tile4[2 * threadIdx.x + 1] = make_uint4(e[4], e[5], e[6], e[7]);
-    __syncthreads();
+            for (int o = 16; o > 0; o >>= 1) bf += __shfl_xor_sync(0xffffffffu, bf, o);
 #pragma unroll
-    for (int k = 0; k < kScanPer; k++) {
-        const int c = k * kScanThreads + (int)threadIdx.x;
-        if (c < nt) {
-            A.cell_start[base + c] = tile[c];
-            A.cell_fill[base + c] = 0u;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+                if (lane >= o) t += y;
+            }
+            warp_tot[lane] = bf + t;  // everything up to and with the warp
         }
+        __syncthreads();
+        const uint32_t last = warp_tot[w];
+        uint32_t excl = last - __shfl_sync(0xffffffffu, x, 31) + x - run;
+        uint32_t e[kScanPer];
+#pragma unroll
+        for (int k = 0; k < kScanPer; k++) {
+            e[k] = excl;
+            excl += v[k];
+        }
+        tile4[2 * threadIdx.x] = make_uint4(e[0], e[1], e[2], e[3]);
+        tile4[2 * threadIdx.x + 1] = make_uint4(e[4], e[5], e[6], e[7]);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kScanPer; k++) {
+            const int c = k * kScanThreads + (int)threadIdx.x;
+            if (c < nt) {
+                A.cell_start[base + c] = tile[c];
+                A.cell_fill[base + c] = 0u;
+            }
+        }
+        if (base + nt == ncell && threadIdx.x == kScanThreads - 1) A.cell_start[ncell] = excl;
+        base += nt;
+        if (base >= end) break;
+        before = threadIdx.x == 0 ? warp_tot[31] : 0u;  // everything up to the tile's end
+        __syncthreads();  // the tile and the totals are written again
     }
-    if (base + nt == ncell && threadIdx.x == kScanThreads - 1) A.cell_start[ncell] = excl;
 }
 
 __global__ void k_scatter(const GridArgs a0, const GridArgs *__restrict__ tab) {
@@ -1229,7 +1243,7 @@ int nlist_rebuild(State &s, bool force, bool conditional, cudaStream_t bstream) 
     const GridArgs *nt = nullptr;
     MDX_CUDA_TRY(launch_pdl(k_check, dim3(nb), dim3(256), 0, s.stream, A, nt, force ? 1 : 0));
     MDX_CUDA_TRY(launch_pdl(k_wrap_bin, dim3(nb), dim3(256), 0, s.stream, A, nt));
-    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_tiles(A.ncell)), dim3(kScanThreads), 0, s.stream, A, nt));
+    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_blocks(A.ncell)), dim3(kScanThreads), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_scatter, dim3(nb), dim3(256), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_gather, dim3(nb), dim3(256), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_copyback, dim3(nb), dim3(256), 0, s.stream, A, nt));
@@ -1288,7 +1302,7 @@ static int nlist_rebuild_mf(State &s, bool force, cudaStream_t bstream) {
     const int nb_mol = (M.nmol + 255) / 256;
     MDX_CUDA_TRY(launch_pdl(k_check, dim3(nb_atoms), dim3(256), 0, s.stream, A, nt, force ? 1 : 0));
     MDX_CUDA_TRY(launch_pdl(k_mf_wrap_bin, dim3(nb_mol), dim3(256), 0, s.stream, M, mnt));
-    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_tiles(Am.ncell)), dim3(kScanThreads), 0, s.stream, Am, nt));
+    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_blocks(Am.ncell)), dim3(kScanThreads), 0, s.stream, Am, nt));
     MDX_CUDA_TRY(launch_pdl(k_mf_scatter, dim3(nb_mol), dim3(256), 0, s.stream, M, mnt));
     MDX_CUDA_TRY(launch_pdl(k_mf_gather, dim3((4 * M.nmol + 255) / 256), dim3(256), 0, s.stream, M, mnt));
     MDX_CUDA_TRY(launch_pdl(k_mf_copyback, dim3((4 * M.nmol + 255) / 256), dim3(256), 0, s.stream, M, mnt));
@@ -1325,7 +1339,7 @@ int nlist_build_atoms_view(State &s) {
     const GridArgs *nt = nullptr;
     MDX_CUDA_TRY(launch_pdl(k_check, dim3(nb), dim3(256), 0, s.stream, A, nt, 1));
     MDX_CUDA_TRY(launch_pdl(k_wrap_bin, dim3(nb), dim3(256), 0, s.stream, A, nt));
-    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_tiles(A.ncell)), dim3(kScanThreads), 0, s.stream, A, nt));
+    MDX_CUDA_TRY(launch_pdl(k_scan_cells, dim3(scan_blocks(A.ncell)), dim3(kScanThreads), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_scatter, dim3(nb), dim3(256), 0, s.stream, A, nt));
     MDX_CUDA_TRY(launch_pdl(k_gather, dim3(nb), dim3(256), 0, s.stream, A, nt));
     if (gr.cap == 0) {
@@ -1602,7 +1616,7 @@ static void batch_rebuild_sites(Batch &b, cudaStream_t st) {
     B.ncell = b.max_cell_ps;
     const dim3 nb((b.max_n_ps + 255) / 256, P);
     k_wrap_bin<<<nb, 256, 0, st>>>(A, tg);
-    k_scan_cells<<<dim3(scan_tiles(A.ncell), P), kScanThreads, 0, st>>>(A, tg);
+    k_scan_cells<<<dim3(scan_blocks(A.ncell), P), kScanThreads, 0, st>>>(A, tg);
     k_scatter<<<nb, 256, 0, st>>>(A, tg);
     k_gather<<<nb, 256, 0, st>>>(A, tg);
     k_copyback<<<nb, 256, 0, st>>>(A, tg);
@@ -1626,7 +1640,7 @@ static void batch_rebuild_mols(Batch &b, cudaStream_t st) {
     M.ncell = b.max_mcell;
     const int nb_mol = (b.max_mol_mf + 255) / 256, nb_site = (4 * b.max_mol_mf + 255) / 256;
     k_mf_wrap_bin<<<dim3(nb_mol, Q), 256, 0, st>>>(M, tm);
-    k_scan_cells<<<dim3(scan_tiles(Am.ncell), Q), kScanThreads, 0, st>>>(Am, ts);
+    k_scan_cells<<<dim3(scan_blocks(Am.ncell), Q), kScanThreads, 0, st>>>(Am, ts);
     k_mf_scatter<<<dim3(nb_mol, Q), 256, 0, st>>>(M, tm);
     k_mf_gather<<<dim3(nb_site, Q), 256, 0, st>>>(M, tm);
     k_mf_copyback<<<dim3(nb_site, Q), 256, 0, st>>>(M, tm);

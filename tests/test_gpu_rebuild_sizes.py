@@ -43,6 +43,34 @@ def test_list_across_scan_tiles(oracle, side):
         assert np.array_equal(np.sort(nb[i, :c[i]]), np.sort(no[i, :co[i]]))
 
 
+# 126 tiles (a block for each), 130 (two to a block), 256 (two to each of the
+# most blocks): a dilute box of few small clumps
+@pytest.mark.parametrize("side", [101, 102, 128])
+def test_list_of_a_large_dilute_box(oracle, side):
+    rng = np.random.default_rng(side)
+    rcut, skin, L = 1.5, 0.2, side * 1.7 * 1.0001
+    pos = (rng.uniform(0, L, (500, 1, 3)) + rng.uniform(-1.5, 1.5, (500, 6, 3))).reshape(-1, 3) % L
+    n = len(pos)
+    st = State()
+    st.units.setLJ()
+    st.bounds = Bounds(st, lo=Vector(0, 0, 0), hi=Vector(L, L, L))
+    st.rCut, st.padding, st.dt = rcut, skin, 0.001
+    st.atomParams.addSpecies("A", 1.0, 1)
+    st.addAtoms(["A"] * n, pos, np.zeros(n))
+    lj = FixLJCut(st, "none")
+    lj.setParameter("sig", "A", "A", 0.1)
+    lj.setParameter("eps", "A", "A", 0.0)
+    st.activateFix(lj)
+    st.prepare()
+    assert int(st.cellsPerSide) == side
+    x = st.getAtoms()[0].astype(np.float32)
+    c, nb, _ = st.getNeighborList()
+    co, no = oracle_nlist_for(oracle, x, np.zeros(3), np.full(3, L), neighbor_cut(rcut, skin), ids=np.arange(n))[:2]
+    assert np.array_equal(c, co)
+    for i in range(n):
+        assert np.array_equal(np.sort(nb[i, :c[i]]), np.sort(no[i, :co[i]]))
+
+
 @pytest.mark.parametrize("n", [1000, 3000, 7000, 15000, 20000])
 def test_forces_at_each_team_size(oracle, n):
     L = (n / 0.8) ** (1 / 3)
