@@ -388,6 +388,8 @@ struct E3BSurrogate {
     DBuf<float> xf;  // host rows before their rounding to BF16
     DBuf<float> yb;
     DBuf<double> loss;
+    DBuf<float> part;        // each block's gradient
+    DBuf<double> part_loss;  // and sum of squared errors
     int batch = 0;
 };
 

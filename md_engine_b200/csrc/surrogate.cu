@@ -243,8 +243,7 @@ __device__ __forceinline__ float dsilu(float z) {
 // that the eight rows of an ldmatrix fall on distinct banks), weights included;
 // pre-activations and the weight-gradient accumulators stay in registers (the
 // warp that computes a 16 x 32 piece of a layer's output computes the same
-// piece of its gradient), and a block adds its gradient to the global one
-// once.  As a chain of 25 GEMM, element-wise and column-sum launches that
+// piece of its gradient), and a block writes its gradient out once.  As a chain of 25 GEMM, element-wise and column-sum launches that
 // passed every activation through global memory, and summed the bias
 // gradients with one thread per column, a call with 4,096 rows of host arrays
 // took 789 us; it takes 248 us so, copies included.
@@ -258,6 +257,7 @@ struct TrainShared {
     __nv_bfloat16 act[3][kTileRows * kPitchH];
     __nv_bfloat16 dz4[kTileRows * kPitchO], dz[2][kTileRows * kPitchH];
     float bias[3 * S::kHid + S::kOut];
+    float db[kTileRows / 16][3 * S::kHid + S::kOut];  // bias gradients by row of warps
     double loss[kTrainThreads / 32];
 };
 
@@ -358,17 +358,15 @@ __device__ __forceinline__ void train_backward(const float (&z)[4][4], const __n
     }
 }
 
-// a 16 x 8 piece of a weight gradient onto the global one
-__device__ __forceinline__ void add_piece(float *g, int ld, int i0, int n0, const float (&acc)[4], int lane) {
+// a 16 x 8 piece of a weight gradient into the block's own
+__device__ __forceinline__ void put_piece(float *g, int ld, int i0, int n0, const float (&acc)[4], int lane) {
     float *p = g + (size_t)(i0 + (lane >> 2)) * ld + n0 + 2 * (lane & 3);
-    atomicAdd(p, acc[0]);
-    atomicAdd(p + 1, acc[1]);
-    atomicAdd(p + 8 * ld, acc[2]);
-    atomicAdd(p + 8 * ld + 1, acc[3]);
+    *reinterpret_cast<float2 *>(p) = make_float2(acc[0], acc[1]);
+    *reinterpret_cast<float2 *>(p + 8 * ld) = make_float2(acc[2], acc[3]);
 }
 // column sums held by the four lanes of each column pair, over the warp's rows
 template <int NT>
-__device__ __forceinline__ void add_bias(float *g, int n0, const float (&db)[NT][2], int lane) {
+__device__ __forceinline__ void put_bias(float *b, int n0, const float (&db)[NT][2], int lane) {
 #pragma unroll
     for (int j = 0; j < NT; j++)
 #pragma unroll
@@ -376,17 +374,19 @@ __device__ __forceinline__ void add_bias(float *g, int n0, const float (&db)[NT]
             float v = db[j][c];
 #pragma unroll
             for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane < 4) atomicAdd(g + n0 + 8 * j + 2 * lane + c, v);
+            if (lane < 4) b[n0 + 8 * j + 2 * lane + c] = v;
         }
 }
 
 // B rows (a multiple of 64) of standardised BF16 features x and targets t:
-// the gradient added to grad, the sum of squared errors to loss
+// each block's gradient into its row of part, its sum of squared errors into
+// part_loss (added up by k_sum_grad in a fixed order: with float atomics onto one
+// gradient it would not repeat bit for bit)
 __global__ void __launch_bounds__(kTrainThreads) k_fwd_bwd(int B, const __nv_bfloat16 *__restrict__ x,
                                                            const float *__restrict__ t,
                                                            const __nv_bfloat16 *__restrict__ wb,
-                                                           const float *__restrict__ wf, float *__restrict__ grad,
-                                                           double *__restrict__ loss) {
+                                                           const float *__restrict__ wf, float *__restrict__ part,
+                                                           double *__restrict__ part_loss) {
     extern __shared__ __align__(16) char train_smem[];
     TrainShared &sh = *reinterpret_cast<TrainShared *>(train_smem);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -460,26 +460,59 @@ __global__ void __launch_bounds__(kTrainThreads) k_fwd_bwd(int B, const __nv_bfl
         for (int h = 0; h < 2; h++)
             tile_mma<kTileRows, 4, true, false>(g1[h], sh.x, kPitchX, i0 + 64 * h, sh.dz[0], kPitchH, n0, lane);
     }
+    float *const grad = part + (size_t)blockIdx.x * S::kParams;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        add_piece(grad + S::kOffW1, S::kHid, i0, n0 + 8 * j, g1[0][j], lane);
-        add_piece(grad + S::kOffW1, S::kHid, i0 + 64, n0 + 8 * j, g1[1][j], lane);
-        add_piece(grad + S::kOffW2, S::kHid, i0, n0 + 8 * j, g2[j], lane);
-        add_piece(grad + S::kOffW3, S::kHid, i0, n0 + 8 * j, g3[j], lane);
+        put_piece(grad + S::kOffW1, S::kHid, i0, n0 + 8 * j, g1[0][j], lane);
+        put_piece(grad + S::kOffW1, S::kHid, i0 + 64, n0 + 8 * j, g1[1][j], lane);
+        put_piece(grad + S::kOffW2, S::kHid, i0, n0 + 8 * j, g2[j], lane);
+        put_piece(grad + S::kOffW3, S::kHid, i0, n0 + 8 * j, g3[j], lane);
     }
-    add_piece(grad + S::kOffW4, S::kOut, i0, 8 * wc, g4[0], lane);
-    add_bias(grad + S::kOffB1, n0, b1, lane);
-    add_bias(grad + S::kOffB2, n0, b2, lane);
-    add_bias(grad + S::kOffB3, n0, b3, lane);
-    add_bias(grad + S::kOffB4, 8 * wc, b4, lane);
+    put_piece(grad + S::kOffW4, S::kOut, i0, 8 * wc, g4[0], lane);
+    put_bias(sh.db[wr], n0, b1, lane);
+    put_bias(sh.db[wr] + S::kHid, n0, b2, lane);
+    put_bias(sh.db[wr] + 2 * S::kHid, n0, b3, lane);
+    put_bias(sh.db[wr] + 3 * S::kHid, 8 * wc, b4, lane);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
     if (lane == 0) sh.loss[w] = lsum;
     __syncthreads();
+    for (int i = tid; i < 3 * S::kHid + S::kOut; i += kTrainThreads) {
+        const int l = i / S::kHid;
+        grad[(l == 0 ? S::kOffB1 : (l == 1 ? S::kOffB2 : (l == 2 ? S::kOffB3 : S::kOffB4))) + i - l * S::kHid] =
+            (sh.db[0][i] + sh.db[1][i]) + (sh.db[2][i] + sh.db[3][i]);
+    }
     if (tid == 0) {
         double l = 0.0;
         for (int k = 0; k < kTrainThreads / 32; k++) l += sh.loss[k];
-        atomicAdd(loss, l);
+        part_loss[blockIdx.x] = l;
+    }
+}
+
+// the blocks' gradients and losses added up in a fixed order: four threads to
+// a parameter, each a stretch of the rows (64 rows of 70 KB at 4,096 rows of a
+// batch, read from L2)
+constexpr int kSumCols = 64;
+__global__ void __launch_bounds__(4 * kSumCols) k_sum_grad(int rows, const float *__restrict__ part,
+                                                           const double *__restrict__ part_loss,
+                                                           float *__restrict__ grad, double *__restrict__ loss) {
+    __shared__ float sh[4][kSumCols];
+    const int col = threadIdx.x % kSumCols, seg = threadIdx.x / kSumCols;
+    const int i = blockIdx.x * kSumCols + col;
+    const int per = (rows + 3) / 4, end = min(rows, (seg + 1) * per);
+    float s = 0.f;
+    if (i < S::kParams)
+#pragma unroll 8
+        for (int r = seg * per; r < end; r++) s += part[(size_t)r * S::kParams + i];
+    sh[seg][col] = s;
+    __syncthreads();
+    if (seg == 0 && i < S::kParams) grad[i] = (sh[0][col] + sh[1][col]) + (sh[2][col] + sh[3][col]);
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        double l = 0.0;
+        for (int r = threadIdx.x; r < rows; r += 32) l += part_loss[r];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+        if (threadIdx.x == 0) *loss = l;
     }
 }
 
@@ -758,17 +791,20 @@ InferArgs infer_args(FixE3B &f, int nmol, float4 *out, int add_o) {
 unsigned infer_blocks(int n) { return (unsigned)((pad16(n) / 16 + kInferWarps - 1) / kInferWarps); }
 
 // forward + backward of one minibatch already in u.xb / u.yb (B rows);
-// gradient into u.grad (zeroed here), loss sum into u.loss
+// gradient into u.grad, loss sum into u.loss
+int sur_blocks(int B) { return std::min(B / kTileRows, num_sms()); }
 int sur_fwd_bwd(S &u, int B, cudaStream_t st) {
     if (B % kTileRows) {
         set_error(MDX_ERR_ARG, "surrogate batch of %d rows not tiled by %d", B, kTileRows);
         return MDX_ERR_ARG;
     }
-    MDX_CUDA_TRY(cudaMemsetAsync(u.grad.p, 0, S::kParams * sizeof(float), st));
-    MDX_CUDA_TRY(cudaMemsetAsync(u.loss.p, 0, sizeof(double), st));
     MDX_CUDA_TRY(cudaFuncSetAttribute(k_fwd_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainShared)));
-    k_fwd_bwd<<<std::min(B / kTileRows, num_sms()), kTrainThreads, sizeof(TrainShared), st>>>(B, u.xb.p, u.yb.p, u.wb.p,
-                                                                                              u.w.p, u.grad.p, u.loss.p);
+    const int nb = sur_blocks(B);
+    k_fwd_bwd<<<nb, kTrainThreads, sizeof(TrainShared), st>>>(B, u.xb.p, u.yb.p, u.wb.p, u.w.p, u.part.p,
+                                                              u.part_loss.p);
+    MDX_LAUNCHED();
+    k_sum_grad<<<(S::kParams + kSumCols - 1) / kSumCols, 4 * kSumCols, 0, st>>>(nb, u.part.p, u.part_loss.p, u.grad.p,
+                                                                               u.loss.p);
     MDX_LAUNCHED();
     MDX_CUDA_TRY(cudaGetLastError());
     return 0;
@@ -778,6 +814,8 @@ int sur_batch_alloc(S &u, int B) {
     if (u.batch >= B) return 0;
     if (int e = u.xb.alloc((size_t)B * S::kIn)) return e;
     if (int e = u.yb.alloc((size_t)B * S::kOut)) return e;
+    if (int e = u.part.alloc((size_t)sur_blocks(B) * S::kParams)) return e;
+    if (int e = u.part_loss.alloc(sur_blocks(B))) return e;
     u.batch = B;
     return 0;
 }

@@ -9,8 +9,7 @@ from oracle import surrogate_ref as SR
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [64, 128, 64 * 301])
-def test_gradient_by_tiles(rows):
+def _surrogate(rows):
     sysd = systems.water_tip4p2005(nside=6, seed=5)
     st, fx = systems.build_water_state(sysd, rcut=6.5, skin=1.0, grid=32, e3b=True)
     st.prepare()
@@ -23,6 +22,12 @@ def test_gradient_by_tiles(rows):
     e3.surrogateSetParams(w, np.zeros(SR.N_IN), np.ones(SR.N_IN), 1.0)
     x = rng.standard_normal((rows, SR.N_IN)).astype(np.float32)
     t = rng.standard_normal((rows, SR.N_OUT)).astype(np.float32)
+    return st, e3, w, x, t
+
+
+@pytest.mark.parametrize("rows", [64, 128, 64 * 301])
+def test_gradient_by_tiles(rows):
+    st, e3, w, x, t = _surrogate(rows)
     loss, g = e3.surrogateGrad(x, t)
     lr, gr = SR.mlp_loss_grad(w, x, t)
     assert loss == pytest.approx(lr, rel=1e-2)
@@ -31,3 +36,13 @@ def test_gradient_by_tiles(rows):
     for k, (o, s) in SR.OFF.items():
         rk = np.linalg.norm(g[o:o + s] - gr[o:o + s]) / np.linalg.norm(gr[o:o + s])
         assert rk < 2e-2, (k, rk)
+
+
+# three and seven tiles, a tile to each of 64 blocks, two and three to each of 148
+@pytest.mark.parametrize("rows", [192, 448, 4096, 64 * 301])
+def test_gradient_repeats_bit_for_bit(rows):
+    st, e3, _, x, t = _surrogate(rows)
+    loss, g = e3.surrogateGrad(x, t)
+    for _ in range(5):
+        loss2, g2 = e3.surrogateGrad(x, t)
+        assert loss2 == loss and np.array_equal(g2, g)
