@@ -385,10 +385,10 @@ struct E3BSurrogate {
     DBuf<float4> fexact;
     // training scratch
     DBuf<__nv_bfloat16> xb;
-    DBuf<float> xf;  // host rows before their rounding to BF16
+    DBuf<float> xf;  // host rows for inference before their rounding to BF16
     DBuf<float> yb;
     DBuf<double> loss;
-    DBuf<float> part;        // each block's gradient
+    DBuf<float> part;        // the batch's host rows before their rounding, then each block's gradient
     DBuf<double> part_loss;  // and sum of squared errors
     int batch = 0;
 };

@@ -814,7 +814,7 @@ int sur_batch_alloc(S &u, int B) {
     if (u.batch >= B) return 0;
     if (int e = u.xb.alloc((size_t)B * S::kIn)) return e;
     if (int e = u.yb.alloc((size_t)B * S::kOut)) return e;
-    if (int e = u.part.alloc((size_t)sur_blocks(B) * S::kParams)) return e;
+    if (int e = u.part.alloc(std::max((size_t)sur_blocks(B) * S::kParams, (size_t)B * S::kIn))) return e;
     if (int e = u.part_loss.alloc(sur_blocks(B))) return e;
     u.batch = B;
     return 0;
@@ -1163,9 +1163,8 @@ int mdx_e3b_surrogate_grad(mdx_state *st, mdx_fix *fix, const float *x, const fl
     S &u = *f->sur;
     if (int e = sur_batch_alloc(u, n)) return e;
     // rounded to BF16 on the device
-    if (int e = u.xf.alloc((size_t)n * S::kIn)) return e;
-    MDX_CUDA_TRY(cudaMemcpyAsync(u.xf.p, x, (size_t)n * S::kIn * sizeof(float), cudaMemcpyHostToDevice, s.stream));
-    k_to_bf16<<<(unsigned)(((size_t)n * S::kIn + 255) / 256), 256, 0, s.stream>>>((size_t)n * S::kIn, u.xf.p, u.xb.p);
+    MDX_CUDA_TRY(cudaMemcpyAsync(u.part.p, x, (size_t)n * S::kIn * sizeof(float), cudaMemcpyHostToDevice, s.stream));
+    k_to_bf16<<<(unsigned)(((size_t)n * S::kIn + 255) / 256), 256, 0, s.stream>>>((size_t)n * S::kIn, u.part.p, u.xb.p);
     MDX_LAUNCHED();
     MDX_CUDA_TRY(cudaMemcpyAsync(u.yb.p, t, (size_t)n * S::kOut * sizeof(float), cudaMemcpyHostToDevice, s.stream));
     if (int e = sur_fwd_bwd(u, n, s.stream)) return e;
