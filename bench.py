@@ -623,7 +623,7 @@ def main():
                            start=f"equilibrated: {args.eq_steps} steps, tight Nose-Hoover, before warm-up",
                            parallelism="replicas only" if world > 1 else "single system",
                            pair_grid_autotuned={"blocks_per_sm": tuned_cap, "ms_per_force_phase": tuned_ms}
-                           if tuned_cap else "per-site form: no grid shape tuned"),
+                           if tuned_ms else "per-site form: no grid shape tuned"),
             "ns_per_day": ns_day,
             "temperature_end_of_timed_region": t_end,
             "e2e": {"value": e2e, "unit": "timesteps/s",

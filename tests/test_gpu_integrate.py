@@ -262,3 +262,12 @@ def test_autotune_keeps_the_state_and_the_trajectory():
     lj = systems.lj_fcc(ncell=6, seed=3)
     st, _ = systems.build_lj_state(lj, rcut=2.5, skin=0.3)
     assert IntegratorVerlet(st).autotune(reps=2) == (0, 0.0)
+
+
+def test_autotune_can_keep_the_automatic_grid():
+    import inspect
+    from md_engine_b200 import IntegratorVerlet
+    assert 0 in inspect.signature(IntegratorVerlet.autotune).parameters["caps"].default
+    st, _ = systems.build_water_state(systems.water_tip4p2005(nside=10, seed=5), rcut=9.0, skin=1.0, grid=32)
+    cap, ms = IntegratorVerlet(st).autotune(reps=2, caps=(0,))
+    assert cap == 0 and ms > 0 and int(st.pairBlocksPerSM) == 0
