@@ -362,7 +362,7 @@ class IntegratorVerlet {
             if (int e = s->prepare()) return e;
         }
         StagingUse use(*s);
-        if (int e = use.take(6 * (size_t)s->gpd.n)) return e;
+        if (int e = use.take(9 * (size_t)s->gpd.n)) return e;
         // the step graphs of this call exist before any copy is queued
         if (int e = precapture(nturns, 0)) return e;
         // inputs: a plain copy into pinned memory, one async copy each, the

@@ -52,17 +52,16 @@ int num_sms() {
 }
 
 // Host arrays cross in pieces through pinned and device memory that all states
-// of a device share: kStageMost doubles at most, for two pieces under way (or
-// one that is all there is), in kSlots slots of which a call takes a free one
-// (a state takes one of its own when there is none), given back with the
-// process's last state.
+// of a device share: kStageMost doubles at most, in kSlots slots of which a
+// call takes a free one (a state takes one of its own when there is none),
+// given back with the process's last state.
 // Pinned memory for each state, 72 bytes an atom taken by its first getAtoms,
 // made the first pass of 64 new replicas 50 ms; it takes 34 so.
 constexpr size_t kStageMost = size_t(1) << 21;
 struct StagingSlot {
     std::mutex mu;
     double *h = nullptr, *d = nullptr;
-    cudaEvent_t done[2] = {nullptr, nullptr};  // of the two pieces under way
+    cudaEvent_t done[3] = {nullptr, nullptr, nullptr};  // of the pieces under way
     size_t size = 0;  // doubles
     int reserve(size_t want) {
         for (cudaEvent_t &e : done)
@@ -330,23 +329,24 @@ __global__ void k_get_by_id(int m, const int *__restrict__ idToIdx, const float4
     o[2] = v.z;
 }
 
-// runs pieces 0 .. n-1 of a slot: send queues one, read takes it in once it
-// has arrived, with the next one on its way meanwhile
-// (piece p in the slot's half p modulo 2)
+// runs pieces 0 .. n-1 through a slot, up to `ways` of them under way: send
+// queues one, read takes it in once it has arrived
 template <class Send, class Read>
-int in_pieces(State &s, StagingSlot &g, int n, Send send, Read read) {
-    for (int p = 0; p <= n; p++) {
+int in_pieces(State &s, StagingSlot &g, int n, int ways, Send send, Read read) {
+    const size_t part = g.size / ways;
+    for (int p = 0; p < n + ways - 1; p++) {
         if (p < n) {
-            const size_t at = (p & 1) * (g.size / 2);
+            const size_t at = p % ways * part;
             const size_t doubles = send(p, g.d + at);
             MDX_LAUNCHED();
             MDX_CUDA_TRY(
                 cudaMemcpyAsync(g.h + at, g.d + at, doubles * sizeof(double), cudaMemcpyDeviceToHost, s.stream));
-            MDX_CUDA_TRY(cudaEventRecord(g.done[p & 1], s.stream));
+            MDX_CUDA_TRY(cudaEventRecord(g.done[p % ways], s.stream));
         }
-        if (p == 0) continue;
-        MDX_CUDA_TRY(cudaEventSynchronize(g.done[(p - 1) & 1]));
-        read(p - 1, g.h + ((p - 1) & 1) * (g.size / 2));
+        const int q = p - (ways - 1);
+        if (q < 0 || q >= n) continue;
+        MDX_CUDA_TRY(cudaEventSynchronize(g.done[q % ways]));
+        read(q, g.h + q % ways * part);
     }
     MDX_CUDA_TRY(cudaGetLastError());
     return 0;
@@ -376,7 +376,9 @@ int StagingUse::put(int k, const double *src) {
 int StagingUse::get(double *const out[3]) {
     StagingSlot &g = *slot;
     const GPUData &d = s.gpd;
-    const int n = d.n, most = (int)(g.size / 6), per = (n + most - 1) / most;
+    // all three arrays on their way at once, or pieces two at a time
+    const int n = d.n, ways = 9 * (size_t)n <= g.size ? 3 : 2;
+    const int most = (int)(g.size / ways / 3), per = (n + most - 1) / most;
     const float4 *src[3];
     double *dst[3];
     int na = 0;
@@ -388,7 +390,7 @@ int StagingUse::get(double *const out[3]) {
     busy = true;
     // array by array, so that each is copied out in long stretches
     const int e = in_pieces(
-        s, g, na * per,
+        s, g, na * per, ways,
         [&](int p, double *buf) {
             const int first = p % per * most, m = std::min(most, n - first);
             const float4 *const a = src[p / per];
@@ -413,9 +415,9 @@ int State::download(double *const *out) {
     MDX_CUDA_TRY(cudaMemcpyAsync(h_status, d_status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, stream));
     // all three arrays of some atoms to a piece: a host atom is touched once
     const size_t size = use.slot->size;
-    const int most = 9 * (size_t)n <= size ? n : (int)(size / 2 / 9);
+    const int ways = 9 * (size_t)n <= size ? 1 : 2, most = (int)(size / ways / 9);
     const int e = in_pieces(
-        *this, *use.slot, (n + most - 1) / most,
+        *this, *use.slot, (n + most - 1) / most, ways,
         [&](int p, double *buf) {
             const int first = p * most, m = std::min(most, n - first);
             k_get_by_id<<<dim3((m + 255) / 256, 3), 256, 0, stream>>>(m, gpd.idToIdx.p + first, gpd.xs.p, gpd.vs.p,
