@@ -61,7 +61,8 @@ __host__ __device__ __forceinline__ double chain_inv_mass(const NHRegs &c, int k
 template <int N, bool SMALL>
 __host__ __device__ __forceinline__ double nh_ex(double x, double &most) {
     if (!SMALL) return exp(x);
-    most = fabs(x) <= most ? most : fabs(x);  // a NaN is kept
+    // (a NaN here is in the chain itself, and stays in what it returns)
+    most = fabs(x) <= most ? most : fabs(x);
     return nh_exp_small(x);
 }
 constexpr double kNHSmall = 0.015625;
@@ -312,7 +313,10 @@ __global__ void k_rigid_maps(const MolArgs a0, const MolArgs *__restrict__ tab, 
 // early: the kernel before this one in the stream is k_step_end, behind whose
 // trigger every earlier kernel has completed and which writes no stream, so
 // the loads go ahead of its end; the first step after a rebuild group, or of
-// a captured chunk, waits first.
+// a captured chunk, waits first.  In a system of rigid molecules and free
+// atoms k_first_mol follows k_first_atoms, whose threads of rigid members
+// return without waiting: its grid still ends only after k_step_end, for a
+// free atom, of which there is one (has_free_atoms), has waited.
 // per-atom: NH rescale (rescale_no_tags_cu) + nve_v + nve_x (+ zero force)
 template <bool NH>
 __global__ void k_first_atoms(int n, float4 *__restrict__ xs, float4 *__restrict__ vs, float4 *__restrict__ fs,

@@ -1166,10 +1166,13 @@ int nlist_init(State &s) {
     gr.m = m;
     gr.ns = ns;
     int ncell = ns.x * ns.y * ns.z;
-    // list build: home atoms tested two at a time, also where cells hold more:
-    // four at a time water (split rows, exclusions) is slower at six atoms in a
-    // cell, 160 us a build against 117, and at 32, 184 against 162; LJ atoms
-    // 18 in a cell 42 against 46 (4,000), 77 against 74 (32,000)
+    // list build: home atoms tested two at a time, also where cells hold more.
+    // Water (split rows, exclusions) is slower four at a time: 160 us a build
+    // against 117 at six atoms in a cell, 184 against 162 at 32.  Where the
+    // grid chosen above puts four to sixteen LJ atoms in a cell it makes
+    // little difference, two against four at density 0.2: 28.1, 28.1 us (4,000
+    // atoms), 54.7, 54.7 (32,000), 242, 248 (256,000); at 0.4: 36.3, 36.2;
+    // 64.9, 69.0; 267, 261
     if (s.gridHomeGroup != 0 && s.gridHomeGroup != 2 && s.gridHomeGroup != 4) {
         set_error(MDX_ERR_ARG, "gridHomeGroup must be 0 (automatic), 2 or 4 (got %d)", s.gridHomeGroup);
         return MDX_ERR_ARG;
@@ -1196,10 +1199,12 @@ int nlist_init(State &s) {
         // a small system leaves lanes idle and waits for each row's chain of
         // gathers: wider teams while they fit the SMs, fewer beside a P3M
         // chain.  Measured on B200, us per step at team 4, 8, 16, 32 -- LJ
-        // fluid 1,500: 17.2 13.9 12.7 11.8; 4,000: 19.0 16.1 14.9 15.3; 8,000:
-        // 19.9 16.8 16.9 17.7; 16,000: 21.9 19.9 21.5 23.6; 32,000: 26.9 27.7
-        // 30.0; salt with P3M 2,000: 28.8 26.6 26.6 26.5; 8,000: 38.7 35.2
-        // 38.0 40.6; 24,000: 65.6 69.4 70.7
+        // fluid (NVE) 1,500: 9.4 7.0 5.9 5.3; 4,000: 9.8 7.4 6.6 6.8; 6,000:
+        // 10.2 7.8 7.2 8.2; 8,000: 10.3 8.0 8.0 9.2; 16,000: 13.2 11.7 12.9
+        // 15.8; 32,000: 15.6 16.2 18.0 24.1; salt with P3M, before the steps
+        // were joined, 2,000: 28.8 26.6 26.6 26.5; 8,000: 38.7 35.2 38.0 40.6;
+        // 24,000: 65.6 69.4 70.7.  The rule takes the best of these but at
+        // 4,000 (32 lanes, 3 % over 16)
         const double lanes = (s.ewaldFix() ? 640.0 : 880.0) * num_sms();
         while (gr.team < 32 && gr.team < nbar && 2.0 * gr.team * n <= lanes) gr.team *= 2;
     }

@@ -120,12 +120,14 @@ PairArgs make_args(State &s, FixPair &f) {
 //    cutoff is within L/2 under it, so it is the pair's minimum image) and
 //    the cutoffs applied as masks, not branches: all lanes run one path.
 // The molecule's own site pairs (the excluded pairs of the reference's list,
-// multiplier by exclusion depth) are added by lanes 0..15, a pair each.  Forces on the four
-// sites are reduced by shuffles and written by lanes 0..3 (one 64-byte store).
+// multiplier by exclusion depth) are added by lanes 0..15, a pair each.  Forces
+// on the four sites are reduced by halving exchanges and written by lanes 0, 8,
+// 16 and 24, a site each (64 bytes in a row).
 // blocks per SM the kernel is compiled for: 80 registers, which lets the nine
 // charge pairs of a molecule pair be in flight beside one another.  Alone at
-// 4,096 / 32,768 molecules, own pairs still on one lane: 22.6 / 137 us (14 blocks, 72 registers: 24.2 / 144;
-// 10 blocks, 94: 22.5 / 136; 8 blocks, 106: 23.5 / 188)
+// 4,096 / 32,768 molecules, own pairs still on one lane: 22.6 / 137 us
+// (14 blocks, 72 registers: 24.2 / 144; 10 blocks, 94: 22.5 / 136; 8 blocks,
+// 106: 23.5 / 188)
 constexpr int kMolPairBlock = 64;
 constexpr int kMolPairBlocksPerSM = 12;
 constexpr int kMolQueue = 64;  // queued entries per warp (two chunks)
@@ -560,10 +562,13 @@ int pair_mol_launch(State &s, FixPair &f, int virialMode, bool accumulate, float
     // kernel must leave SM slots for that chain's blocks, and a warp that
     // takes one molecule more than another is a tail: the grid is cut to the
     // fewest rounds the SMs' capacity allows and then to the fewest blocks
-    // that need no more rounds.  Measured on B200, water step at 4,096
-    // molecules (two rounds, 7 blocks per SM): 50.4 us; 8, 10, 12 blocks per
-    // SM 50.3, 52.4, 57.3; with E3B 60.9; 61.0, 62.6, 64.8; at 32,768 (ten
-    // rounds, 11 blocks) 279; 8, 10, 12: 293, 276, 274.
+    // that need no more rounds.  Measured on B200, us per water step so and
+    // with 6, 8, 10, 12 blocks per SM and uncapped -- 1,000 molecules: 29.9;
+    // 29.9 30.0 29.9 30.0 31.3; 4,096: 51.9; 50.7 50.9 52.5 57.6 58.9; 8,192:
+    // 74.8; 79.3 75.3 76.3 82.8 82.8; 16,384: 131; 137 128 127 133 133; 32,768:
+    // 279; 325 292 276 273 275; with E3B, 4,096 molecules: 60.9; 8, 10, 12:
+    // 61.0, 62.6, 64.8.  So it is the best with E3B, within 4 % of the best
+    // otherwise (a cap of 10 is too), and the autotuner times both.
     // Else, and for pairBlocksPerSM -1, a warp per molecule
     int mb = 0;
     if (s.pairBlocksPerSM > 0) {
