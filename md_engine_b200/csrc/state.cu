@@ -58,6 +58,10 @@ int num_sms() {
 // Pinned memory for each state, 72 bytes an atom taken by its first getAtoms,
 // made the first pass of 64 new replicas 50 ms; it takes 34 so.
 constexpr size_t kStageMost = size_t(1) << 21;
+// a call that a program may make but once asks for no more than this, 1.5 MB:
+// above 2 MB pinned and device memory take milliseconds to get (first getAtoms
+// of a process's only state, 32,000 atoms: 0.9 ms so, 2.5 with 2.3 MB)
+constexpr size_t kStageOnce = size_t(3) << 16;
 struct StagingSlot {
     std::mutex mu;
     double *h = nullptr, *d = nullptr;
@@ -410,7 +414,7 @@ int State::download(double *const *out) {
     if (!uploaded) return 0;
     const int n = gpd.n;
     StagingUse use(*this);
-    if (int e = use.take(9 * (size_t)n)) return e;
+    if (int e = use.take(std::min(9 * (size_t)n, kStageOnce))) return e;
     use.busy = true;
     MDX_CUDA_TRY(cudaMemcpyAsync(h_status, d_status.p, sizeof(DeviceStatus), cudaMemcpyDeviceToHost, stream));
     // all three arrays of some atoms to a piece: a host atom is touched once
@@ -448,7 +452,7 @@ int State::download(double *const *out) {
 int State::put(const double *pos, const double *vel) {
     const int n = gpd.n;
     StagingUse use(*this);
-    if (int e = use.take(6 * (size_t)n)) return e;
+    if (int e = use.take(std::min(6 * (size_t)n, kStageOnce))) return e;
     if (pos)
         if (int e = use.put(0, pos)) return e;
     if (vel)

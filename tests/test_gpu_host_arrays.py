@@ -33,9 +33,10 @@ def _state(n, seed, L=80.0):
     return st, x0, v0
 
 
-# 233,016 atoms cross to the host in one piece, more in pieces of 116,508; an
-# array of 349,525 atoms is one piece
-@pytest.mark.parametrize("n", [1, 255, 44000, 90001, 175001, 233016, 233017, 350001])
+# 21,845 atoms cross to the host in one piece, more in pieces of 10,922; an array
+# of 32,768 atoms to the device; in a host-buffer run the three results of
+# 233,016 atoms at once, else arrays of 349,525 atoms in one piece
+@pytest.mark.parametrize("n", [1, 255, 21845, 21846, 32769, 44000, 90001, 175001, 233016, 233017, 350001])
 def test_round_trip(n):
     rng, L = np.random.default_rng(n + 1), 80.0
     st, x0, v0 = _state(n, n)
